@@ -757,7 +757,7 @@ std::vector<float> pack_table(const HostRep& h, const std::vector<float>& params
       q[2] = p[2];
       q[3] = c_s;
       q[4] = c_u0;
-      q[5] = c_s;
+      q[5] = 6.f * p[2];
     } else if (pot == POT_LJ_12_6_SMOOTH_2_4) {
       // u = 4eps [(s/r)^12 - (s/r)^6 + c2 (r/s)^2 + c4 (r/s)^4]: the r^2 and
       // r^4 terms folded into b, c (force) and e, g (energy) per unit of d^2

@@ -55,13 +55,13 @@ enum { POT_LJ_12_6 = 0, POT_LJ_12_6_SMOOTH_2_4 = 1, POT_IPL_N = 2 };
 
 // Packed pair row (kParStride floats; slot 6 is (rc+skin)^2 for every pair
 // function, read by the list build).  The cut-off method is folded into c_s,
-// c_u0 (and c_ur):
-//   LJ 12-6:          rc^2, A12, A6, c_s, c_u0, c_ur, (rc+skin)^2, 0, ...
+// c_u0:
+//   LJ 12-6:          rc^2, A12, A6, c_s, c_u0, 6 A6, (rc+skin)^2, 0, ...
 //   LJ 12-6 smooth:   rc^2, sigma^2, 4 eps, b, c, e, (rc+skin)^2, g, c_s, c_u0
 //                     (b = -2 c2 4eps/sigma^2, c = -4 c4 4eps/sigma^4,
 //                      e = c2 4eps/sigma^2, g = c4 4eps/sigma^4)
 //   IPL n:            rc^2, sigma^2, eps, n/2, n eps, 0, (rc+skin)^2, 0, c_s, c_u0
-// (see lj_pair).
+// (see pair_add).
 struct RepDev {
   int n, p0, tile0, ntiles;
   int group0, ngroups;

@@ -6,9 +6,8 @@
 //     (SimulationBox.h:111-125, NeighborList.cu:1106-1140, 1282-1285) with the
 //     multiply-add contractions that nvcc applies to it written out as
 //     __fmaf_rn, so list sets and the sort permutation are bit-exact.
-//   * Pair forces are FP32 (PairPotential.h:161-168, 1198-1244); 1/r is the
-//     hardware reciprocal square root refined by one Newton-Raphson step and
-//     1/r^2 its square.
+//   * Pair forces are FP32 (PairPotential.h:161-168, 1198-1244); 1/r^2 and 1/r
+//     are the hardware reciprocal and reciprocal square root.
 //   * Reductions (pe, virial, kinetic energy, momentum) are FP64 with a fixed
 //     summation tree, so results do not depend on scheduling or on which other
 //     replicas share the launch; the thermostat state is FP64.
@@ -19,21 +18,31 @@
 
 namespace b2md {
 
-__device__ __forceinline__ double warp_sum_d(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-
 // Block sum of kNPart doubles per thread -> s_out[kNPart] (valid after return,
-// fixed tree: warp butterfly then warps in index order).
+// fixed tree).  The warp's 8 x 32 values are summed by a transposing exchange
+// -- at each of the first three levels a lane gives away half of its sums and
+// keeps the other half, then two plain levels -- which is 9 shuffles of a
+// double where a butterfly per value takes 40; lane 4k holds sum k.  Then the
+// warps are added in index order.
 __device__ __forceinline__ void block_sum8(double (&v)[kNPart], double* s_warp, double* s_out) {
+  static_assert(kNPart == 8, "three halving levels");
+  constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  double a[4], b[2];
 #pragma unroll
-  for (int k = 0; k < kNPart; ++k) {
-    double x = warp_sum_d(v[k]);
-    if (lane == 0) s_warp[wid * kNPart + k] = x;
+  for (int k = 0; k < 4; ++k) {
+    const double keep = lane & 16 ? v[k + 4] : v[k], give = lane & 16 ? v[k] : v[k + 4];
+    a[k] = keep + __shfl_xor_sync(FULL, give, 16);
   }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double keep = lane & 8 ? a[k + 2] : a[k], give = lane & 8 ? a[k] : a[k + 2];
+    b[k] = keep + __shfl_xor_sync(FULL, give, 8);
+  }
+  double c = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(FULL, lane & 4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(FULL, c, 2);
+  c += __shfl_xor_sync(FULL, c, 1);
+  if ((lane & 3) == 0) s_warp[wid * kNPart + (lane >> 2)] = c;
   __syncthreads();
   if (threadIdx.x < kNPart) {
     double s = 0.0;
@@ -225,17 +234,39 @@ __device__ int claim_tile(const EngArgs& a) {
   return tile;
 }
 
+// What a step's integration needs of its replica, the same for every
+// particle: the thermostat's coefficients and, on steps that remove the
+// centre-of-mass momentum, the velocity to subtract.  Computed once per tile
+// (a correctly rounded division, up to three FP64 divisions and a remainder,
+// which as per-thread code took a fifth of the tile's instructions).
+struct StepCoef {
+  NvtCoef c;
+  float3 vshift;
+  int reset;
+};
+
+__device__ __forceinline__ void step_coef(StepCoef& o, const RepDev& R, double xi, long long run_step, double M,
+                                          double Px, double Py, double Pz) {
+  o.c = nvt_coef((float)xi, R.dt);
+  bool reset = false;
+  if (R.reset_interval > 0)
+    reset = (run_step >> 31) == 0 ? (unsigned)run_step % (unsigned)R.reset_interval == 0u
+                                  : run_step % R.reset_interval == 0;
+  o.vshift = make_float3(0.f, 0.f, 0.f);
+  if (reset && M > 0.0) o.vshift = make_float3((float)(Px / M), (float)(Py / M), (float)(Pz / M));
+  o.reset = reset;
+}
+
 // Nose-Hoover leap-frog for one particle (integrateNVTAlgorithm,
-// IntegratorNVT.cu:364-418); accumulates FP64 kinetic sums.
-__device__ __forceinline__ void integrate_one(const RepDev& R, float xi_f, float3 vshift, bool do_reset,
-                                              float4 r, float4 f, float4& v, int4& im, float4& rn,
-                                              double (&acc)[kNPart], bool& exceed, float4 lr) {
+// IntegratorNVT.cu:364-418); accumulates FP64 kinetic sums.  A type without
+// thermostat has xi = 0, whose coefficients are exactly 1.
+__device__ __forceinline__ void integrate_one(const RepDev& R, const StepCoef& sc, float4 r, float4 f, float4& v,
+                                              int4& im, float4& rn, double (&acc)[kNPart], bool& exceed, float4 lr) {
   const int ti = __float_as_int(r.w);
   const bool thermo = (R.thermo_mask >> ti) & 1u;
-  if (do_reset) { v.x -= vshift.x; v.y -= vshift.y; v.z -= vshift.z; }
-  const float xs = thermo ? xi_f : 0.f;
+  if (sc.reset) { v.x -= sc.vshift.x; v.y -= sc.vshift.y; v.z -= sc.vshift.z; }
   const float dt = R.dt;
-  const NvtCoef c = nvt_coef(xs, dt);
+  const NvtCoef c{thermo ? sc.c.plus : 1.f, thermo ? sc.c.minus : 1.f};
   const double vb = (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z;
   float vx = nvt_velocity(c, v.x, v.w, f.x, dt);
   float vy = nvt_velocity(c, v.y, v.w, f.y, dt);
@@ -246,7 +277,7 @@ __device__ __forceinline__ void integrate_one(const RepDev& R, float xi_f, float
   im.x += (int)kx; im.y += (int)ky; im.z += (int)kz;
   v.x = vx; v.y = vy; v.z = vz;
   rn = make_float4(x, y, z, r.w);
-  const double m = 1.0 / (double)v.w;
+  const double m = v.w == 1.f ? 1.0 : 1.0 / (double)v.w;
   const double vf = (double)vx * vx + (double)vy * vy + (double)vz * vz;
   acc[P_KET] += 0.25 * m * (vb + vf);
   if (thermo) acc[P_KE2] += m * vf;
@@ -396,45 +427,40 @@ struct PairAcc {
 // The pair rows of particle i's type, looked up by the neighbour's type.
 //   RowsShared  the packed rows in shared memory: any pair function, any
 //               number of types;
-//   RowsLJ<NT>  the LJ 12-6 rows (rc^2, A12, A6, c_s, c_u0) of a replica with
+//   RowsLJ<NT>  the LJ 12-6 rows (rc^2, A12, A6, c_s, c_u0, 6 A6) of a replica with
 //               NT = 1 or 2 types, held in registers: no lookup (NT = 1) or a
 //               select (NT = 2), which keeps the table reads off the L1 data
 //               pipe that the neighbour gathers use.
 struct RowsShared {
   const float* prow;
   __device__ __forceinline__ const float* row(int tj) const { return prow + tj * kParStride; }
-  __device__ __forceinline__ void lj(int tj, float4& q, float& cu0) const {
+  __device__ __forceinline__ void lj(int tj, float4& q, float2& p) const {
     const float* pp = row(tj);
     q = *reinterpret_cast<const float4*>(pp);
-    cu0 = pp[4];
+    p = *reinterpret_cast<const float2*>(pp + 4);
   }
 };
 
 template <int NT>
 struct RowsLJ {
   float4 q0, q1;
-  float c0, c1;
+  float2 p0, p1;
   __device__ __forceinline__ explicit RowsLJ(const float* prow) {
     q0 = *reinterpret_cast<const float4*>(prow);
-    c0 = prow[4];
+    p0 = *reinterpret_cast<const float2*>(prow + 4);
     if (NT == 2) {
       q1 = *reinterpret_cast<const float4*>(prow + kParStride);
-      c1 = prow[kParStride + 4];
+      p1 = *reinterpret_cast<const float2*>(prow + kParStride + 4);
     } else {
       q1 = q0;
-      c1 = c0;
+      p1 = p0;
     }
   }
   __device__ __forceinline__ const float* row(int) const { return nullptr; }
-  __device__ __forceinline__ void lj(int tj, float4& q, float& cu0) const {
-    if (NT == 1) {
-      q = q0;
-      cu0 = c0;
-    } else {
-      const bool b = tj != 0;
-      q = make_float4(b ? q1.x : q0.x, b ? q1.y : q0.y, b ? q1.z : q0.z, b ? q1.w : q0.w);
-      cu0 = b ? c1 : c0;
-    }
+  __device__ __forceinline__ void lj(int tj, float4& q, float2& p) const {
+    const bool b = NT == 2 && tj != 0;
+    q = make_float4(b ? q1.x : q0.x, b ? q1.y : q0.y, b ? q1.z : q0.z, b ? q1.w : q0.w);
+    p = make_float2(b ? p1.x : p0.x, b ? p1.y : p0.y);
   }
 };
 
@@ -445,36 +471,59 @@ struct RowsLJ {
 //   POT_LJ_12_6_SMOOTH_2_4 Pot_LJ_12_6_smooth_2_4::ComputeInteraction
 //                          (PairPotential.h:248-255)
 //   POT_IPL_N              Pot_IPL_n::ComputeInteraction (PairPotential.h:630-636)
-// 1/r comes from one MUFU rsqrt refined by one Newton-Raphson step
-// (y <- y (3/2 - x y^2 / 2)); 1/r^2 = y^2.  The cut-off method is folded into
+// 1/r^2 is the hardware reciprocal of d^2 (one unit in the last place); 1/r,
+// which only the small shifted-force term uses, the hardware reciprocal
+// square root.  (1/r^2 as the square of a Newton-refined rsqrt took five
+// operations more per pair and was no closer: forces are 2.2e-6 rms-rel from
+// the FP64 sums either way, KA N=32000.)  The cut-off method is folded into
 // the packed pair row: s -= c_s / r and u += c_s r + c_u0, which is
 // s(rc) rc / r and s(rc) rc (r - rc) - u(rc) for SF, -u(rc) for SP, 0 for NS.
-// WRAP = false skips the minimum-image step; the caller uses it only when it
-// is exactly the identity (see k_force).
-template <bool STRESS, bool WRAP, int POT, class Rows>
-__device__ __forceinline__ void lj_pair(PairAcc& A, const float4& ri, const float4& rj, const Rows& rows, float Lx,
-                                        float Ly, float Lz, float iLx, float iLy, float iLz) {
-  float dx = ri.x - rj.x, dy = ri.y - rj.y, dz = ri.z - rj.z;
-  if (WRAP) {
-    dx = mi_comp(dx, Lx, iLx);
-    dy = mi_comp(dy, Ly, iLy);
-    dz = mi_comp(dz, Lz, iLz);
+// wrap: the dimensions (x 1, y 2, z 4) in which the minimum-image step is not
+// exactly the identity for every particle of the warp (see k_force); the same
+// for the whole warp.  ok = false: the entry is not one of the lane's.
+struct PairDisp {
+  float dx, dy, dz;
+};
+
+template <int U>
+__device__ __forceinline__ void pair_disp(PairDisp (&d)[U], const float4& ri, const float4 (&rj)[U], unsigned wrap,
+                                          float Lx, float Ly, float Lz, float iLx, float iLy, float iLz) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    d[u].dx = ri.x - rj[u].x;
+    d[u].dy = ri.y - rj[u].y;
+    d[u].dz = ri.z - rj[u].z;
   }
+  if (wrap & 1u) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u].dx = mi_comp(d[u].dx, Lx, iLx);
+  }
+  if (wrap & 2u) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u].dy = mi_comp(d[u].dy, Ly, iLy);
+  }
+  if (wrap & 4u) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u].dz = mi_comp(d[u].dz, Lz, iLz);
+  }
+}
+
+template <bool STRESS, int POT, class Rows>
+__device__ __forceinline__ void pair_add(PairAcc& A, bool ok, const PairDisp& d, int tj, const Rows& rows) {
+  const float dx = d.dx, dy = d.dy, dz = d.dz;
   const float d2 = dist2_ref(dx, dy, dz);
-  const int tj = __float_as_int(rj.w);
-  float y = rsqrt_approx(d2);
-  y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
-  const float i2 = y * y;
+  const float i2 = rcp_approx(d2), y = rsqrt_approx(d2);
   float s, u;
   bool in;
   if constexpr (POT == POT_LJ_12_6) {
-    float4 q;  // rc^2, A12, A6, c_s (= c_ur)
-    float cu0;
-    rows.lj(tj, q, cu0);
+    float4 q;  // rc^2, A12, A6, c_s
+    float2 p;  // c_u0, 6 A6
+    rows.lj(tj, q, p);
     const float i6 = i2 * i2 * i2;
     const float t = q.y * i6;
-    s = __fmaf_rn(-q.w, y, i6 * i2 * __fmaf_rn(12.f, t, 6.f * q.z));
-    u = __fmaf_rn(i6, t + q.z, __fmaf_rn(q.w, d2 * y, cu0));
+    const float w = q.w * y;
+    s = __fmaf_rn(i6 * i2, __fmaf_rn(12.f, t, p.y), -w);
+    u = __fmaf_rn(w, d2, __fmaf_rn(i6, t + q.z, p.x));
     in = d2 < q.x;
   } else if constexpr (POT == POT_LJ_12_6_SMOOTH_2_4) {
     const float* pp = rows.row(tj);
@@ -496,6 +545,7 @@ __device__ __forceinline__ void lj_pair(PairAcc& A, const float4& ri, const floa
     u = __fmaf_rn(q.z, tn, __fmaf_rn(q2.x, d2 * y, q2.y));
     in = d2 < q.x;
   }
+  in = in && ok;
   s = in ? s : 0.f;
   u = in ? u : 0.f;
   A.fx = __fmaf_rn(dx, s, A.fx);
@@ -555,61 +605,94 @@ __device__ __forceinline__ unsigned lane_count(unsigned nn, unsigned t) {
   return (nn >> 3) * (unsigned)E + (unsigned)min(E, max(0, rem));
 }
 
-// List-entry readers for force_loop: one(k) is entry k of the particle;
-// group<TP>(q, t) is lane t's entries q .. q+3 (q a multiple of 4).
-// Streamed: read from the global list inside the loop, past L1.
-struct IdxStreamed {
-  const unsigned* base;  // the replica's list
-  unsigned i;            // the particle's slot
-  size_t stride;
-  __device__ __forceinline__ unsigned one(unsigned k) const { return ld_stream(base + lpos(k, i, stride)); }
-  template <int TP>
-  __device__ __forceinline__ uint4 group(unsigned q, unsigned t) const {
-    constexpr unsigned E = 8 / TP;
-    if (E >= 4) return ld_stream_v4(base + lpos(lane_entry<TP>(q, t), i, stride));
-    if (E == 2) {
-      const uint2 a = ld_stream_v2(base + lpos(lane_entry<TP>(q, t), i, stride));
-      const uint2 b = ld_stream_v2(base + lpos(lane_entry<TP>(q + 2, t), i, stride));
-      return make_uint4(a.x, a.y, b.x, b.y);
-    }
-    return make_uint4(one(lane_entry<TP>(q, t)), one(lane_entry<TP>(q + 1, t)), one(lane_entry<TP>(q + 2, t)),
-                      one(lane_entry<TP>(q + 3, t)));
+// List-entry readers for force_loop: group<TP>(q, t, left) is lane t's entries
+// q .. q+3 (q a multiple of 4) of which the first `left` exist.  Only blocks
+// of 8 that hold one of those are read (the list's last block may be its
+// replica's last); entries past `left` are unspecified.  Rd reads 1, 2 or 4
+// consecutive entries.
+template <class Rd>
+struct IdxList {
+  const typename Rd::T* base;  // entry k of the particle at base + (k / 8) bstride + k % 8
+  size_t bstride;
+  __device__ __forceinline__ const typename Rd::T* at(unsigned k) const {
+    return base + (size_t)(k >> 3) * bstride + (k & 7u);
   }
+  template <int TP>
+  __device__ __forceinline__ uint4 group(unsigned q, unsigned t, unsigned left) const {
+    constexpr unsigned E = 8 / TP;
+    uint4 j = make_uint4(0u, 0u, 0u, 0u);
+    if (E >= 4) {
+      if (left > 0) j = Rd::four(at(lane_entry<TP>(q, t)));
+    } else if (E == 2) {
+      uint2 a = make_uint2(0u, 0u), b = make_uint2(0u, 0u);
+      if (left > 0) a = Rd::two(at(lane_entry<TP>(q, t)));
+      if (left > 2) b = Rd::two(at(lane_entry<TP>(q + 2, t)));
+      j = make_uint4(a.x, a.y, b.x, b.y);
+    } else {
+      if (left > 0) j.x = Rd::one(at(lane_entry<TP>(q, t)));
+      if (left > 1) j.y = Rd::one(at(lane_entry<TP>(q + 1, t)));
+      if (left > 2) j.z = Rd::one(at(lane_entry<TP>(q + 2, t)));
+      if (left > 3) j.w = Rd::one(at(lane_entry<TP>(q + 3, t)));
+    }
+    return j;
+  }
+};
+struct RdStream {  // the global list, past L1
+  using T = unsigned;
+  __device__ __forceinline__ static unsigned one(const T* p) { return ld_stream(p); }
+  __device__ __forceinline__ static uint2 two(const T* p) { return ld_stream_v2(p); }
+  __device__ __forceinline__ static uint4 four(const T* p) { return ld_stream_v4(p); }
 };
 // Streamed through L2 only (ld.global.cg): for kernels that rewrite the
 // list while they run (k_batch builds lists and reads them in one launch),
 // where the read-only path may not see those writes.
-__device__ __forceinline__ unsigned ld_cg_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint2 ld_cg_v2(const unsigned* p) {
-  uint2 v;
-  asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint4 ld_cg_v4(const unsigned* p) {
-  uint4 v;
-  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-struct IdxStreamedCg {
-  const unsigned* base;
-  unsigned i;
-  size_t stride;
-  __device__ __forceinline__ unsigned one(unsigned k) const { return ld_cg_u32(base + lpos(k, i, stride)); }
-  template <int TP>
-  __device__ __forceinline__ uint4 group(unsigned q, unsigned t) const {
-    constexpr unsigned E = 8 / TP;
-    if (E >= 4) return ld_cg_v4(base + lpos(lane_entry<TP>(q, t), i, stride));
-    if (E == 2) {
-      const uint2 a = ld_cg_v2(base + lpos(lane_entry<TP>(q, t), i, stride));
-      const uint2 b = ld_cg_v2(base + lpos(lane_entry<TP>(q + 2, t), i, stride));
-      return make_uint4(a.x, a.y, b.x, b.y);
-    }
-    return make_uint4(one(lane_entry<TP>(q, t)), one(lane_entry<TP>(q + 1, t)), one(lane_entry<TP>(q + 2, t)),
-                      one(lane_entry<TP>(q + 3, t)));
+struct RdStreamCg {
+  using T = unsigned;
+  __device__ __forceinline__ static unsigned one(const T* p) {
+    unsigned v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+  }
+  __device__ __forceinline__ static uint2 two(const T* p) {
+    uint2 v;
+    asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+  }
+  __device__ __forceinline__ static uint4 four(const T* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+  }
+};
+struct RdShared {  // the tile's list blocks copied to shared memory
+  using T = unsigned;
+  __device__ __forceinline__ static unsigned one(const T* p) { return *p; }
+  __device__ __forceinline__ static uint2 two(const T* p) { return *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ static uint4 four(const T* p) { return *reinterpret_cast<const uint4*>(p); }
+};
+struct RdWindow {  // the 16-bit window list (offsets into the tile's position window)
+  using T = unsigned short;
+  __device__ __forceinline__ static unsigned one(const T* p) { return ld_stream_u16(p); }
+  __device__ __forceinline__ static uint2 two(const T* p) {
+    const unsigned w = ld_stream(reinterpret_cast<const unsigned*>(p));
+    return make_uint2(w & 0xffffu, w >> 16);
+  }
+  __device__ __forceinline__ static uint4 four(const T* p) {
+    const uint2 w = ld_stream_v2(reinterpret_cast<const unsigned*>(p));
+    return make_uint4(w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16);
+  }
+};
+struct RdWindowShared {  // the tile's window-list blocks copied to shared memory
+  using T = unsigned short;
+  __device__ __forceinline__ static unsigned one(const T* p) { return *p; }
+  __device__ __forceinline__ static uint2 two(const T* p) {
+    const unsigned w = *reinterpret_cast<const unsigned*>(p);
+    return make_uint2(w & 0xffffu, w >> 16);
+  }
+  __device__ __forceinline__ static uint4 four(const T* p) {
+    const uint2 w = *reinterpret_cast<const uint2*>(p);
+    return make_uint4(w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16);
   }
 };
 // A position through L1 with a plain (coherent) load, for data the running
@@ -619,81 +702,6 @@ __device__ __forceinline__ float4 ld_ca_f4(const float4* p) {
   asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
-
-// Staged: the tile's list blocks copied to shared memory, block b of slot lp
-// at p[(b * pb + lp) * 8]; p points at this particle's first block.
-struct IdxStaged {
-  const unsigned* p;
-  int bstride;  // pb * 8
-  __device__ __forceinline__ unsigned one(unsigned k) const { return p[(k >> 3) * bstride + (k & 7u)]; }
-  template <int TP>
-  __device__ __forceinline__ uint4 group(unsigned q, unsigned t) const {
-    constexpr unsigned E = 8 / TP;
-    if (E >= 4) {
-      const unsigned k = lane_entry<TP>(q, t);
-      return *reinterpret_cast<const uint4*>(p + (k >> 3) * bstride + (k & 7u));
-    }
-    if (E == 2) {
-      const unsigned k0 = lane_entry<TP>(q, t), k1 = lane_entry<TP>(q + 2, t);
-      const uint2 a = *reinterpret_cast<const uint2*>(p + (k0 >> 3) * bstride + (k0 & 7u));
-      const uint2 b = *reinterpret_cast<const uint2*>(p + (k1 >> 3) * bstride + (k1 & 7u));
-      return make_uint4(a.x, a.y, b.x, b.y);
-    }
-    return make_uint4(one(lane_entry<TP>(q, t)), one(lane_entry<TP>(q + 1, t)), one(lane_entry<TP>(q + 2, t)),
-                      one(lane_entry<TP>(q + 3, t)));
-  }
-};
-// Window: the 16-bit window list (offsets into the tile's position window),
-// in the list's layout.
-struct IdxWindow {
-  const unsigned short* base;
-  unsigned i;
-  size_t stride;
-  __device__ __forceinline__ unsigned one(unsigned k) const { return ld_stream_u16(base + lpos(k, i, stride)); }
-  template <int TP>
-  __device__ __forceinline__ uint4 group(unsigned q, unsigned t) const {
-    constexpr unsigned E = 8 / TP;
-    if (E >= 4) {
-      // four 16-bit entries = 8 bytes
-      const uint2 w = ld_stream_v2(reinterpret_cast<const unsigned*>(base + lpos(lane_entry<TP>(q, t), i, stride)));
-      return make_uint4(w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16);
-    }
-    if (E == 2) {
-      const unsigned a = ld_stream(reinterpret_cast<const unsigned*>(base + lpos(lane_entry<TP>(q, t), i, stride)));
-      const unsigned b =
-          ld_stream(reinterpret_cast<const unsigned*>(base + lpos(lane_entry<TP>(q + 2, t), i, stride)));
-      return make_uint4(a & 0xffffu, a >> 16, b & 0xffffu, b >> 16);
-    }
-    return make_uint4(one(lane_entry<TP>(q, t)), one(lane_entry<TP>(q + 1, t)), one(lane_entry<TP>(q + 2, t)),
-                      one(lane_entry<TP>(q + 3, t)));
-  }
-};
-
-// Window, staged: the tile's 16-bit window-list blocks copied to shared
-// memory, block b of slot lp at p[(b * pb + lp) * 8]; p points at this
-// particle's first block.
-struct IdxWindowStaged {
-  const unsigned short* p;
-  int bstride;  // pb * 8
-  __device__ __forceinline__ unsigned one(unsigned k) const { return p[(k >> 3) * bstride + (k & 7u)]; }
-  template <int TP>
-  __device__ __forceinline__ uint4 group(unsigned q, unsigned t) const {
-    constexpr unsigned E = 8 / TP;
-    if (E >= 4) {
-      const unsigned k = lane_entry<TP>(q, t);
-      const uint2 w = *reinterpret_cast<const uint2*>(p + (k >> 3) * bstride + (k & 7u));
-      return make_uint4(w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16);
-    }
-    if (E == 2) {
-      const unsigned k0 = lane_entry<TP>(q, t), k1 = lane_entry<TP>(q + 2, t);
-      const unsigned a = *reinterpret_cast<const unsigned*>(p + (k0 >> 3) * bstride + (k0 & 7u));
-      const unsigned b = *reinterpret_cast<const unsigned*>(p + (k1 >> 3) * bstride + (k1 & 7u));
-      return make_uint4(a & 0xffffu, a >> 16, b & 0xffffu, b >> 16);
-    }
-    return make_uint4(one(lane_entry<TP>(q, t)), one(lane_entry<TP>(q + 1, t)), one(lane_entry<TP>(q + 2, t)),
-                      one(lane_entry<TP>(q + 3, t)));
-  }
-};
 
 // Neighbour-position readers: gathered from global memory (through L1), or
 // from the tile's position window in shared memory.
@@ -717,53 +725,55 @@ struct PosWindow {
 };
 
 // The neighbour loop of one thread: its entries (lane_entry) in groups of
-// four -- one vector load of list entries, four neighbour positions in
-// flight -- then the remaining ones singly.  Only entries below nn are read.
-template <int TP, bool STRESS, bool WRAP, int POT, class Idx, class Pos, class Rows>
-__device__ __forceinline__ void force_loop(PairAcc& A, const Idx& idx, const Pos& pos, unsigned lane_t, unsigned nn,
-                                           const float4& ri, const Rows& prow, float Lx, float Ly, float Lz,
+// four -- one vector load of list entries, four neighbour positions in flight
+// -- the last group masked.  A group's entries are loaded while the group
+// before is computed, so that only the gathers' latency is left in the chain
+// (with both and a serial tail of up to three entries, warps spent 7.4 of
+// 13.3 cycles per instruction waiting for loads).
+template <int TP, bool STRESS, int POT, class Idx, class Pos, class Rows>
+__device__ __forceinline__ void force_loop(PairAcc& A, unsigned wrap, const Idx& idx, const Pos& pos, unsigned lane_t,
+                                           unsigned nn, const float4& ri, const Rows& rows, float Lx, float Ly, float Lz,
                                            float iLx, float iLy, float iLz) {
-  const unsigned cnt = lane_count<TP>(nn, lane_t);
-  unsigned q = 0;
-  for (; q + 4 <= cnt; q += 4) {
-    const uint4 j = idx.template group<TP>(q, lane_t);
-    const float4 r0 = pos(j.x), r1 = pos(j.y), r2 = pos(j.z), r3 = pos(j.w);
-    lj_pair<STRESS, WRAP, POT>(A, ri, r0, prow, Lx, Ly, Lz, iLx, iLy, iLz);
-    lj_pair<STRESS, WRAP, POT>(A, ri, r1, prow, Lx, Ly, Lz, iLx, iLy, iLz);
-    lj_pair<STRESS, WRAP, POT>(A, ri, r2, prow, Lx, Ly, Lz, iLx, iLy, iLz);
-    lj_pair<STRESS, WRAP, POT>(A, ri, r3, prow, Lx, Ly, Lz, iLx, iLy, iLz);
+  unsigned left = lane_count<TP>(nn, lane_t), q = 0;
+  uint4 j = idx.template group<TP>(0u, lane_t, left);
+#pragma unroll 1
+  while (left >= 4u) {
+    const float4 r[4] = {pos(j.x), pos(j.y), pos(j.z), pos(j.w)};
+    q += 4u;
+    left -= 4u;
+    j = idx.template group<TP>(q, lane_t, left);
+    PairDisp d[4];
+    pair_disp<4>(d, ri, r, wrap, Lx, Ly, Lz, iLx, iLy, iLz);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) pair_add<STRESS, POT>(A, true, d[u], __float_as_int(r[u].w), rows);
   }
-  for (; q < cnt; ++q) {
-    const float4 r0 = pos(idx.one(lane_entry<TP>(q, lane_t)));
-    lj_pair<STRESS, WRAP, POT>(A, ri, r0, prow, Lx, Ly, Lz, iLx, iLy, iLz);
+  if (left > 0u) {
+    const float4 r[3] = {pos(j.x), pos(left > 1u ? j.y : j.x), pos(left > 2u ? j.z : j.x)};
+    PairDisp d[3];
+    pair_disp<3>(d, ri, r, wrap, Lx, Ly, Lz, iLx, iLy, iLz);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) pair_add<STRESS, POT>(A, left > (unsigned)u, d[u], __float_as_int(r[u].w), rows);
   }
 }
 
-// The loop for the replica's pair function and type count (block-uniform)
-// and minimum-image need.  REG: single-type LJ 12-6 replicas hold their row
-// in registers (3.5 % faster at N = 1M; for two types the selects cost more
-// than the shared-memory lookups they replace, 40.2 vs 37.6 us at KA 65536).
+// The loop for the replica's pair function and type count (block-uniform).
+// REG: single-type LJ 12-6 replicas hold their row in registers (3.5 % faster
+// at N = 1M; for two types the selects cost more than the shared-memory
+// lookups they replace, 40.2 vs 37.6 us at KA 65536).
 template <int TP, bool STRESS, bool REG, class Idx, class Pos>
-__device__ __forceinline__ void force_loop_any(bool fast, int pot, int nt, PairAcc& A, const Idx& idx, const Pos& pos,
-                                               unsigned lane_t, unsigned nn, const float4& ri, const float* prow,
-                                               float Lx, float Ly, float Lz, float iLx, float iLy, float iLz) {
-#define FL(W, P, ROWS) force_loop<TP, STRESS, W, P>(A, idx, pos, lane_t, nn, ri, ROWS, Lx, Ly, Lz, iLx, iLy, iLz)
+__device__ __forceinline__ void force_loop_any(unsigned wrap, int pot, int nt, PairAcc& A, const Idx& idx,
+                                               const Pos& pos, unsigned lane_t, unsigned nn, const float4& ri,
+                                               const float* prow, float Lx, float Ly, float Lz, float iLx, float iLy,
+                                               float iLz) {
+#define FL(P, ROWS) force_loop<TP, STRESS, P>(A, wrap, idx, pos, lane_t, nn, ri, ROWS, Lx, Ly, Lz, iLx, iLy, iLz)
   const RowsShared sh{prow};
   if (pot == POT_LJ_12_6) {
-    if (REG && nt == 1) {
-      const RowsLJ<1> rg(prow);
-      if (fast) FL(false, POT_LJ_12_6, rg);
-      else FL(true, POT_LJ_12_6, rg);
-    } else {
-      if (fast) FL(false, POT_LJ_12_6, sh);
-      else FL(true, POT_LJ_12_6, sh);
-    }
+    if (REG && nt == 1) FL(POT_LJ_12_6, RowsLJ<1>(prow));
+    else FL(POT_LJ_12_6, sh);
   } else if (pot == POT_LJ_12_6_SMOOTH_2_4) {
-    if (fast) FL(false, POT_LJ_12_6_SMOOTH_2_4, sh);
-    else FL(true, POT_LJ_12_6_SMOOTH_2_4, sh);
+    FL(POT_LJ_12_6_SMOOTH_2_4, sh);
   } else {
-    if (fast) FL(false, POT_IPL_N, sh);
-    else FL(true, POT_IPL_N, sh);
+    FL(POT_IPL_N, sh);
   }
 #undef FL
 }
@@ -855,8 +865,8 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
   RepState* S = a.st + rep;
   // PERSIST: the block's view of its replica's state, kept by k_steps
   // (the buffer parity, step counters); xi and the momentum come from the
-  // previous step's finalizer just before the integration
-  __shared__ double s_xi, s_M, s_P[3];
+  // previous step's finalizer just before the integration, as s_sc
+  __shared__ StepCoef s_sc;
 #define SV(f) (PERSIST ? pv->f : S->f)
   const bool skip = (SV(overflow) != 0) || (FUSED && SV(steps_left) <= 0) || !R.active;
   if (!skip) {
@@ -924,6 +934,10 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
     const int nt = R.ntypes;
     if (!PERSIST)
       for (int k = threadIdx.x; k < nt * nt * kParStride; k += blockDim.x) s_par[k] = a.par[R.par0 + k];
+    if constexpr (FUSED && !PERSIST) {
+      // (published by the barrier before the neighbour loop)
+      if (threadIdx.x == blockDim.x - 1) step_coef(s_sc, R, S->xi, S->run_step, S->M, S->P[0], S->P[1], S->P[2]);
+    }
     const int lp = threadIdx.x / TP, lane_t = threadIdx.x % TP;
     const int i = first + lp;
     const bool valid = i < R.n;
@@ -936,27 +950,31 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
     const size_t lstride = (size_t)R.nbl_stride;
     const unsigned* lbase = a.nbl + R.nbl0;
     const unsigned short* wbase = a.wl + R.nbl0;
-    // A particle farther than rc_max + 2 skin from every face of the box has
-    // all its listed neighbours (within rc + skin at the build, each moved at
-    // most skin/2 since) inside the box at their minimum image, so the
-    // minimum-image correction is exactly zero; warps made only of such
-    // particles skip it.
-    const bool inner = fabsf(ri.x) < R.ilim[0] && fabsf(ri.y) < R.ilim[1] && fabsf(ri.z) < R.ilim[2];
-    const bool fast = __all_sync(0xffffffffu, !valid || inner);
+    // A particle farther than rc_max + 2 skin from both faces of a dimension
+    // has all its listed neighbours (within rc + skin at the build, each moved
+    // at most skin/2 since) at their minimum image in it, so the correction is
+    // exactly zero there; warps made only of such particles skip it.  Decided
+    // per dimension: a warp's particles are a run of cells along x, so at KA
+    // N=65536 about half of the warps need some dimension and few need all.
+    const unsigned wrap = (__any_sync(0xffffffffu, valid && !(fabsf(ri.x) < R.ilim[0])) ? 1u : 0u) |
+                          (__any_sync(0xffffffffu, valid && !(fabsf(ri.y) < R.ilim[1])) ? 2u : 0u) |
+                          (__any_sync(0xffffffffu, valid && !(fabsf(ri.z) < R.ilim[2])) ? 4u : 0u);
     PairAcc A;
     if (use_bar) {
       // 4. bounded wait for the copies (the barrier also publishes the pair table)
       const bool ok = __syncthreads_and(mbar_wait_bounded(&s_bar, 0, kWaitPolls));
       if (ok) {
         if (MODE == FM_STAGED)
-          force_loop_any<TP, STRESS, false>(fast, R.potential, nt, A, IdxStaged{s_idx + lp * 8, pitch * 8}, PosGlobal{rc}, lane_t, nn, ri, prow,
-                                     Lx, Ly, Lz, iLx, iLy, iLz);
+          force_loop_any<TP, STRESS, false>(wrap, R.potential, nt, A, IdxList<RdShared>{s_idx + lp * 8, (size_t)pitch * 8},
+                                            PosGlobal{rc}, lane_t, nn, ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
         else if (wl_staged)
-          force_loop_any<TP, STRESS, false>(fast, R.potential, nt, A, IdxWindowStaged{s_wl + lp * 8, pitch * 8}, PosWindow{s_win}, lane_t, nn,
-                                     ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
+          force_loop_any<TP, STRESS, false>(wrap, R.potential, nt, A,
+                                            IdxList<RdWindowShared>{s_wl + lp * 8, (size_t)pitch * 8}, PosWindow{s_win},
+                                            lane_t, nn, ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
         else
-          force_loop_any<TP, STRESS, false>(fast, R.potential, nt, A, IdxWindow{wbase, (unsigned)i, lstride}, PosWindow{s_win}, lane_t, nn, ri, prow,
-                                     Lx, Ly, Lz, iLx, iLy, iLz);
+          force_loop_any<TP, STRESS, false>(wrap, R.potential, nt, A,
+                                            IdxList<RdWindow>{wbase + (size_t)i * 8, lstride * 8}, PosWindow{s_win}, lane_t,
+                                            nn, ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
       } else {
         // the copies did not land in time: record it for the host and wait
         // (bounded) for them before this block's shared memory is released
@@ -966,9 +984,9 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
     } else {
       if (!PERSIST) __syncthreads();  // the pair table (k_steps loads it once per launch)
       using PosS = typename Pick<PERSIST || COH, PosCoherent, PosGlobal>::type;
-      using IdxS = typename Pick<COH, IdxStreamedCg, IdxStreamed>::type;
-      force_loop_any<TP, STRESS, true>(fast, R.potential, nt, A, IdxS{lbase, (unsigned)i, lstride}, PosS{rc}, lane_t, nn,
-                                       ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
+      using IdxS = IdxList<typename Pick<COH, RdStreamCg, RdStream>::type>;
+      force_loop_any<TP, STRESS, true>(wrap, R.potential, nt, A, IdxS{lbase + (size_t)i * 8, lstride * 8}, PosS{rc},
+                                       lane_t, nn, ri, prow, Lx, Ly, Lz, iLx, iLy, iLz);
     }
     float fx = A.fx, fy = A.fy, fz = A.fz, uu = A.uu, ww = A.ww;
     double sxx = A.sxx, syy = A.syy, szz = A.szz, syz = A.syz, sxz = A.sxz, sxy = A.sxy;
@@ -999,8 +1017,9 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
         // PairPotential.cu:370-388
         PairAcc B;
         const float* prow1 = a.par + R.par1 + ti * nt * kParStride;
-        force_loop_any<TP, STRESS, false>(fast, R.potential1, nt, B, IdxStreamed{lbase, (unsigned)i, lstride},
-                                          PosGlobal{rc}, lane_t, nn, ri, prow1, Lx, Ly, Lz, iLx, iLy, iLz);
+        force_loop_any<TP, STRESS, false>(wrap, R.potential1, nt, B,
+                                          IdxList<RdStream>{lbase + (size_t)i * 8, lstride * 8}, PosGlobal{rc}, lane_t, nn,
+                                          ri, prow1, Lx, Ly, Lz, iLx, iLy, iLz);
         if (TP > 1) {
 #pragma unroll
           for (int o = TP / 2; o > 0; o >>= 1) {
@@ -1038,15 +1057,11 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
           }
           __nanosleep(32);
         }
-        s_xi = __ldcg(&S->xi);
-        s_M = __ldcg(&S->M);
-        s_P[0] = __ldcg(&S->P[0]);
-        s_P[1] = __ldcg(&S->P[1]);
-        s_P[2] = __ldcg(&S->P[2]);
+        step_coef(s_sc, R, __ldcg(&S->xi), pv->run_step, __ldcg(&S->M), __ldcg(&S->P[0]), __ldcg(&S->P[1]),
+                  __ldcg(&S->P[2]));
       }
       __syncthreads();
     }
-#define SVS(f, pf) (PERSIST ? (pf) : S->f)
     double acc[kNPart];
 #pragma unroll
     for (int k = 0; k < kNPart; ++k) acc[k] = 0.0;
@@ -1063,15 +1078,8 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
         const int ab = SV(abuf);
         float4 v = PERSIST ? pr->v : a.v[ab][gi];
         int4 im = PERSIST ? pr->im : a.im[ab][gi];
-        const bool do_reset = R.reset_interval > 0 && (SV(run_step) % R.reset_interval) == 0;
-        float3 vs = make_float3(0.f, 0.f, 0.f);
-        const double M = SVS(M, s_M);
-        if (do_reset && M > 0.0)
-          vs = make_float3((float)(SVS(P[0], s_P[0]) / M), (float)(SVS(P[1], s_P[1]) / M),
-                           (float)(SVS(P[2], s_P[2]) / M));
         float4 rn;
-        integrate_one(R, (float)SVS(xi, s_xi), vs, do_reset, ri, fo, v, im, rn, acc, exceed,
-                      PERSIST ? pr->lr : a.last_r[gi]);
+        integrate_one(R, s_sc, ri, fo, v, im, rn, acc, exceed, PERSIST ? pr->lr : a.last_r[gi]);
         a.v[ab][gi] = v;
         a.im[ab][gi] = im;
         if (PERSIST) {
@@ -1108,7 +1116,6 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
         }
       }
     }
-#undef SVS
   }
 #undef SV
   return !skip;
@@ -1125,8 +1132,11 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
 //                TMA bulk copy per segment, and the 16-bit window list read
 //                from global memory: every neighbour position comes from shared
 //                memory.  Tiles without a window (wmeta < 0) stream.
+// The neighbour loop hides its gathers' latency with resident warps: at most
+// 64 registers (two blocks of 512) -- without the bound the compiler takes 100
+// for the same code, 343 instead of 234 us per step at LJ N = 2^20.
 template <int TP, bool FUSED, bool STRESS, int MODE>
-__global__ void __launch_bounds__(kMaxBlock) k_force(EngArgs a, int has_cond, cudaGraphConditionalHandle h) {
+__global__ void __launch_bounds__(kMaxBlock, STRESS ? 1 : 2) k_force(EngArgs a, int has_cond, cudaGraphConditionalHandle h) {
   extern __shared__ __align__(128) unsigned char s_dyn[];
   __shared__ double s_blk[kNPart], s_tot[kNPart];
   __shared__ __align__(8) uint64_t s_bar;
@@ -1401,7 +1411,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate(EngArgs a, int tp) {
     float4 r = a.r[rb][gi], f = a.f[gi], v = a.v[ab][gi];
     int4 im = a.im[ab][gi];
     float4 rn;
-    integrate_one(R, (float)S->xi, make_float3(0.f, 0.f, 0.f), false, r, f, v, im, rn, acc, exceed, a.last_r[gi]);
+    StepCoef sc{nvt_coef((float)S->xi, R.dt), make_float3(0.f, 0.f, 0.f), 0};
+    integrate_one(R, sc, r, f, v, im, rn, acc, exceed, a.last_r[gi]);
     acc[P_PE] = 0.0; acc[P_W] = 0.0;
     a.v[ab][gi] = v; a.im[ab][gi] = im; a.r[rb ^ 1][gi] = rn;
   }
