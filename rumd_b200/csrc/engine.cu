@@ -882,8 +882,10 @@ void launch_rebuild(b2md_engine* e, cudaStream_t s, const EngArgs& a) {
   // exceed a block), the list either assembled in shared memory or stored
   // straight to global memory
   if (e->build_lanes == 0 && !a.win_on) {
-    // one warp per cell, contiguous candidate runs per lane
-    k_rb_build_runs<<<T, kRunWarps * 32, 0, s>>>(a);
+    // one warp per cell; with few tiles, as many blocks per tile as the GPU
+    // holds at once and the tile has cells for (about three particles each)
+    const int parts = std::max(1, std::min(e->nsm * 8 / T, e->pb / (3 * kRunWarps)));
+    k_rb_build_runs<<<T * parts, kRunWarps * 32, 0, s>>>(a, parts);
     return;
   }
   if (e->build_lanes == 32 && !a.win_on) {
@@ -1121,7 +1123,7 @@ bool single_potential(const b2md_engine* e) {
 // Dynamic shared memory of k_batch: the larger of the force tile's region and
 // the list build's, then the per-block rebuild-list tables.
 size_t batch_smem(const b2md_engine* e, EngArgs& a) {
-  const size_t build = (size_t)kCs2Floats * sizeof(float) + (size_t)(e->pb * e->tp / 32) * 32 * kRunStride * sizeof(int);
+  const size_t build = (size_t)kBuildFloats * sizeof(float) + (size_t)(e->pb * e->tp / 32) * kRunRows * sizeof(int4);
   const size_t tile = std::max(force_smem(e, a), build);
   a.bshared_off = (int)((tile + 15) & ~(size_t)15);
   return (size_t)a.bshared_off + sizeof(BatchShared);
@@ -1130,7 +1132,7 @@ size_t batch_smem(const b2md_engine* e, EngArgs& a) {
 // Dynamic shared memory of k_flow: the larger of the force tile's region and
 // the list build's.
 size_t flow_smem(const b2md_engine* e, const EngArgs& a) {
-  const size_t build = (size_t)kCs2Floats * sizeof(float) + (size_t)(e->pb * e->tp / 32) * 32 * kRunStride * sizeof(int);
+  const size_t build = (size_t)kBuildFloats * sizeof(float) + (size_t)(e->pb * e->tp / 32) * kRunRows * sizeof(int4);
   return (std::max(force_smem(e, a), build) + 15) & ~(size_t)15;
 }
 

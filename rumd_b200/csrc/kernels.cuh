@@ -2384,107 +2384,120 @@ __global__ void __launch_bounds__(kCwWarps * 32) k_rb_build_cw(EngArgs a) {
   }
 }
 
-// (7'') The same list with one warp per cell and contiguous candidate runs:
-//       the cell's candidates (its 25 row parts, numbered in the reference's
-//       order) are cut into chunks of up to 32 * kRunMax, and lane l of the
-//       warp takes the consecutive run [l K, (l + 1) K) of a chunk (K <= 16).
-//       For two of the cell's particles at a time, a lane tests its run with
-//       no cross-lane traffic, keeping one accept bit per candidate; one
-//       exclusive scan of the lanes' accept counts then gives each lane the
-//       list position of its first accepted candidate, and the lane writes its
-//       accepted ones in run order.  Runs follow one another in candidate
-//       order, so the list is the reference's entry for entry.  Only the
-//       candidates' slots are staged (in shared memory, lane-major with an odd
-//       stride so that a warp's reads are bank-conflict free); their
-//       positions are read through L1, where the cell's other particles and
-//       the neighbouring cells' warps find them again.
-constexpr int kRunWarps = 4;                 // warps (cells in flight) per block
-constexpr int kRunMax = 16;                  // candidates per lane per chunk
-constexpr int kRunStride = kRunMax + 1;      // odd: conflict-free lane-major slots
-constexpr int kRunChunk = 32 * kRunMax;      // candidates per chunk
+// (7'') The default list build, one warp per cell: the cell's candidates (its
+//       25 row parts, numbered in the reference's order) are tested 32 at a
+//       time, one per lane, against up to four of the cell's particles held in
+//       registers.  A ballot gives each accepted candidate its place in the
+//       particle's list, so entries are stored in candidate order, the
+//       reference's, and a particle's entries of one round go to one or two
+//       32-byte sectors.  A lane finds the row of candidate number v by
+//       counting the rows that start at or before v: a 32-bit mask of the
+//       row starts in the round, plus the rows of earlier rounds.
+constexpr int kRunWarps = 4;  // warps (cells in flight) per block
+constexpr int kRunRows = 25;  // rows of a warp's table in shared memory
+// The build's shared table: the cut-offs, then the box lengths and their
+// inverses (read from there in the loop: the compiler must assume that the
+// list stores change the replica's descriptor).
+constexpr int kBuildFloats = kCs2Floats + 8;
 
-struct Cs2One {
-  float c0;
-  __device__ __forceinline__ float operator()(int) const { return c0; }
-};
-struct Cs2Two {
-  float c0, c1;
-  __device__ __forceinline__ float operator()(int tj) const { return tj ? c1 : c0; }
-};
-struct Cs2Table {
-  const float* row;
-  __device__ __forceinline__ float operator()(int tj) const { return row[tj]; }
+// One warp's row table: candidate v of a row is slot v + (v < z ? y : w); x is
+// the row's first candidate number.
+struct CellRows {
+  int off, len, total;  // this lane's row: first candidate, candidates; of all rows
+  const int4* tab;      // the non-empty rows in order
 };
 
-// Accept bits of a lane's run for G (4 or 2) of the cell's particles (a
-// missing one repeats the last; its bits are unused): each candidate's
-// position is read once and tested against all G.  G = 2 serves the last
-// one or two particles of a cell, so that cells of 1, 2, 5 or 6 particles do
-// not test padding copies.
-template <bool WRAP, bool COH, int G, class CS2>
-__device__ __forceinline__ void run_tests(const int* __restrict__ run, int nrun, const float4* rc,
-                                          const float4 (&rp)[4], const int (&ip)[4], const CS2 (&cs)[4],
-                                          float Lx, float Ly, float Lz, float iLx, float iLy, float iLz,
-                                          unsigned (&bits)[4]) {
+// Lists the particles [pg, pg + G) of a cell.  NT: 1 or 2 particle types (the
+// cut-offs in registers) or 0 (any number, from the table).  wrap: the
+// dimensions (1, 2, 4) in which a neighbour cell wraps around the box or the
+// box has fewer than 7 cells; in the others the minimum-image step is exactly
+// the identity.  Returns the longest list.
+template <int G, int NT, bool COH>
+__device__ __forceinline__ int build_cell(const RepDev& R, const float4* rc, const CellRows& cr, int pg, unsigned wrap,
+                                          const float* s_cs2, unsigned* __restrict__ lbase, unsigned* __restrict__ nn,
+                                          float4* __restrict__ last_r) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const unsigned stride8 = 8u * (unsigned)R.nbl_stride;
+  const unsigned maxn = (unsigned)R.max_nbrs;
+  const int nt = R.ntypes;
+  const float c00 = s_cs2[0], c01 = NT == 2 ? s_cs2[1] : 0.f, c10 = NT == 2 ? s_cs2[2] : 0.f,
+              c11 = NT == 2 ? s_cs2[3] : 0.f;
+  float4 rp[G];
+  unsigned cnt[G];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) bits[q] = 0u;
-#pragma unroll 2
-  for (int k = 0; k < kRunMax; ++k) {
-    if (k < nrun) {
-      const int j = run[k];
-      const float4 rj = COH ? ld_ca_f4(rc + j) : __ldg(rc + j);
-      const int tj = __float_as_int(rj.w);
+  for (int q = 0; q < G; ++q) {
+    rp[q] = COH ? ld_ca_f4(rc + pg + q) : __ldg(rc + pg + q);
+    cnt[q] = 0u;
+  }
+  int rows = 0;  // non-empty rows that start before this round
+#pragma unroll 1
+  for (int ch = 0; ch < cr.total; ch += 32) {
+    const int v = ch + lane;
+    const unsigned rel = (unsigned)(cr.off - ch);
+    const unsigned st = __reduce_or_sync(FULL, cr.len > 0 && rel < 32u ? 1u << rel : 0u);
+    const int4 t = cr.tab[rows + __popc(st & (lt + lt + 1u)) - 1];
+    rows += __popc(st);
+    const bool have = v < cr.total;
+    const int j = have ? v + (v < t.z ? t.y : t.w) : pg;
+    const float4 rj = COH ? ld_ca_f4(rc + j) : __ldg(rc + j);
+    const int tj = __float_as_int(rj.w);
+    float dx[G], dy[G], dz[G];
 #pragma unroll
-      for (int q = 0; q < G; ++q) {
-        float dx = rp[q].x - rj.x, dy = rp[q].y - rj.y, dz = rp[q].z - rj.z;
-        if (WRAP) {
-          dx = mi_comp(dx, Lx, iLx);
-          dy = mi_comp(dy, Ly, iLy);
-          dz = mi_comp(dz, Lz, iLz);
-        }
-        if (dist2_ref(dx, dy, dz) < cs[q](tj) && j != ip[q]) bits[q] |= 1u << k;
-      }
+    for (int q = 0; q < G; ++q) {
+      dx[q] = rp[q].x - rj.x;
+      dy[q] = rp[q].y - rj.y;
+      dz[q] = rp[q].z - rj.z;
+    }
+    if (wrap & 1u) {
+#pragma unroll
+      for (int q = 0; q < G; ++q) dx[q] = mi_comp(dx[q], s_cs2[kCs2Floats], s_cs2[kCs2Floats + 3]);
+    }
+    if (wrap & 2u) {
+#pragma unroll
+      for (int q = 0; q < G; ++q) dy[q] = mi_comp(dy[q], s_cs2[kCs2Floats + 1], s_cs2[kCs2Floats + 4]);
+    }
+    if (wrap & 4u) {
+#pragma unroll
+      for (int q = 0; q < G; ++q) dz[q] = mi_comp(dz[q], s_cs2[kCs2Floats + 2], s_cs2[kCs2Floats + 5]);
+    }
+    const float ca = NT == 2 && tj ? c01 : c00, cb = NT == 2 && tj ? c11 : c10;  // of types 0 and 1
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      const int tq = __float_as_int(rp[q].w);
+      const float cs = NT == 1 ? c00 : NT == 2 ? (tq ? cb : ca) : s_cs2[tq * nt + tj];
+      const bool in = have && dist2_ref(dx[q], dy[q], dz[q]) < cs && j != pg + q;
+      const unsigned m = __ballot_sync(FULL, in);
+      const unsigned pos = cnt[q] + __popc(m & lt);
+      if (in && pos < maxn) lbase[(pos >> 3) * stride8 + ((unsigned)(pg + q) << 3) + (pos & 7u)] = (unsigned)j;
+      cnt[q] += __popc(m);
     }
   }
-}
-
-// Writes particle p's accepted candidates of this chunk: `bits` of the lane's
-// run, after `cnt` entries already in p's list (32-bit offsets from the
-// replica's list: entry k of slot p at (k/8) 8 stride + 8 p + k%8).
-// Returns the chunk's total for p.
-__device__ __forceinline__ int run_store(unsigned bits, const int* __restrict__ run, int cnt, int maxn,
-                                         unsigned* __restrict__ lbase, unsigned p, unsigned stride8) {
-  const int lane = threadIdx.x & 31;
-  const int c = __popc(bits);
-  int incl = c;
+  int wmax = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
+  for (int q = 0; q < G; ++q) {
+    wmax = max(wmax, (int)cnt[q]);
+    if (lane == q) {
+      nn[pg + q] = min(cnt[q], maxn);
+      last_r[pg + q] = rp[q];
+    }
   }
-  unsigned pos = (unsigned)(cnt + incl - c);
-  const unsigned pb = p << 3;
-  while (bits) {
-    const int k = __ffs(bits) - 1;
-    bits &= bits - 1u;
-    if (pos < (unsigned)maxn) lbase[(pos >> 3) * stride8 + pb + (pos & 7u)] = (unsigned)run[k];
-    ++pos;
-  }
-  return __shfl_sync(0xffffffffu, incl, 31);
+  return wmax;
 }
 
-// The run build of one tile by the calling block (blockDim a multiple of 32:
-// one cell per warp at a time).  s_cs2: the cut-off table (kCs2Floats),
-// s_run: 32 * kRunStride ints per warp, s_max: one int.  COH: the positions
-// and cell arrays were written earlier in the same launch (k_batch), so they
-// are read with coherent loads.
-// GRID: the block's warps claim cells of the whole replica from its counter
+// The build of one tile by `parts` blocks, of which the calling one is number
+// `part` (blockDim a multiple of 32: one cell per warp at a time).  s_cs2: the
+// build's table (kBuildFloats), s_rows: kRunRows int4 per warp, s_max: one
+// int.  COH: the positions and cell arrays were written earlier in the same
+// launch (k_batch), so they are read with coherent loads.
+// GRID: the blocks' warps claim cells of the whole replica from its counter
 // (S->build_next) and list every particle of a claimed cell, so the work of
 // all the replica's blocks evens out (cell method only); the tile's range
 // then serves only the bookkeeping.
 template <bool COH, bool GRID = false>
-__device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, float* s_cs2, int* s_run, int* s_max,
-                                                int* s_last = nullptr, int* s_next = nullptr) {
+__device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, float* s_cs2, int4* s_rows, int* s_max,
+                                                int* s_last = nullptr, int part = 0, int parts = 1) {
   constexpr unsigned FULL = 0xffffffffu;
   const int rep = a.tile_rep[tile];
   const RepDev& R = a.rep[rep];
@@ -2492,62 +2505,69 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
   const int nt = R.ntypes;
   const int nwarps = blockDim.x >> 5;
   for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) s_cs2[k] = a.par[R.par0 + k * kParStride + 6];
-  if (threadIdx.x == 0) {
-    *s_max = 0;
-    if (s_next) *s_next = nwarps;
-  }
+  if (threadIdx.x < 6) s_cs2[kCs2Floats + threadIdx.x] = threadIdx.x < 3 ? R.L[threadIdx.x] : R.invL[threadIdx.x - 3];
+  if (threadIdx.x == 0) *s_max = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = a.tile_first[tile];
   const int last = (tile + 1 < R.tile0 + R.ntiles) ? a.tile_first[tile + 1] : R.n;
   const float4* rc = a.r[COH ? __ldcg(&S->rbuf) : S->rbuf] + R.p0;
-  const int maxn = R.max_nbrs;
-  const unsigned stride8 = 8u * (unsigned)R.nbl_stride;
   unsigned* __restrict__ lbase = a.nbl + R.nbl0;
-  int* wrun = s_run + warp * 32 * kRunStride;
-  const int* run = wrun + lane * kRunStride;
+  unsigned* __restrict__ nn = a.nn + R.p0;
+  float4* __restrict__ last_r = a.last_r + R.p0;
+  int4* tab = s_rows + warp * kRunRows;
   const bool cells = R.nb_method == NB_CELLS;
   const int nx = R.nc[0], ny = R.nc[1], nz = R.nc[2];
   const int* cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_fix / block_sort)
   const int* ccnt = a.cnt + R.cell0;
-  // units of work: the cells from the first to the last particle's (keys
-  // ascend along the slots), or one unit for all pairs
-  int k0 = 0, k1 = 0;
+  // units of work: cells (of the replica, or from the tile's first to its last
+  // particle's: keys ascend along the slots), or four particles each for all
+  // pairs
+  int k0 = 0, k1 = -1;
   if (GRID) {
     k1 = R.ncell - 1;
-  } else if (cells && last > first) {
+  } else if (!cells) {
+    k1 = (last - first + 3) / 4 - 1;
+  } else if (last > first) {
     const float4 rf = rc[first], rl = rc[last - 1];
     const float iLx = R.invL[0], iLy = R.invL[1], iLz = R.invL[2];
     k0 = cell_coord(rf.x, iLx, nx) + cell_coord(rf.y, iLy, ny) * nx + cell_coord(rf.z, iLz, nz) * nx * ny;
     k1 = cell_coord(rl.x, iLx, nx) + cell_coord(rl.y, iLy, ny) * nx + cell_coord(rl.z, iLz, nz) * nx * ny;
   }
   int wmax = 0;
-  // cells in order, each warp taking the next unclaimed one (s_next: the
-  // warps' cells even out within the block), or every nwarps-th
-  auto next_cell = [&](int c) -> int {
-    if (GRID) {
-      int v = 0;
-      if (lane == 0) v = atomicAdd(&S->build_next, 1);
-      return __shfl_sync(FULL, v, 0);
-    }
-    if (!s_next) return c + nwarps;
-    int v = 0;
-    if (lane == 0) v = atomicAdd(s_next, 1);
-    return k0 + __shfl_sync(FULL, v, 0);
+  // units in order, each warp taking the replica's next unclaimed cell (lane 0
+  // asks for it before the current one is listed, so that the claim's round
+  // trip overlaps the work) or every (nwarps parts)-th unit
+  auto claim = [&](int c) -> int {
+    if (GRID) return lane == 0 ? atomicAdd(&S->build_next, 1) : 0;
+    return c + nwarps * parts;
   };
-  for (int c = GRID ? next_cell(0) : k0 + warp; c <= k1; c = next_cell(c)) {
-    const int p0 = GRID ? cbeg[c] : cells ? max(cbeg[c], first) : first;
-    const int p1 = GRID ? cbeg[c] + ccnt[c] : cells ? min(cbeg[c] + ccnt[c], last) : last;
+  int nextc = GRID ? claim(0) : k0 + part * nwarps + warp;
+  for (;;) {
+    const int c = __shfl_sync(FULL, nextc, 0);
+    if (c > k1) break;
+    nextc = claim(c);
+    int p0, p1;
+    if (GRID) {
+      p0 = cbeg[c];
+      p1 = p0 + ccnt[c];
+    } else if (cells) {
+      p0 = max(cbeg[c], first);
+      p1 = min(cbeg[c] + ccnt[c], last);
+    } else {
+      p0 = first + 4 * c;
+      p1 = min(p0 + 4, last);
+    }
     if (p0 >= p1) continue;  // no particle of this tile in the cell
     // lane r < 25: row (dz, dy) = (r/5 - 2, r%5 - 2) as one or two slot parts
     int b0 = 0, e0 = 0, b1 = 0, e1 = 0;
-    bool wrap = true;
+    unsigned wrap = 7u;
     if (cells) {
       const int cx = c % nx, cy = (c / nx) % ny, cz = c / (nx * ny);
-      // no wrapped cell among the 5x5x5 and at least 7 cells a side: the
-      // minimum-image step is exactly the identity
-      wrap = !(nx >= 7 && ny >= 7 && nz >= 7 && cx >= 2 && cx < nx - 2 && cy >= 2 && cy < ny - 2 && cz >= 2 &&
-               cz < nz - 2);
+      // a dimension with at least 7 cells of which none of the five wraps:
+      // the minimum-image step is exactly the identity in it
+      wrap = (nx >= 7 && cx >= 2 && cx < nx - 2 ? 0u : 1u) | (ny >= 7 && cy >= 2 && cy < ny - 2 ? 0u : 2u) |
+             (nz >= 7 && cz >= 2 && cz < nz - 2 ? 0u : 4u);
       if (lane < 25) {
         const int dz = lane / 5 - 2, dy = lane % 5 - 2;
         int oz = cz + dz;
@@ -2581,86 +2601,29 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
       const int y = __shfl_up_sync(FULL, incl, o);
       if (lane >= o) incl += y;
     }
-    const int off = incl - len;                 // this lane's first candidate number
-    const int M = __shfl_sync(FULL, incl, 31);  // candidates of the unit
-    for (int pg = p0; pg < p1; pg += 32) {
-      const int pe = min(p1, pg + 32);
-      int cnt_reg = 0;  // lane k: list length so far of particle pg + k
-      for (int ch = 0; ch < M; ch += kRunChunk) {
-        const int mc = min(kRunChunk, M - ch);
-        const int K = (mc + 31) >> 5;  // run length of every lane but the last ones
-        __syncwarp();
-        // candidate number v of the chunk goes to lane v / K, place v % K:
-        // each row lane writes its own parts' candidates, stepping the
-        // (lane, place) pair instead of dividing per candidate
-        {
-          const int v0 = max(off, ch), v1 = min(off + len, ch + mc);
-          if (v0 < v1) {
-            int qk = (v0 - ch) / K, rk = (v0 - ch) - qk * K;
-            for (int v = v0; v < v1; ++v) {
-              wrun[qk * kRunStride + rk] = v - off < l0 ? b0 + (v - off) : b1 + (v - off - l0);
-              if (++rk == K) {
-                rk = 0;
-                ++qk;
-              }
-            }
-          }
-        }
-        __syncwarp();
-        const int nrun = min(K, max(0, mc - lane * K));
-        for (int p = pg; p < pe; p += 4) {
-          // up to four of the cell's particles against the chunk
-          float4 rp[4];
-          int ip[4];
-          const float* crow[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            ip[q] = min(p + q, pe - 1);
-            rp[q] = rc[ip[q]];
-            crow[q] = s_cs2 + __float_as_int(rp[q].w) * nt;
-          }
-          unsigned bits[4];
-#define RUNS(W, T, MK)                                                                                    \
-  {                                                                                                       \
-    const T cs[4] = {MK(crow[0]), MK(crow[1]), MK(crow[2]), MK(crow[3])};                                 \
-    if (pe - p <= 2)                                                                                      \
-      run_tests<W, COH, 2>(run, nrun, rc, rp, ip, cs, R.L[0], R.L[1], R.L[2], R.invL[0], R.invL[1], R.invL[2], bits); \
-    else                                                                                                  \
-      run_tests<W, COH, 4>(run, nrun, rc, rp, ip, cs, R.L[0], R.L[1], R.L[2], R.invL[0], R.invL[1], R.invL[2], bits); \
+    const int off = incl - len;  // this lane's first candidate number
+    const CellRows cr{off, len, __shfl_sync(FULL, incl, 31), tab};
+    const unsigned ne = __ballot_sync(FULL, len > 0);
+    __syncwarp();
+    if (len > 0) tab[__popc(ne & ((1u << lane) - 1u))] = make_int4(off, b0 - off, off + l0, b1 - off - l0);
+    __syncwarp();
+    for (int pg = p0; pg < p1; pg += 4) {
+#define BC(G, NT) wmax = max(wmax, build_cell<G, NT, COH>(R, rc, cr, pg, wrap, s_cs2, lbase, nn, last_r))
+#define BCN(G)              \
+  {                         \
+    if (nt == 1) BC(G, 1);  \
+    else if (nt == 2) BC(G, 2); \
+    else BC(G, 0);          \
   }
-#define ONE(c) Cs2One{(c)[0]}
-#define TWO(c) Cs2Two{(c)[0], (c)[1]}
-#define TAB(c) Cs2Table{(c)}
-          if (nt == 1) {
-            if (wrap) RUNS(true, Cs2One, ONE) else RUNS(false, Cs2One, ONE)
-          } else if (nt == 2) {
-            if (wrap) RUNS(true, Cs2Two, TWO) else RUNS(false, Cs2Two, TWO)
-          } else {
-            if (wrap) RUNS(true, Cs2Table, TAB) else RUNS(false, Cs2Table, TAB)
-          }
-#undef RUNS
-#undef ONE
-#undef TWO
-#undef TAB
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (p + q < pe) {
-              const int cq = __shfl_sync(FULL, cnt_reg, p + q - pg);
-              const int tot = run_store(bits[q], run, cq, maxn, lbase, (unsigned)(p + q), stride8);
-              if (lane == p + q - pg) cnt_reg = cq + tot;
-            }
-          }
-        }
-      }
-      if (pg + lane < pe) {
-        const int p = pg + lane;
-        a.nn[(size_t)R.p0 + p] = (unsigned)min(cnt_reg, maxn);
-        a.last_r[(size_t)R.p0 + p] = rc[p];
-        wmax = max(wmax, cnt_reg);
-      }
+      const int np = p1 - pg;
+      if (np >= 4) BCN(4)
+      else if (np == 3) BCN(3)
+      else if (np == 2) BCN(2)
+      else BCN(1)
+#undef BCN
+#undef BC
     }
   }
-  wmax = __reduce_max_sync(FULL, wmax);
   if (lane == 0) atomicMax(s_max, wmax);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -2672,8 +2635,9 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
     }
     __threadfence();
     const unsigned cdone = atomicAdd(&a.rctr[rep], 1u);
-    if (s_last) *s_last = cdone == (unsigned)(R.ntiles - 1);
-    if (cdone == (unsigned)(R.ntiles - 1)) {
+    const bool fin = cdone == (unsigned)(R.ntiles * parts - 1);
+    if (s_last) *s_last = fin;
+    if (fin) {
       a.rctr[rep] = 0u;
       if (GRID) S->build_next = 0;
       S->nrebuilds += 1;
@@ -2685,26 +2649,29 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
 
 // k_batch's call of the build: kept out of line so that its registers do
 // not add to those of k_batch's force path.
-__device__ __noinline__ void build_runs_tile_batch(const EngArgs& a, int tile, float* s_cs2, int* s_run, int* s_max) {
-  build_runs_tile<true>(a, tile, s_cs2, s_run, s_max);
+__device__ __noinline__ void build_runs_tile_batch(const EngArgs& a, int tile, float* s_cs2, int4* s_rows, int* s_max) {
+  build_runs_tile<true>(a, tile, s_cs2, s_rows, s_max);
 }
 // k_flow's: also reports whether this item's build was the replica's last;
 // cell-method replicas claim cells replica-wide (an item queued late finds
-// the cells taken and ends at once), others by the block's counter s_next.
-__device__ __noinline__ void build_runs_tile_flow(const EngArgs& a, int tile, float* s_cs2, int* s_run, int* s_max,
-                                                  int* s_last, int* s_next) {
-  if (a.rep[a.tile_rep[tile]].nb_method == NB_CELLS) build_runs_tile<true, true>(a, tile, s_cs2, s_run, s_max, s_last);
-  else build_runs_tile<true>(a, tile, s_cs2, s_run, s_max, s_last, s_next);
+// the cells taken and ends at once).
+__device__ __noinline__ void build_runs_tile_flow(const EngArgs& a, int tile, float* s_cs2, int4* s_rows, int* s_max,
+                                                  int* s_last) {
+  if (a.rep[a.tile_rep[tile]].nb_method == NB_CELLS) build_runs_tile<true, true>(a, tile, s_cs2, s_rows, s_max, s_last);
+  else build_runs_tile<true>(a, tile, s_cs2, s_rows, s_max, s_last);
 }
 
-__global__ void __launch_bounds__(kRunWarps * 32) k_rb_build_runs(EngArgs a) {
-  __shared__ float s_cs2[kCs2Floats];
-  __shared__ int s_run[kRunWarps * 32 * kRunStride];
-  __shared__ int s_max, s_next;
-  const int rep = a.tile_rep[blockIdx.x];
+// `parts` blocks per tile (launch_rebuild: small systems have too few tiles to
+// fill the GPU with a block each).
+__global__ void __maxnreg__(64) k_rb_build_runs(EngArgs a, int parts) {
+  __shared__ float s_cs2[kBuildFloats];
+  __shared__ int4 s_rows[kRunWarps * kRunRows];
+  __shared__ int s_max;
+  const int tile = blockIdx.x / parts, part = blockIdx.x - tile * parts;
+  const int rep = a.tile_rep[tile];
   if (!rb_active(a, rep)) return;
-  if (a.rep[rep].nb_method == NB_CELLS) build_runs_tile<false, true>(a, blockIdx.x, s_cs2, s_run, &s_max);
-  else build_runs_tile<false>(a, blockIdx.x, s_cs2, s_run, &s_max, nullptr, &s_next);
+  if (a.rep[rep].nb_method == NB_CELLS) build_runs_tile<false, true>(a, tile, s_cs2, s_rows, &s_max, nullptr, part, parts);
+  else build_runs_tile<false>(a, tile, s_cs2, s_rows, &s_max, nullptr, part, parts);
 }
 
 // ---------------------------------------------------------------------------
@@ -3357,8 +3324,8 @@ __global__ void __maxnreg__(64) k_batch(EngArgs a, cudaGraphConditionalHandle h_
         if (s_ok) {
           if (build) {
             float* s_cs2 = reinterpret_cast<float*>(s_dyn);
-            int* s_run = reinterpret_cast<int*>(s_dyn + kCs2Floats * sizeof(float));
-            build_runs_tile_batch(a, tile, s_cs2, s_run, &s_max);
+            int4* s_cr = reinterpret_cast<int4*>(s_dyn + kBuildFloats * sizeof(float));
+            build_runs_tile_batch(a, tile, s_cs2, s_cr, &s_max);
           } else {
             force_tile<TP, true, false, FM_STREAMED, false, true>(a, tile, s_dyn, s_blk, s_tot, s_bar, s_rows,
                                                                   nullptr, 0, nullptr, nullptr, nullptr, par ^ 1);
@@ -3624,8 +3591,8 @@ __global__ void __maxnreg__(64) k_flow(EngArgs a, cudaGraphConditionalHandle h_l
       }
     } else {
       float* s_cs2 = reinterpret_cast<float*>(s_dyn);
-      int* s_run = reinterpret_cast<int*>(s_dyn + kCs2Floats * sizeof(float));
-      build_runs_tile_flow(a, R.tile0 + idx, s_cs2, s_run, &s_max, &s_last, &s_flag);  // s_flag: cell claims
+      int4* s_cr = reinterpret_cast<int4*>(s_dyn + kBuildFloats * sizeof(float));
+      build_runs_tile_flow(a, R.tile0 + idx, s_cs2, s_cr, &s_max, &s_last);
       __syncthreads();
       if (s_last) {
         // the replica's lists are complete: its force tiles, unless a list
