@@ -409,9 +409,10 @@ B2MD_API int b2md_probe_nvt(const float* r4, const float* v4, const float* f4, c
  *   force4  DEVICE pointer, n*4 floats out (fx, fy, fz, u_i)
  *   sums    DEVICE pointer, 2 doubles out (sum u_i, virial W)
  *   stream  cudaStream_t to run on (NULL = default stream); returns at launch
- * All pairs within the cut-off are summed (no neighbour list).  n is at most
- * 65536: the only scratch is a fixed array of that capacity in the library's
- * device image, one per GPU, kept until the process exits and shared by every
+ * All pairs within the cut-off are summed (no neighbour list; the particles
+ * are binned in cells where that pays).  n is at most 65536: the only scratch
+ * is a fixed array of that capacity (about 3 MB) in the library's device
+ * image, one per GPU, kept until the process exits and shared by every
  * call, so calls that overlap on the GPU race; order them on one stream.  The
  * first call on each device looks up the array's device address
  * (cudaGetSymbolAddress) with that device current; make that first call

@@ -7,15 +7,16 @@
 // cudaMalloc/cudaFree because those may synchronise the device and take
 // unbounded time.  b2md_forces_noalloc serves them: the caller passes device
 // pointers to its own inputs and outputs, and the only scratch memory (the
-// per-block FP64 partial sums of the energy and virial and a completion
-// counter) is a fixed, statically allocated array in this library's device
-// image, sized for at most kNoAllocMaxParticles particles.
+// particles binned in cells, the per-block FP64 partial sums of the energy and
+// virial and a completion counter) is a fixed, statically allocated array in
+// this library's device image, sized for at most kNoAllocMaxParticles
+// particles.
 //
 // The array exists once per GPU that loads the library and lives until the
 // process exits.  Every call shares it, so calls whose kernels overlap on the
 // GPU (different streams, no ordering between them) race on it; order them on
-// one stream or with events.  The completion counter is cleared at the start
-// of every call; the partial sums are overwritten before they are read.
+// one stream or with events.  The completion counter and the cell counts are
+// cleared at the start of every call; the rest is overwritten before it is read.
 //
 // Host code cannot use the array's name as a device address (it names a
 // host-side stand-in).  The first call on a device, with that device current,
@@ -32,6 +33,9 @@
 // Its results match b2md_calc_f for the same configuration: the same pair
 // function (shifted-force / shifted-potential / plain LJ), all pairs within
 // the cut-off under the minimum-image convention, per-particle energies halved.
+#include <algorithm>
+#include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <mutex>
 
@@ -42,14 +46,29 @@ namespace {
 
 constexpr int kNoAllocMaxParticles = 65536;
 constexpr int kNoAllocBlock = 128;
-constexpr int kNoAllocMaxBlocks = kNoAllocMaxParticles / kNoAllocBlock;
+constexpr int kNoAllocWarps = kNoAllocBlock / 32;
+constexpr int kNoAllocMaxBlocks = 2048;
+constexpr int kNoAllocMaxCells = 65536;
 constexpr int kNoAllocMaxTypes = 8;
-constexpr int kRow = 8;  // rc^2, A12, A6, c_s, c_u0, c_ur, unused x2
+constexpr int kRow = 8;    // rc^2, A12, A6, c_s, c_u0, 6 A6, unused x2
+constexpr int kRows = 25;  // (dz, dy) rows of a cell's 5x5x5 neighbourhood
 
 struct NoAllocScratch {
+  unsigned counter;            // blocks finished in this call; cleared with cnt
+  int dense;                   // a cell holds more than kDense particles: all pairs instead
+  unsigned pad[62];
+  int cnt[kNoAllocMaxCells];   // particles per cell
+  int start[kNoAllocMaxCells]; // first sorted place of each cell
+  int key[kNoAllocMaxParticles], rank[kNoAllocMaxParticles], order[kNoAllocMaxParticles];
+  float4 pos[kNoAllocMaxParticles];   // sorted by (cell, index), wrapped into the box
+  unsigned id[kNoAllocMaxParticles];  // the particle of each sorted place; kBadType set: unknown type
   double part[kNoAllocMaxBlocks][2];  // per-block sums of u_i and w_i
-  unsigned counter;                    // blocks finished in this call
 };
+constexpr unsigned kBadType = 0x80000000u;
+// One warp lists a cell's particles, so a few crowded cells (a cluster in a
+// box so large that its cells cannot be small) would leave the work to a few
+// warps: then the all-pairs form runs, which spreads evenly.
+constexpr int kDense = 64;
 
 // The scratch: a fixed array in the library's device image (no allocation).
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
@@ -64,71 +83,365 @@ std::mutex g_mu;
 NoAllocScratch* g_scratch_ptr[64] = {};
 void* g_scratch_ctx[64] = {};
 
-__global__ void __launch_bounds__(kNoAllocBlock)
-    k_forces_noalloc(const float4* __restrict__ pos, int n, float3 L, float3 iL, int ntypes, PairTable tab,
+struct Grid3 {
+  int nx, ny, nz;
+};
+
+// ---- particles binned in cells: sorted by (cell, index), so that every sum
+// below has a fixed order ----
+__device__ __forceinline__ float wrapped(float x, float L, float iL) {
+  return __fmaf_rn(-L, rintf(x * iL), x);  // x itself inside the box
+}
+__device__ __forceinline__ int cell_of(float x, float iL, int nc) {
+  const int c = __float2int_rz(__fmaf_rn(x, iL, 0.5f) * (float)nc);  // 0 for NaN
+  return min(max(c, 0), nc - 1);
+}
+
+__global__ void __launch_bounds__(256) k_na_count(const float4* __restrict__ pos, int n, float3 L, float3 iL, Grid3 g,
+                                                  NoAllocScratch* scr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 r = pos[i];
+  const int c = cell_of(wrapped(r.x, L.x, iL.x), iL.x, g.nx) +
+                g.nx * (cell_of(wrapped(r.y, L.y, iL.y), iL.y, g.ny) + g.ny * cell_of(wrapped(r.z, L.z, iL.z), iL.z, g.nz));
+  scr->key[i] = c;
+  scr->rank[i] = atomicAdd(&scr->cnt[c], 1);
+}
+
+// exclusive scan of the cell counts (and the largest) by one block: thread t
+// owns a run of cells
+__global__ void __launch_bounds__(1024) k_na_scan(int ncell, NoAllocScratch* scr) {
+  __shared__ int s_w[32], s_m[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int run = ((ncell + 1023) / 1024 + 3) & ~3;  // whole int4 loads
+  const int c0 = threadIdx.x * run, c1 = min(ncell, c0 + run);
+  int tot = 0, most = 0;
+  for (int c = c0; c < c1; c += 4) {  // counts past ncell are zero
+    const int4 x = *reinterpret_cast<const int4*>(scr->cnt + c);
+    tot += x.x + x.y + x.z + x.w;
+    most = max(max(most, max(x.x, x.y)), max(x.z, x.w));
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  int incl = tot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) {
+    s_w[wid] = incl;
+    s_m[wid] = most;
+  }
+  __syncthreads();
+  int first = incl - tot;
+  for (int w = 0; w < wid; ++w) first += s_w[w];
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 32; ++w) most = max(most, s_m[w]);
+    scr->dense = most > kDense;
+  }
+  for (int c = c0; c < c1; c += 4) {
+    const int4 x = *reinterpret_cast<const int4*>(scr->cnt + c);
+    const int4 o = make_int4(first, first + x.x, first + x.x + x.y, first + x.x + x.y + x.z);
+    *reinterpret_cast<int4*>(scr->start + c) = o;
+    first = o.w + x.w;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_na_scatter(int n, NoAllocScratch* scr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) scr->order[scr->start[scr->key[i]] + scr->rank[i]] = i;
+}
+
+// Each bucket by index (its members counted against each other; a few per
+// cell), positions wrapped into the box.  A particle of unknown type gets a
+// NaN position: no pair with it is in range.
+__global__ void __launch_bounds__(256) k_na_gather(const float4* __restrict__ pos, int n, float3 L, float3 iL,
+                                                   int ntypes, NoAllocScratch* scr) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n || scr->dense) return;
+  const int i = scr->order[s], c = scr->key[i], b = scr->start[c], m = scr->cnt[c];
+  int place = b;
+  for (int k = 0; k < m; ++k) place += scr->order[b + k] < i;
+  float4 r = pos[i];
+  const int t = __float_as_int(r.w);
+  const bool ok = t >= 0 && t < ntypes;
+  r.x = ok ? wrapped(r.x, L.x, iL.x) : __int_as_float(0x7fc00000);
+  r.y = wrapped(r.y, L.y, iL.y);
+  r.z = wrapped(r.z, L.z, iL.z);
+  r.w = ok ? r.w : 0.f;
+  scr->pos[place] = r;
+  scr->id[place] = (unsigned)i | (ok ? 0u : kBadType);
+}
+
+// ---- pair sums ----
+struct Sum5 {
+  float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f, w = 0.f;
+};
+
+// The warp's sums of G particles' values: lane q 32/G holds particle q's
+// total (fixed tree; halving exchanges while more than one particle is left).
+template <int G>
+__device__ __forceinline__ float warp_sum(const float (&v)[G]) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  float x;
+  int o = 16;
+  if constexpr (G == 4) {
+    float a[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float keep = lane & 16 ? v[k + 2] : v[k], give = lane & 16 ? v[k] : v[k + 2];
+      a[k] = keep + __shfl_xor_sync(FULL, give, 16);
+    }
+    x = (lane & 8 ? a[1] : a[0]) + __shfl_xor_sync(FULL, lane & 8 ? a[0] : a[1], 8);
+    o = 4;
+  } else if constexpr (G == 2) {
+    x = (lane & 16 ? v[1] : v[0]) + __shfl_xor_sync(FULL, lane & 16 ? v[0] : v[1], 16);
+    o = 8;
+  } else {
+    x = v[0];
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
+  return x;
+}
+
+// Candidate j of every lane (a NaN position where the lane has none) against
+// the warp's G particles.  wrap: the dimensions (1, 2, 4) that need the
+// minimum-image step; uniform in the warp.
+template <int G>
+__device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G], int p0, int j, const float4& rj,
+                                              unsigned wrap, const float* s_tab, int ntypes, const float3& L,
+                                              const float3& iL) {
+  const int tj = __float_as_int(rj.w);
+  float dx[G], dy[G], dz[G];
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    dx[q] = rp[q].x - rj.x;
+    dy[q] = rp[q].y - rj.y;
+    dz[q] = rp[q].z - rj.z;
+  }
+  if (wrap & 1u)
+#pragma unroll
+    for (int q = 0; q < G; ++q) dx[q] = b2md::mi_comp(dx[q], L.x, iL.x);
+  if (wrap & 2u)
+#pragma unroll
+    for (int q = 0; q < G; ++q) dy[q] = b2md::mi_comp(dy[q], L.y, iL.y);
+  if (wrap & 4u)
+#pragma unroll
+    for (int q = 0; q < G; ++q) dz[q] = b2md::mi_comp(dz[q], L.z, iL.z);
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    const float d2 = b2md::dist2_ref(dx[q], dy[q], dz[q]);
+    const float* row = s_tab + (__float_as_int(rp[q].w) * ntypes + tj) * kRow;
+    const float4 c = *reinterpret_cast<const float4*>(row);  // rc^2, A12, A6, c_s
+    const bool in = d2 < c.x && j != p0 + q;
+    if (!__any_sync(0xffffffffu, in)) continue;
+    // the engine's pair function (pair_add of the step kernels)
+    const float2 e = *reinterpret_cast<const float2*>(row + 4);  // c_u0, 6 A6
+    const float i2 = b2md::rcp_approx(d2), y = b2md::rsqrt_approx(d2);
+    const float i6 = i2 * i2 * i2, t = c.y * i6, w = c.w * y;
+    const float s = __fmaf_rn(i6 * i2, __fmaf_rn(12.f, t, e.y), -w);
+    if (in) {  // (dx is NaN in lanes without a candidate)
+      A[q].u += __fmaf_rn(w, d2, __fmaf_rn(i6, t + c.z, e.x));
+      A[q].fx = __fmaf_rn(dx[q], s, A[q].fx);
+      A[q].fy = __fmaf_rn(dy[q], s, A[q].fy);
+      A[q].fz = __fmaf_rn(dz[q], s, A[q].fz);
+      A[q].w = __fmaf_rn(d2, s, A[q].w);
+    }
+  }
+}
+
+// Forces of particles p0 .. p0 + G - 1 from the sums, by the lanes that hold
+// them; their energies and virials are added to u, w.
+template <int G>
+__device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned (&id)[G], float4* __restrict__ force,
+                                             double& u, double& w) {
+  float v[5][G];
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    v[0][q] = A[q].fx; v[1][q] = A[q].fy; v[2][q] = A[q].fz; v[3][q] = A[q].u; v[4][q] = A[q].w;
+  }
+  const float fx = warp_sum<G>(v[0]), fy = warp_sum<G>(v[1]), fz = warp_sum<G>(v[2]), uu = warp_sum<G>(v[3]),
+              ww = warp_sum<G>(v[4]);
+  const int lane = threadIdx.x & 31;
+  if (lane % (32 / G) == 0) {
+    unsigned me = id[0];
+#pragma unroll
+    for (int q = 1; q < G; ++q) me = lane / (32 / G) == q ? id[q] : me;
+    if (me & kBadType) {
+      const float nanf_ = __int_as_float(0x7fc00000);
+      force[me & ~kBadType] = make_float4(nanf_, nanf_, nanf_, nanf_);
+    } else {
+      force[me] = make_float4(fx, fy, fz, 0.5f * uu);
+      u += 0.5 * (double)uu;
+      w += (double)ww;
+    }
+  }
+}
+
+template <int G>
+__device__ __forceinline__ void cell_group(NoAllocScratch* scr, const int4* tab, int off, int len, int total, int p0,
+                                           unsigned wrap, const float* s_tab, int ntypes, const float3& L,
+                                           const float3& iL, float4* __restrict__ force, double& u, double& w) {
+  const int lane = threadIdx.x & 31;
+  const float4* __restrict__ sp = scr->pos;
+  Sum5 A[G];
+  float4 rp[G];
+  unsigned id[G];
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    rp[q] = sp[p0 + q];
+    id[q] = scr->id[p0 + q];
+  }
+  int rows = 0;  // non-empty rows that start before this round
+#pragma unroll 1
+  for (int ch = 0; ch < total; ch += 32) {
+    const int v = ch + lane;
+    const unsigned rel = (unsigned)(off - ch);
+    const unsigned st = __reduce_or_sync(0xffffffffu, len > 0 && rel < 32u ? 1u << rel : 0u);
+    const int4 t = tab[rows + __popc(st & ((2u << lane) - 1u)) - 1];
+    rows += __popc(st);
+    const int j = v < total ? v + (v < t.z ? t.y : t.w) : p0;
+    float4 rj = sp[j];
+    if (v >= total) rj.x = __int_as_float(0x7fc00000);
+    add_candidate<G>(A, rp, p0, j, rj, wrap, s_tab, ntypes, L, iL);
+  }
+  store_forces<G>(A, id, force, u, w);
+}
+
+template <int G>
+__device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, int n, int p0, const float* s_tab,
+                                                int ntypes, const float3& L, const float3& iL,
+                                                float4* __restrict__ force, double& u, double& w) {
+  const int lane = threadIdx.x & 31;
+  Sum5 A[G];
+  float4 rp[G];
+  unsigned id[G];
+#pragma unroll
+  for (int q = 0; q < G; ++q) {
+    rp[q] = pos[p0 + q];
+    const int t = __float_as_int(rp[q].w);
+    const bool ok = t >= 0 && t < ntypes;
+    id[q] = (unsigned)(p0 + q) | (ok ? 0u : kBadType);
+    if (!ok) rp[q].w = 0.f;
+  }
+#pragma unroll 2
+  for (int ch = 0; ch < n; ch += 32) {
+    const int j = ch + lane;
+    float4 rj = pos[min(j, n - 1)];
+    const int t = __float_as_int(rj.w);
+    if (j >= n || t < 0 || t >= ntypes) {
+      rj.x = __int_as_float(0x7fc00000);
+      rj.w = 0.f;
+    }
+    add_candidate<G>(A, rp, p0, j, rj, 7u, s_tab, ntypes, L, iL);
+  }
+  store_forces<G>(A, id, force, u, w);
+}
+
+// One warp works on up to four particles at a time, 32 candidates a round, one
+// per lane: of a cell's particles against its 5x5x5 neighbourhood (CELLS), or
+// of G consecutive particles against all.  Units go to warps in a fixed order.
+// What bounds the cell form is the pair arithmetic: about 300 candidates per
+// particle at KA density, of which a quarter is in range.  Held to 80
+// registers for six blocks per SM (137 us with 109 registers, 119 with 80, the
+// same with 64 and spills; KA N=65521).  Calls back to back, all pairs by one
+// thread per particle before: N=65521 7275 -> 119 us, N=16384 1388 -> 52,
+// N=4000 369 -> 37, N=1000 109 -> 17 (the last three mostly launches).
+template <int G, bool CELLS>
+__global__ void __launch_bounds__(kNoAllocBlock, 6)
+    k_forces_noalloc(const float4* __restrict__ pos, int n, float3 L, float3 iL, Grid3 g, int ntypes, PairTable tab,
                      float4* __restrict__ force, double* __restrict__ sums, NoAllocScratch* scr) {
-  __shared__ float4 s_r[kNoAllocBlock];
-  __shared__ float s_tab[kNoAllocMaxTypes * kNoAllocMaxTypes * kRow];
-  __shared__ double s_red[kNoAllocBlock / 32][2];
+  __shared__ __align__(16) float s_tab[kNoAllocMaxTypes * kNoAllocMaxTypes * kRow];
+  __shared__ int4 s_rows[kNoAllocWarps * kRows];
+  __shared__ double s_red[kNoAllocBlock][2];
   __shared__ int s_last;
   for (int k = threadIdx.x; k < ntypes * ntypes * kRow; k += blockDim.x) s_tab[k] = tab.p[k];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < n;
-  const float4 ri = valid ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const int ti = __float_as_int(ri.w);
-  const bool type_ok = ti >= 0 && ti < ntypes;
-  float fx = 0.f, fy = 0.f, fz = 0.f, uu = 0.f, ww = 0.f;
-  // all pairs, j staged through shared memory one block-width at a time
-  for (int base = 0; base < n; base += blockDim.x) {
-    __syncthreads();
-    if (base + threadIdx.x < n) s_r[threadIdx.x] = pos[base + threadIdx.x];
-    __syncthreads();
-    const int m = min((int)blockDim.x, n - base);
-    if (!valid || !type_ok) continue;
-    const float* row = s_tab + ti * ntypes * kRow;
-    for (int k = 0; k < m; ++k) {
-      const float4 rj = s_r[k];
-      const int tj = __float_as_int(rj.w);
-      if (base + k == i || tj < 0 || tj >= ntypes) continue;
-      const float dx = b2md::mi_comp(ri.x - rj.x, L.x, iL.x);
-      const float dy = b2md::mi_comp(ri.y - rj.y, L.y, iL.y);
-      const float dz = b2md::mi_comp(ri.z - rj.z, L.z, iL.z);
-      const float d2 = b2md::dist2_ref(dx, dy, dz);
-      const float* q = row + tj * kRow;
-      if (d2 < q[0]) {
-        // 1/r by rsqrt plus one Newton-Raphson step; the cut-off method is
-        // folded into c_s, c_u0, c_ur as in the engine's pair rows
-        float y = b2md::rsqrt_approx(d2);
-        y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
-        const float i2 = y * y, i6 = i2 * i2 * i2, t = q[1] * i6;
-        const float s = __fmaf_rn(-q[3], y, i6 * i2 * __fmaf_rn(12.f, t, 6.f * q[2]));
-        uu += __fmaf_rn(i6, t + q[2], __fmaf_rn(q[5], d2 * y, q[4]));
-        fx = __fmaf_rn(dx, s, fx);
-        fy = __fmaf_rn(dy, s, fy);
-        fz = __fmaf_rn(dz, s, fz);
-        ww = __fmaf_rn(d2, s, ww);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int stride = gridDim.x * kNoAllocWarps;
+  double u = 0.0, w = 0.0;
+  const bool by_cell = CELLS && !scr->dense;
+  if (by_cell) {
+    int4* rowtab = s_rows + warp * kRows;
+    const int ncell = g.nx * g.ny * g.nz;
+    for (int c = blockIdx.x * kNoAllocWarps + warp; c < ncell; c += stride) {
+      const int p0 = scr->start[c], p1 = p0 + scr->cnt[c];
+      if (p0 >= p1) continue;
+      const int cx = c % g.nx, cy = (c / g.nx) % g.ny, cz = c / (g.nx * g.ny);
+      // with at least 7 cells and none of the five wrapped, candidates are
+      // within 3/7 of a box length: the minimum-image step is the identity
+      const unsigned wrap = (g.nx >= 7 && cx >= 2 && cx < g.nx - 2 ? 0u : 1u) |
+                            (g.ny >= 7 && cy >= 2 && cy < g.ny - 2 ? 0u : 2u) |
+                            (g.nz >= 7 && cz >= 2 && cz < g.nz - 2 ? 0u : 4u);
+      int b0 = 0, l0 = 0, b1 = 0, l1 = 0;  // lane r < 25: row (dz, dy) as one or two runs of places
+      if (lane < kRows) {
+        int z = cz + lane / 5 - 2, y = cy + lane % 5 - 2;
+        z += ((z < 0) - (z >= g.nz)) * g.nz;
+        y += ((y < 0) - (y >= g.ny)) * g.ny;
+        const int row = g.nx * (y + g.ny * z), lo = cx - 2, hi = cx + 2;
+        const int ca = row + (lo < 0 ? lo + g.nx : lo), cb = row + (hi >= g.nx ? hi - g.nx : hi);
+        const bool two = lo < 0 || hi >= g.nx;
+        const int ce = two ? row + g.nx - 1 : cb;  // last cell of the first run
+        b0 = scr->start[ca];
+        l0 = scr->start[ce] + scr->cnt[ce] - b0;
+        if (two) {
+          b1 = scr->start[row];
+          l1 = scr->start[cb] + scr->cnt[cb] - b1;
+        }
+      }
+      const int len = l0 + l1;
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const int off = incl - len, total = __shfl_sync(0xffffffffu, incl, 31);
+      const unsigned ne = __ballot_sync(0xffffffffu, len > 0);
+      __syncwarp();
+      if (len > 0) rowtab[__popc(ne & ((1u << lane) - 1u))] = make_int4(off, b0 - off, off + l0, b1 - off - l0);
+      __syncwarp();
+      for (int p = p0; p < p1; p += 4) {
+        const int m = p1 - p;
+#define CG(K) cell_group<K>(scr, rowtab, off, len, total, p, wrap, s_tab, ntypes, L, iL, force, u, w)
+        if (m >= 3) {
+          if (m >= 4) CG(4);
+          else {
+            CG(2);
+            cell_group<1>(scr, rowtab, off, len, total, p + 2, wrap, s_tab, ntypes, L, iL, force, u, w);
+          }
+        } else if (m == 2) CG(2);
+        else CG(1);
+#undef CG
+      }
+    }
+  } else {
+    const int units = (n + G - 1) / G;
+    for (int k = blockIdx.x * kNoAllocWarps + warp; k < units; k += stride) {
+      const int p = k * G;
+      if (p + G <= n) {
+        all_pairs_group<G>(pos, n, p, s_tab, ntypes, L, iL, force, u, w);
+      } else {
+        for (int r = p; r < n; ++r) all_pairs_group<1>(pos, n, r, s_tab, ntypes, L, iL, force, u, w);
       }
     }
   }
-  if (valid) {
-    const float nanf_ = __int_as_float(0x7fc00000);
-    force[i] = type_ok ? make_float4(fx, fy, fz, 0.5f * uu) : make_float4(nanf_, nanf_, nanf_, nanf_);
-  }
-  // FP64 block sums, then the last block adds the blocks in index order
-  double u = valid && type_ok ? 0.5 * (double)uu : 0.0, w = valid && type_ok ? (double)ww : 0.0;
+  // FP64 block sums; the last block adds the blocks in a fixed order
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     u += __shfl_xor_sync(0xffffffffu, u, o);
     w += __shfl_xor_sync(0xffffffffu, w, o);
   }
-  if ((threadIdx.x & 31) == 0) {
-    s_red[threadIdx.x >> 5][0] = u;
-    s_red[threadIdx.x >> 5][1] = w;
+  if (lane == 0) {
+    s_red[warp][0] = u;
+    s_red[warp][1] = w;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double bu = 0.0, bw = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+    for (int k = 0; k < kNoAllocWarps; ++k) {
       bu += s_red[k][0];
       bw += s_red[k][1];
     }
@@ -138,17 +451,49 @@ __global__ void __launch_bounds__(kNoAllocBlock)
     s_last = atomicAdd(&scr->counter, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (s_last && threadIdx.x == 0) {
-    __threadfence();
-    double su = 0.0, sw = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) {
-      su += __ldcg(&scr->part[b][0]);
-      sw += __ldcg(&scr->part[b][1]);
+  if (!s_last) return;
+  __threadfence();
+  double su = 0.0, sw = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kNoAllocBlock) {
+    su += __ldcg(&scr->part[b][0]);
+    sw += __ldcg(&scr->part[b][1]);
+  }
+  s_red[threadIdx.x][0] = su;
+  s_red[threadIdx.x][1] = sw;
+  __syncthreads();
+  for (int h = kNoAllocBlock / 2; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h) {
+      s_red[threadIdx.x][0] += s_red[threadIdx.x + h][0];
+      s_red[threadIdx.x][1] += s_red[threadIdx.x + h][1];
     }
-    sums[0] = su;        // potential energy, sum of u_i
-    sums[1] = sw / 6.0;  // virial W = sum w_i / 6
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    sums[0] = s_red[0][0];        // potential energy, sum of u_i
+    sums[1] = s_red[0][1] / 6.0;  // virial W = sum w_i / 6
     scr->counter = 0u;
   }
+}
+
+// Cells of half the largest cut-off (5x5x5 then covers it), made larger where
+// there would be more than the scratch holds; false when a dimension has
+// fewer than five, so that the neighbourhood would count a cell twice.
+bool cell_grid(const float* box, float rcmax, Grid3* g) {
+  double nc[3];
+  for (int d = 0; d < 3; ++d) {
+    // a cell is wider than rc/2 by more than the rounding of positions to cells
+    // (2e-7 of a box length, which is at most 1400 cut-offs in cells this small)
+    nc[d] = std::floor(2.0 * (double)box[d] / ((double)rcmax * 1.001));
+    if (!(nc[d] >= 5.0)) return false;
+    nc[d] = std::min(nc[d], 1048576.0);
+  }
+  while (nc[0] * nc[1] * nc[2] > (double)kNoAllocMaxCells) {
+    const int d = nc[0] >= nc[1] && nc[0] >= nc[2] ? 0 : (nc[1] >= nc[2] ? 1 : 2);
+    if (nc[d] <= 5.0) return false;
+    nc[d] = std::max(5.0, std::floor(nc[d] * 0.9));
+  }
+  *g = Grid3{(int)nc[0], (int)nc[1], (int)nc[2]};
+  return true;
 }
 
 // The current CUDA context (driver call cuCtxGetCurrent, fetched through the
@@ -247,11 +592,22 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
     q[2] = p[2];
     q[3] = sf ? sc : 0.f;
     q[4] = sf ? -(sc * rc + uc) : (sp ? -uc : 0.f);
-    q[5] = sf ? sc : 0.f;
+    q[5] = 6.f * p[2];
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the completion counter must start at zero for every call
-  const cudaError_t me = cudaMemsetAsync(&scr->counter, 0, sizeof(unsigned), s);
+  // Cells pay from about 3000 particles (N=2000: 25 us all pairs, 35 cells;
+  // N=4000: 50 and 37) and where a cell's neighbourhood is a third of the box
+  // or less; otherwise every warp tests its particles against all, one
+  // particle per warp while that is what fills the GPU.
+  Grid3 g{1, 1, 1};
+  float reach = 0.f;  // (a pair's range is its cut-off squared, whatever its sign)
+  for (int k = 0; k < ntypes * ntypes; ++k) reach = std::max(reach, fabsf(params[k * 12]));
+  const bool cells = n >= 3000 && cell_grid(box, reach, &g) && g.nx * g.ny * g.nz >= 3 * 125;
+  const int ncell = cells ? g.nx * g.ny * g.nz : 0;
+  // the completion counter and the cell counts must start at zero for every
+  // call (the counts rounded up to whole int4 loads of the scan)
+  const size_t clear = cells ? offsetof(NoAllocScratch, cnt) + ((size_t)ncell + 3) / 4 * 4 * sizeof(int) : sizeof(unsigned);
+  const cudaError_t me = cudaMemsetAsync(scr, 0, clear, s);
   if (me != cudaSuccess) {
     char msg[200];
     snprintf(msg, sizeof(msg), "b2md_forces_noalloc: clearing the scratch counter failed: %s",
@@ -260,9 +616,26 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
   }
   const float3 L = make_float3(box[0], box[1], box[2]);
   const float3 iL = make_float3(1.f / box[0], 1.f / box[1], 1.f / box[2]);
-  const int blocks = (n + kNoAllocBlock - 1) / kNoAllocBlock;
-  k_forces_noalloc<<<blocks, kNoAllocBlock, 0, s>>>(reinterpret_cast<const float4*>(pos4), n, L, iL, ntypes, tab,
-                                                     reinterpret_cast<float4*>(force4), sums, scr);
+  const float4* p4 = reinterpret_cast<const float4*>(pos4);
+  float4* f4 = reinterpret_cast<float4*>(force4);
+  const int tb = (n + 255) / 256;
+#define NA(G, C, UNITS)                                                                                               \
+  k_forces_noalloc<G, C><<<std::min(((UNITS) + kNoAllocWarps - 1) / kNoAllocWarps, kNoAllocMaxBlocks), kNoAllocBlock, \
+                           0, s>>>(p4, n, L, iL, g, ntypes, tab, f4, sums, scr)
+  if (cells) {
+    k_na_count<<<tb, 256, 0, s>>>(p4, n, L, iL, g, scr);
+    k_na_scan<<<1, 1024, 0, s>>>(ncell, scr);
+    k_na_scatter<<<tb, 256, 0, s>>>(n, scr);
+    k_na_gather<<<tb, 256, 0, s>>>(p4, n, L, iL, ntypes, scr);
+    NA(4, true, ncell);
+  } else if (n <= 2400) {
+    NA(1, false, n);
+  } else if (n <= 4800) {
+    NA(2, false, (n + 1) / 2);
+  } else {
+    NA(4, false, (n + 3) / 4);
+  }
+#undef NA
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) {
     char msg[200];

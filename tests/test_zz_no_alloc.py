@@ -78,6 +78,93 @@ def test_noalloc_forces_equal_engine_forces_on_two_calls(cutoff, n, stretch):
         assert abs(s[1] - vir) <= 1e-5 * abs(vir) + 1e-3, (cutoff, call, s[1], vir)
 
 
+def _brute_force(pos4, box, params, cutoff):
+    """FP64 minimum-image pair sum of the valid types: [n, 4] and (U, W)."""
+    r = pos4[:, :3].astype(np.float64)
+    t = pos4[:, 3].view(np.int32)
+    ok = (t >= 0) & (t < 2)
+    p = params.reshape(2, 2, 12).astype(np.float64)
+    L = box.astype(np.float64)
+    out, w = np.zeros((len(r), 4)), 0.0
+    for i in np.flatnonzero(ok):
+        d = r[i] - r
+        d -= L * np.rint(d / L)
+        d2 = (d * d).sum(1)
+        q = p[t[i]][np.where(ok, t, 0)]
+        j = np.flatnonzero((d2 < q[:, 0] ** 2) & ok & (np.arange(len(r)) != i))
+        d, d2, q = d[j], d2[j], q[j]
+        i2, rc, sc, uc = 1.0 / d2, q[:, 0], q[:, 10], q[:, 11]
+        i6 = i2 ** 3
+        s = i6 * i2 * (12.0 * q[:, 1] * i6 + 6.0 * q[:, 2])
+        u = i6 * (q[:, 1] * i6 + q[:, 2])
+        if cutoff == "SF":
+            s, u = s - sc / np.sqrt(d2), u + sc * (np.sqrt(d2) - rc) - uc
+        out[i, :3], out[i, 3] = (d * s[:, None]).sum(0), 0.5 * u.sum()
+        w += (d2 * s).sum()
+    return out, ok, w / 6.0
+
+
+# (particles, box, spread): the last sizes of the one-, two- and four-particle
+# all-pairs forms, the first of the cell form, a box too thin for cells, a
+# cluster that crowds its cells (all pairs again), and positions several box
+# lengths outside
+EDGES = [(2, (9, 9, 9), "all"), (33, (9, 9, 9), "all"), (2400, (13, 13, 13), "all"), (2401, (13, 13, 13), "all"),
+         (2999, (14, 14, 13), "all"), (3000, (14, 14, 13), "all"), (3001, (40, 11, 6.2), "all"),
+         (3100, (15, 13, 17.5), "outside"), (3500, (400, 390, 410), "cluster"), (4801, (36, 36, 6), "all")]
+
+
+@pytest.mark.parametrize("n,lengths,spread", EDGES)
+def test_noalloc_forms_against_fp64_sums(n, lengths, spread):
+    """The form that a size and box select, with particles of unknown type
+    among them (NaN forces, no pairs), against FP64 sums; two calls agree bit
+    for bit.  Bound: the force tolerance of the tests above."""
+    import torch
+    from rumd_b200 import capi, initconf
+    rng = np.random.default_rng(n)
+    box = np.array(lengths, np.float32)
+    ext = np.array((14.0, 14.0, 14.0)) if spread == "cluster" else box.astype(np.float64)
+    if n == 2:
+        ext = np.full(3, 2.0)  # in range of each other
+    m = np.maximum(1, np.ceil(ext * (n / ext.prod()) ** (1 / 3) * 1.08)).astype(int)
+    while m.prod() < n:
+        m[np.argmin(m / ext)] += 1
+    g = np.stack(np.meshgrid(*[np.arange(k) for k in m], indexing="ij"), -1).reshape(-1, 3)
+    sites = g[rng.permutation(len(g))[:n]]
+    pos = (sites + 0.5 + rng.uniform(-0.1, 0.1, (n, 3))) * (ext / m) - ext / 2
+    if spread == "outside":
+        pos += rng.integers(-2, 3, (n, 3)) * box
+    types = (rng.random(n) < 0.2).astype(np.int32)
+    if n == 2:
+        types[:] = 0
+    if n > 100:
+        types[rng.integers(0, n, 3)] = [2, -1, 77]
+    pos4 = np.zeros((n, 4), np.float32)
+    pos4[:, :3] = pos
+    pos4[:, 3] = types.view(np.float32)
+    params = np.ascontiguousarray(initconf.lj_params(2, initconf.KA), np.float32)
+    ref, ok, W = _brute_force(pos4, box, params, "SF")
+    lib = capi.lib()
+    dev = torch.device("cuda:0")
+    p = torch.from_numpy(pos4).to(dev)
+    got = []
+    for _ in range(2):
+        force = torch.zeros((n, 4), dtype=torch.float32, device=dev)
+        sums = torch.zeros(2, dtype=torch.float64, device=dev)
+        rc = _call(lib, ctypes.c_void_p(p.data_ptr()), n, box, params, capi.CUTOFF["SF"],
+                   ctypes.c_void_p(force.data_ptr()), ctypes.c_void_p(sums.data_ptr()),
+                   ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+        assert rc == capi.B2MD_OK, lib.b2md_last_error()
+        torch.cuda.synchronize(dev)
+        got.append((force.cpu().numpy(), sums.cpu().numpy()))
+    assert np.array_equal(got[0][0], got[1][0], equal_nan=True) and np.array_equal(got[0][1], got[1][1])
+    f, s = got[0]
+    assert np.isnan(f[~ok]).all() and np.isfinite(f[ok]).all()
+    err = np.linalg.norm(f[ok, :3] - ref[ok, :3]) / np.linalg.norm(ref[ok, :3])
+    assert err <= 1e-5, err
+    assert abs(s[0] - ref[ok, 3].sum()) <= 1e-5 * np.abs(ref[ok, 3]).sum()
+    assert abs(s[1] - W) <= 1e-5 * np.abs(ref[ok, :3]).sum()
+
+
 def test_noalloc_rejects_sizes_beyond_its_maximum():
     from rumd_b200 import capi
     lib = capi.lib()
