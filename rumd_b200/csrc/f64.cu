@@ -23,11 +23,22 @@
 // recomputed here in FP64 from them, as the double build's CopyParamsToGPU
 // (PairPotential.cu:82-125) would.
 //
-// Layout: particles stay in the caller's order (no spatial sort).  Cells are
-// at least rc_max + skin wide (27-cell stencil); boxes with fewer than three
-// cells along a side use all pairs.  Within a cell, particles are listed in
-// ascending index, so lists and sums are deterministic.  All sums are FP64
-// with a fixed tree (block partials added in block order).
+// Layout: at every list build the particles are sorted by (cell, place), so
+// that a warp's neighbours share cache lines; uid holds each place's particle
+// in the caller's order, which get and set use.  Cells are at least
+// rc_max + skin wide (27-cell stencil); boxes with fewer than three cells
+// along a side use all pairs.  Lists and sums have a fixed order: runs are
+// deterministic.  All sums are FP64 with a fixed tree (block partials added in
+// block order).
+//
+// A step is three launches: the list build (one cooperative kernel that
+// returns at once unless a build is due), the forces, and the integration
+// with the step's totals.  What bounds a step is the latency of dependent
+// FP64 arithmetic and of the neighbour gathers, so 4 to 32 lanes share a
+// particle, the more the fewer particles there are.  One thread per particle,
+// in the caller's order, with ten launches a step took 191 us per step at LJ
+// N=32000.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -44,7 +55,8 @@ namespace {
 
 constexpr int kB = 256;        // threads per block
 constexpr int kMaxT = 16;      // particle types
-constexpr int kNPartF64 = 4;   // per-block partials: pe, w, ke_t, ke2
+constexpr int kNPartF64 = 4;   // per-block partials of the momentum: P, M
+constexpr unsigned kPolls = 1u << 22;  // grid-barrier polls before a wait gives up
 
 struct F64Pair {
   double rc, rc2, a12, a6, cs, cu, nb2;  // cs = s(rc) rc, cu = u(rc), nb2 = (rc + skin)^2
@@ -54,22 +66,31 @@ struct F64Dev {  // device-resident scalars
   double xi, P[3], M, pe, W, ke_t, ke2;
   long long rebuilds, steps;
   int need, overflow;
+  unsigned arrive, gen;  // grid barrier of the list build
+  unsigned done;         // blocks of the list build / integration finished
+  int err;               // a grid-barrier wait gave up
 };
 
 struct F64Args {
-  int n, ntypes, cutoff, max_nbrs, ncell, allpairs, thermo;
+  int n, ntypes, cutoff, max_nbrs, ncell, allpairs, thermo, fblocks;
   int nc[3];
-  double L[3], invL[3], dt, skin2_4, T, omega2, dof;
+  double L[3], invL[3], ilim[3], dt, skin2_4, T, omega2, dof;
   double4 *r, *v, *f, *last_r;
-  int4* im;
-  int *cell, *cnt, *cstart, *cfill, *cidx;
-  unsigned *nn, *nbl;
-  double* part;
+  int4 *im, *im2;          // (im2, uid2: the sort's copies; f and last_r serve for r and v)
+  unsigned *uid, *uid2;    // the caller's particle of each place
+  int *cell, *rank, *order, *cnt, *cstart, *ctot;
+  unsigned *nn, *nbl;      // entry k of place i at nbl[((k / 4) n + i) 4 + k % 4]
+  double *part, *part_f;   // per-block sums of the integration (and momentum); of the forces
   F64Dev* st;
   const F64Pair* par;
 };
 
-__device__ __forceinline__ double mi64(double d, double L, double iL) { return d - L * rint(d * iL); }
+// d - L rint(d / L); adding and subtracting 1.5 2^52 rounds |x| < 2^51 to an
+// integer, ties to even, in two additions.
+__device__ __forceinline__ double mi64(double d, double L, double iL) {
+  const double M = 6755399441055744.0;
+  return d - L * __dsub_rn(__dadd_rn(d * iL, M), M);
+}
 
 __device__ __forceinline__ int type_of(const double4& r) { return (int)r.w; }
 
@@ -94,18 +115,17 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* s_warp, double
   __syncthreads();
 }
 
-// Sums partial columns [k0, k0+K) over `nblocks` rows of part (row stride
-// kNPartF64) in a fixed order: thread t adds rows t, t+kB, ...; then the
-// block adds the threads in order.
+// Sums the K columns of `nblocks` rows of partials (row stride K) in a fixed
+// order: thread t adds rows t, t+kB, ...; then the block adds the threads in
+// order.  Read past L1: other blocks of the same launch may have written them.
 template <int K>
-__device__ __forceinline__ void sum_partials(const F64Args& a, int nblocks, int k0, double* s_out) {
-  __shared__ double s_warp[(kB / 32) * K];
+__device__ __forceinline__ void sum_partials(const double* part, int nblocks, double* s_warp, double* s_out) {
   double v[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) v[k] = 0.0;
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += a.part[(size_t)b * kNPartF64 + k0 + k];
+    for (int k = 0; k < K; ++k) v[k] += __ldcg(part + (size_t)b * K + k);
   block_sum<K>(v, s_warp, s_out);
 }
 
@@ -124,8 +144,8 @@ __global__ void __launch_bounds__(kB) k64_momentum_part(F64Args a) {
 }
 
 __global__ void __launch_bounds__(kB) k64_momentum_total(F64Args a, int nblocks) {
-  __shared__ double s_out[4];
-  sum_partials<4>(a, nblocks, 0, s_out);
+  __shared__ double s_warp[(kB / 32) * 4], s_out[4];
+  sum_partials<4>(a.part, nblocks, s_warp, s_out);
   if (threadIdx.x == 0) {
     a.st->P[0] = s_out[0]; a.st->P[1] = s_out[1]; a.st->P[2] = s_out[2]; a.st->M = s_out[3];
   }
@@ -152,158 +172,260 @@ __device__ __forceinline__ int cell_of(const F64Args& a, const double4& r) {
   return c[0] + a.nc[0] * (c[1] + a.nc[1] * c[2]);
 }
 
-__global__ void __launch_bounds__(kB) k64_rb_clear(F64Args a) {
-  if (!a.st->need || a.allpairs) return;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.ncell; c += gridDim.x * blockDim.x) a.cnt[c] = 0;
-}
-
-__global__ void __launch_bounds__(kB) k64_rb_count(F64Args a) {
-  if (!a.st->need || a.allpairs) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const int c = cell_of(a, a.r[i]);
-  a.cell[i] = c;
-  atomicAdd(&a.cnt[c], 1);
-}
-
-// exclusive scan of the cell counts by one block: each thread scans a
-// contiguous chunk, the chunk totals are scanned in shared memory
-__global__ void __launch_bounds__(1024) k64_rb_scan(F64Args a) {
-  if (!a.st->need || a.allpairs) return;
-  __shared__ int s_tot[1024];
-  const int chunk = (a.ncell + blockDim.x - 1) / blockDim.x;
-  const int b = threadIdx.x * chunk, e = min(a.ncell, b + chunk);
-  int s = 0;
-  for (int c = b; c < e; ++c) s += a.cnt[c];
-  s_tot[threadIdx.x] = s;
+// Grid barrier of the list build (every block resident: cooperative launch);
+// false, in every thread, when the wait gave up.
+__device__ bool grid_barrier(F64Dev* st) {
+  __shared__ int s_ok;
   __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-    const int t = threadIdx.x >= (unsigned)o ? s_tot[threadIdx.x - o] : 0;
-    __syncthreads();
-    s_tot[threadIdx.x] += t;
-    __syncthreads();
-  }
-  int run = s_tot[threadIdx.x] - s;  // exclusive prefix of this chunk
-  for (int c = b; c < e; ++c) {
-    a.cstart[c] = run;
-    a.cfill[c] = run;
-    run += a.cnt[c];
-  }
-}
-
-__global__ void __launch_bounds__(kB) k64_rb_fill(F64Args a) {
-  if (!a.st->need || a.allpairs) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  a.cidx[atomicAdd(&a.cfill[a.cell[i]], 1)] = i;
-}
-
-// particles of each cell in ascending index (insertion sort; a few per cell)
-__global__ void __launch_bounds__(kB) k64_rb_sort(F64Args a) {
-  if (!a.st->need || a.allpairs) return;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < a.ncell; c += gridDim.x * blockDim.x) {
-    int* p = a.cidx + a.cstart[c];
-    const int m = a.cnt[c];
-    for (int k = 1; k < m; ++k) {
-      const int x = p[k];
-      int q = k - 1;
-      while (q >= 0 && p[q] > x) {
-        p[q + 1] = p[q];
-        --q;
+  if (threadIdx.x == 0) {
+    s_ok = 1;
+    volatile unsigned* gen = &st->gen;
+    const unsigned g = *gen;
+    __threadfence();
+    if (atomicAdd(&st->arrive, 1u) == gridDim.x - 1) {
+      st->arrive = 0u;
+      __threadfence();
+      *gen = g + 1u;
+    } else {
+      unsigned it = 0;
+      while (*gen == g && it < kPolls) {
+        __nanosleep(32);
+        ++it;
       }
-      p[q + 1] = x;
+      if (it >= kPolls) {
+        atomicExch(&st->err, 1);
+        s_ok = 0;
+      }
     }
+    __threadfence();
   }
+  __syncthreads();
+  return s_ok != 0;
 }
 
-__global__ void __launch_bounds__(kB) k64_rb_build(F64Args a) {
-  if (!a.st->need) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const double4 ri = a.r[i];
-  const F64Pair* row = a.par + type_of(ri) * a.ntypes;
-  unsigned count = 0;
-  auto test = [&](int j) {
-    if (j == i) return;
-    const double4 rj = a.r[j];
-    const double dx = mi64(ri.x - rj.x, a.L[0], a.invL[0]);
-    const double dy = mi64(ri.y - rj.y, a.L[1], a.invL[1]);
-    const double dz = mi64(ri.z - rj.z, a.L[2], a.invL[2]);
-    if (dx * dx + dy * dy + dz * dz < row[type_of(rj)].nb2) {
-      if ((int)count < a.max_nbrs) a.nbl[(size_t)count * a.n + i] = (unsigned)j;
-      ++count;
-    }
-  };
-  if (a.allpairs) {
-    for (int j = 0; j < a.n; ++j) test(j);
-  } else {
-    const int c = a.cell[i];
-    const int cx = c % a.nc[0], cy = (c / a.nc[0]) % a.nc[1], cz = c / (a.nc[0] * a.nc[1]);
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int ox = (cx + dx + a.nc[0]) % a.nc[0], oy = (cy + dy + a.nc[1]) % a.nc[1];
-          const int oz = (cz + dz + a.nc[2]) % a.nc[2];
-          const int o = ox + a.nc[0] * (oy + a.nc[1] * oz);
-          const int b = a.cstart[o], e = b + a.cnt[o];
-          for (int s = b; s < e; ++s) test(a.cidx[s]);
-        }
-  }
-  a.nn[i] = min(count, (unsigned)a.max_nbrs);
-  if ((int)count > a.max_nbrs) a.st->overflow = 1;
-  a.last_r[i] = ri;
-}
-
-__global__ void k64_rb_done(F64Args a) {
-  if (a.st->need) {
-    a.st->need = 0;
-    a.st->rebuilds += 1;
-  }
-}
-
-// ---- 3. pair forces ----
-__global__ void __launch_bounds__(kB) k64_forces(F64Args a) {
-  __shared__ double s_warp[(kB / 32) * 2], s_out[2];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double acc[2] = {0.0, 0.0};
-  if (i < a.n) {
-    const double4 ri = a.r[i];
-    const F64Pair* row = a.par + type_of(ri) * a.ntypes;
-    double fx = 0.0, fy = 0.0, fz = 0.0, u = 0.0, w = 0.0;
-    const unsigned nn = a.nn[i];
-    for (unsigned k = 0; k < nn; ++k) {
-      const double4 rj = a.r[a.nbl[(size_t)k * a.n + i]];
+// Appends the accepted candidates [b, e) (places) of particle i to its list;
+// the particle's 8 lanes test 8 consecutive ones a round, in order.  All lanes
+// of the warp call it (others with an empty range).
+__device__ __forceinline__ unsigned list_run(const F64Args& a, int i, const double4& ri, const F64Pair* row, int b,
+                                             int e, unsigned count) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u, l8 = lane & 7u, shift = lane & 24u;
+  const int rounds = __reduce_max_sync(FULL, e > b ? (e - b + 7) >> 3 : 0);
+  for (int k = 0; k < rounds; ++k) {
+    const int j = b + 8 * k + (int)l8;
+    bool in = false;
+    if (j < e && j != i) {
+      const double4 rj = a.r[j];
       const double dx = mi64(ri.x - rj.x, a.L[0], a.invL[0]);
       const double dy = mi64(ri.y - rj.y, a.L[1], a.invL[1]);
       const double dz = mi64(ri.z - rj.z, a.L[2], a.invL[2]);
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      const F64Pair& p = row[type_of(rj)];
-      if (d2 < p.rc2) {
-        const double i2 = 1.0 / d2, i6 = i2 * i2 * i2, t = p.a12 * i6;
-        double s = i6 * i2 * (12.0 * t + 6.0 * p.a6);
-        double uu = i6 * (t + p.a6);
-        if (a.cutoff == B2MD_CUTOFF_SF) {
-          const double r = sqrt(d2);
-          s -= p.cs / r;
-          uu += p.cs * (r - p.rc) - p.cu;
-        } else if (a.cutoff == B2MD_CUTOFF_SP) {
-          uu -= p.cu;
+      in = dx * dx + dy * dy + dz * dz < row[type_of(rj)].nb2;
+    }
+    const unsigned m = (__ballot_sync(FULL, in) >> shift) & 0xffu;
+    if (in) {
+      const unsigned pos = count + __popc(m & ((1u << l8) - 1u));
+      if (pos < (unsigned)a.max_nbrs) a.nbl[((size_t)(pos >> 2) * a.n + i) * 4 + (pos & 3u)] = (unsigned)j;
+    }
+    count += __popc(m);
+  }
+  return count;
+}
+
+// The list build: one cooperative launch whose blocks meet between the phases
+// of the sort; it returns at once unless a build is due.
+__global__ void __launch_bounds__(kB) k64_rebuild(F64Args a) {
+  F64Dev* st = a.st;
+  if (!st->need || st->err) return;
+  __shared__ int s_w[kB / 32 + 1];
+  const int tid = threadIdx.x, gid = blockIdx.x * blockDim.x + tid, gsz = gridDim.x * blockDim.x;
+  const int lane = tid & 31, wid = tid >> 5;
+  for (int c = gid; c < a.ncell; c += gsz) a.cnt[c] = 0;
+  if (!grid_barrier(st)) return;  // (also: every block has seen that a build is due)
+  if (!a.allpairs) {
+    for (int i = gid; i < a.n; i += gsz) {
+      const int c = cell_of(a, a.r[i]);
+      a.cell[i] = c;
+      a.rank[i] = atomicAdd(&a.cnt[c], 1);
+    }
+    if (!grid_barrier(st)) return;
+    // exclusive scan of the counts: block b owns a run of cells; first the
+    // runs' totals, then every block adds the totals before its own
+    const int run = (a.ncell + gridDim.x - 1) / gridDim.x;
+    const int c0 = min(a.ncell, (int)blockIdx.x * run), c1 = min(a.ncell, c0 + run);
+    auto block_total = [&](int x) -> int {
+      x = __reduce_add_sync(0xffffffffu, x);
+      __syncthreads();
+      if (lane == 0) s_w[wid] = x;
+      __syncthreads();
+      int t = 0;
+      for (int w = 0; w < kB / 32; ++w) t += s_w[w];
+      return t;
+    };
+    {
+      int x = 0;
+      for (int c = c0 + tid; c < c1; c += kB) x += __ldcg(a.cnt + c);
+      x = block_total(x);
+      if (tid == 0) a.ctot[blockIdx.x] = x;
+    }
+    if (!grid_barrier(st)) return;
+    {
+      int x = 0;
+      for (int b = tid; b < (int)blockIdx.x; b += kB) x += __ldcg(a.ctot + b);
+      int first = block_total(x);
+      for (int cb = c0; cb < c1; cb += kB) {
+        const int c = cb + tid;
+        const int m = c < c1 ? __ldcg(a.cnt + c) : 0;
+        int incl = m;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
         }
-        fx += dx * s; fy += dy * s; fz += dz * s;
-        u += uu; w += d2 * s;
+        __syncthreads();
+        if (lane == 31) s_w[wid] = incl;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < kB / 32; ++w) {
+          if (w < wid) before += s_w[w];
+          all += s_w[w];
+        }
+        if (c < c1) a.cstart[c] = first + before + incl - m;
+        first += all;
       }
     }
+    if (!grid_barrier(st)) return;
+    for (int i = gid; i < a.n; i += gsz) a.order[__ldcg(a.cstart + a.cell[i]) + a.rank[i]] = i;
+    if (!grid_barrier(st)) return;
+    // each bucket by place (members counted against each other), state copied
+    // in that order
+    for (int s = gid; s < a.n; s += gsz) {
+      const int i = __ldcg(a.order + s), c = __ldcg(a.cell + i), b = __ldcg(a.cstart + c), m = __ldcg(a.cnt + c);
+      int place = b;
+      for (int k = 0; k < m; ++k) place += __ldcg(a.order + b + k) < i;
+      a.f[place] = a.r[i];
+      a.last_r[place] = a.v[i];
+      a.im2[place] = a.im[i];
+      a.uid2[place] = a.uid[i];
+    }
+    if (!grid_barrier(st)) return;
+    for (int i = gid; i < a.n; i += gsz) {
+      const double4 r = a.f[i];
+      a.v[i] = a.last_r[i];
+      a.r[i] = r;
+      a.last_r[i] = r;
+      a.im[i] = a.im2[i];
+      a.uid[i] = a.uid2[i];
+    }
+    if (!grid_barrier(st)) return;
+  } else {
+    for (int i = gid; i < a.n; i += gsz) a.last_r[i] = a.r[i];
+  }
+  // the lists: 8 lanes per particle, four particles per warp
+  const int nwarps = gsz >> 5;
+  for (int i0 = (gid >> 5) * 4; i0 < a.n; i0 += nwarps * 4) {
+    const int i = i0 + (lane >> 3);
+    const bool valid = i < a.n;
+    const double4 ri = a.r[valid ? i : 0];
+    const F64Pair* row = a.par + type_of(ri) * a.ntypes;
+    unsigned count = 0;
+    if (a.allpairs) {
+      count = list_run(a, i, ri, row, 0, valid ? a.n : 0, count);
+    } else {
+      const int c = cell_of(a, ri);
+      const int cx = c % a.nc[0], cy = (c / a.nc[0]) % a.nc[1], cz = c / (a.nc[0] * a.nc[1]);
+      for (int k = 0; k < 9; ++k) {
+        const int oy = (cy + k % 3 - 1 + a.nc[1]) % a.nc[1], oz = (cz + k / 3 - 1 + a.nc[2]) % a.nc[2];
+        const int base = a.nc[0] * (oy + a.nc[1] * oz);
+        // x cells cx-1 .. cx+1: one run of places, or two when the row wraps
+        const int lo = max(cx - 1, 0), hi = min(cx + 1, a.nc[0] - 1);
+        const int b = a.cstart[base + lo], e = a.cstart[base + hi] + a.cnt[base + hi];
+        count = list_run(a, i, ri, row, b, valid ? e : b, count);
+        const int o = cx == 0 ? base + a.nc[0] - 1 : base;  // the wrapped cell
+        const bool two = valid && (cx == 0 || cx == a.nc[0] - 1);
+        count = list_run(a, i, ri, row, two ? a.cstart[o] : 0, two ? a.cstart[o] + a.cnt[o] : 0, count);
+      }
+    }
+    if (valid && (lane & 7) == 0) {
+      a.nn[i] = min(count, (unsigned)a.max_nbrs);
+      if ((int)count > a.max_nbrs) st->overflow = 1;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(&st->done, 1u) == gridDim.x - 1) {
+      st->done = 0u;
+      st->need = 0;
+      st->rebuilds += 1;
+    }
+  }
+}
+
+// ---- 3. pair forces: TP lanes per particle, lane t takes entries t, t + TP, ... ----
+template <int TP>
+__global__ void __launch_bounds__(kB) k64_forces(F64Args a) {
+  __shared__ double s_warp[(kB / 32) * 2], s_out[2];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / TP, t = threadIdx.x % TP;
+  const bool valid = i < a.n;
+  const double4 ri = a.r[valid ? i : 0];
+  const F64Pair* row = a.par + type_of(ri) * a.ntypes;
+  // a particle farther than rc_max + 2 skin from both faces of a dimension has
+  // its listed neighbours at their minimum image in it
+  const bool wx = __any_sync(FULL, !(fabs(ri.x) < a.ilim[0])), wy = __any_sync(FULL, !(fabs(ri.y) < a.ilim[1])),
+             wz = __any_sync(FULL, !(fabs(ri.z) < a.ilim[2]));
+  double fx = 0.0, fy = 0.0, fz = 0.0, u = 0.0, w = 0.0;
+  const unsigned nn = valid ? a.nn[i] : 0u;
+  const unsigned* list = a.nbl + (size_t)i * 4;
+  auto entry = [&](unsigned k) { return k < nn ? __ldg(list + (size_t)(k >> 2) * a.n * 4 + (k & 3u)) : 0u; };
+  unsigned j = entry(t);
+  for (unsigned k = t; k < nn; k += TP) {
+    const double4 rj = a.r[j];
+    j = entry(k + TP);
+    double dx = ri.x - rj.x, dy = ri.y - rj.y, dz = ri.z - rj.z;
+    if (wx) dx = mi64(dx, a.L[0], a.invL[0]);
+    if (wy) dy = mi64(dy, a.L[1], a.invL[1]);
+    if (wz) dz = mi64(dz, a.L[2], a.invL[2]);
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    const F64Pair& p = row[type_of(rj)];
+    if (d2 < p.rc2) {
+      const double i2 = 1.0 / d2, i6 = i2 * i2 * i2, q = p.a12 * i6;
+      double s = i6 * i2 * (12.0 * q + 6.0 * p.a6);
+      double uu = i6 * (q + p.a6);
+      if (a.cutoff == B2MD_CUTOFF_SF) {
+        const double y = rsqrt(d2);
+        s -= p.cs * y;
+        uu += p.cs * (d2 * y - p.rc) - p.cu;
+      } else if (a.cutoff == B2MD_CUTOFF_SP) {
+        uu -= p.cu;
+      }
+      fx += dx * s; fy += dy * s; fz += dz * s;
+      u += uu; w += d2 * s;
+    }
+  }
+#pragma unroll
+  for (int o = TP / 2; o > 0; o >>= 1) {
+    fx += __shfl_xor_sync(FULL, fx, o);
+    fy += __shfl_xor_sync(FULL, fy, o);
+    fz += __shfl_xor_sync(FULL, fz, o);
+    u += __shfl_xor_sync(FULL, u, o);
+    w += __shfl_xor_sync(FULL, w, o);
+  }
+  double acc[2] = {0.0, 0.0};
+  if (valid && t == 0) {
     a.f[i] = make_double4(fx, fy, fz, 0.5 * u);
     acc[0] = 0.5 * u;
     acc[1] = w;
   }
   block_sum<2>(acc, s_warp, s_out);
-  if (threadIdx.x < 2) a.part[(size_t)blockIdx.x * kNPartF64 + threadIdx.x] = s_out[threadIdx.x];
+  if (threadIdx.x < 2) a.part_f[(size_t)blockIdx.x * 2 + threadIdx.x] = s_out[threadIdx.x];
 }
 
-// ---- 4. Nose-Hoover leap-frog ----
-__global__ void __launch_bounds__(kB) k64_integrate(F64Args a) {
-  __shared__ double s_warp[(kB / 32) * 2], s_out[2];
+// ---- 4. Nose-Hoover leap-frog; the last block adds up the step: totals,
+// thermostat, energy log ----
+__global__ void __launch_bounds__(kB) k64_integrate(F64Args a, double* elog) {
+  __shared__ double s_warp[(kB / 32) * 2], s_out[2], s_for[2];
+  __shared__ int s_last;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[2] = {0.0, 0.0};
   if (i < a.n) {
@@ -331,22 +453,26 @@ __global__ void __launch_bounds__(kB) k64_integrate(F64Args a) {
     if (ex * ex + ey * ey + ez * ez > a.skin2_4) a.st->need = 1;
   }
   block_sum<2>(acc, s_warp, s_out);
-  if (threadIdx.x < 2) a.part[(size_t)blockIdx.x * kNPartF64 + 2 + threadIdx.x] = s_out[threadIdx.x];
-}
-
-// ---- 5. totals, thermostat, energy log ----
-__global__ void __launch_bounds__(kB) k64_finish(F64Args a, int nblocks, int integrated, double* elog) {
-  __shared__ double s_out[4];
-  sum_partials<4>(a, nblocks, 0, s_out);
+  if (threadIdx.x < 2) a.part[(size_t)blockIdx.x * 2 + threadIdx.x] = s_out[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.st->done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  sum_partials<2>(a.part_f, a.fblocks, s_warp, s_for);
+  sum_partials<2>(a.part, gridDim.x, s_warp, s_out);
   if (threadIdx.x != 0) return;
   F64Dev* S = a.st;
-  S->pe = s_out[0];
-  S->W = s_out[1] / 6.0;
-  if (!integrated) return;
-  S->ke_t = s_out[2];
-  S->ke2 = s_out[3];
+  S->done = 0u;
+  S->pe = s_for[0];
+  S->W = s_for[1] / 6.0;
+  S->ke_t = s_out[0];
+  S->ke2 = s_out[1];
   if (a.thermo) {
-    double dev = s_out[3] / (a.dof * a.T) - 1.0;
+    double dev = s_out[1] / (a.dof * a.T) - 1.0;
     if (dev > 10.0) dev = 10.0;
     S->xi += a.dt * a.omega2 * dev;
   }
@@ -359,6 +485,20 @@ __global__ void __launch_bounds__(kB) k64_finish(F64Args a, int nblocks, int int
   }
 }
 
+// ---- 5. the force evaluation's totals alone (b2md_f64_calc_f) ----
+__global__ void __launch_bounds__(kB) k64_finish(F64Args a) {
+  __shared__ double s_warp[(kB / 32) * 2], s_out[2];
+  sum_partials<2>(a.part_f, a.fblocks, s_warp, s_out);
+  if (threadIdx.x != 0) return;
+  a.st->pe = s_out[0];
+  a.st->W = s_out[1] / 6.0;
+}
+
+__global__ void __launch_bounds__(kB) k64_iota(unsigned* ids, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) ids[i] = (unsigned)i;
+}
+
 }  // namespace
 
 struct b2md_f64 {
@@ -369,6 +509,10 @@ struct b2md_f64 {
   F64Pair* par = nullptr;
   int reset_interval = 100;
   bool have_state = false;
+  int tp = 4;           // lanes per particle of the force kernel
+  int rb_grid = 1;      // blocks of the list build, all resident at once
+  double* elog = nullptr;  // energies of a run, kept for the next
+  long long elog_cap = 0;
   std::vector<void*> bufs;
 };
 
@@ -407,19 +551,17 @@ int f64_alloc(b2md_f64* h, T*& p, size_t count) {
 
 int nblocks(const b2md_f64* h) { return (h->a.n + kB - 1) / kB; }
 
-// step 2 + 3: list (when due) and forces; the launches of one step
+// step 2 + 3: list (when due) and forces
 int launch_forces(b2md_f64* h) {
-  const F64Args& a = h->a;
-  const int B = nblocks(h), s_cells = std::max(1, std::min((a.ncell + kB - 1) / kB, 4096));
+  F64Args a = h->a;
   cudaStream_t s = h->stream;
-  k64_rb_clear<<<s_cells, kB, 0, s>>>(a);
-  k64_rb_count<<<B, kB, 0, s>>>(a);
-  k64_rb_scan<<<1, 1024, 0, s>>>(a);
-  k64_rb_fill<<<B, kB, 0, s>>>(a);
-  k64_rb_sort<<<s_cells, kB, 0, s>>>(a);
-  k64_rb_build<<<B, kB, 0, s>>>(a);
-  k64_rb_done<<<1, 1, 0, s>>>(a);
-  k64_forces<<<B, kB, 0, s>>>(a);
+  void* args[] = {&a};
+  F64_CK(cudaLaunchCooperativeKernel((const void*)k64_rebuild, dim3(h->rb_grid), dim3(kB), args, 0, s));
+  switch (h->tp) {
+    case 32: k64_forces<32><<<a.fblocks, kB, 0, s>>>(a); break;
+    case 8: k64_forces<8><<<a.fblocks, kB, 0, s>>>(a); break;
+    default: k64_forces<4><<<a.fblocks, kB, 0, s>>>(a); break;
+  }
   F64_CK(cudaGetLastError());
   return B2MD_OK;
 }
@@ -434,6 +576,7 @@ int check_overflow(b2md_f64* h) {
   F64Dev d;
   int rc = read_dev(h, &d);
   if (rc) return rc;
+  if (d.err) return f64_fail(B2MD_ERR_CUDA, "b2md_f64: a grid-barrier wait of the list build gave up");
   if (d.overflow)
     return f64_fail(B2MD_ERR_OVERFLOW, "b2md_f64: a particle has more than %d neighbours within rc + skin; "
                                        "the run is invalid (create the engine with a larger max_nbrs)",
@@ -483,7 +626,11 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
     a.nc[d] = (int)std::floor(box3[d] / (rc_max + skin));
     if (a.nc[d] < 3) a.allpairs = 1;
     a.ncell *= std::max(a.nc[d], 1);
+    a.ilim[d] = 0.5 * box3[d] - (rc_max + 2.0 * skin) - 1e-9 * box3[d];
   }
+  // lanes per particle: about as many threads as the GPU holds
+  h->tp = n < 8192 ? 32 : n < 65536 ? 8 : 4;
+  a.fblocks = (int)(((long long)n * h->tp + kB - 1) / kB);
   const double vol = box3[0] * box3[1] * box3[2];
   const double est = n / vol * 4.0 / 3.0 * M_PI * std::pow(rc_max + skin, 3.0);
   a.max_nbrs = max_nbrs > 0 ? max_nbrs : (int)std::min<double>(n - 1, 1.6 * est + 32.0);
@@ -499,12 +646,21 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
   if (cudaSetDevice(device) != cudaSuccess) return done(f64_fail(B2MD_ERR_CUDA, "b2md_f64_create: bad device %d", device));
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
     return done(f64_fail(B2MD_ERR_CUDA, "b2md_f64_create: stream creation failed"));
-  const size_t nb = (size_t)((n + kB - 1) / kB);
+  int sms = 0, per_sm = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k64_rebuild, kB, 0) != cudaSuccess || per_sm < 1)
+    return done(f64_fail(B2MD_ERR_CUDA, "b2md_f64_create: the list build does not fit on the device"));
+  // the list build's blocks: enough for 8 lanes per particle, two per SM at
+  // most (its barriers cost more the more blocks meet)
+  h->rb_grid = (int)std::max(1LL, std::min((long long)sms * std::min(per_sm, 2), (8LL * n + kB - 1) / kB));
+  const size_t nb = (size_t)((n + kB - 1) / kB), rows = ((size_t)a.max_nbrs + 3) / 4 * 4;
   if ((rc = f64_alloc(h, a.r, n)) || (rc = f64_alloc(h, a.v, n)) || (rc = f64_alloc(h, a.f, n)) ||
-      (rc = f64_alloc(h, a.last_r, n)) || (rc = f64_alloc(h, a.im, n)) || (rc = f64_alloc(h, a.cell, n)) ||
-      (rc = f64_alloc(h, a.cnt, a.ncell)) || (rc = f64_alloc(h, a.cstart, a.ncell)) ||
-      (rc = f64_alloc(h, a.cfill, a.ncell)) || (rc = f64_alloc(h, a.cidx, n)) || (rc = f64_alloc(h, a.nn, n)) ||
-      (rc = f64_alloc(h, a.nbl, (size_t)a.max_nbrs * n)) || (rc = f64_alloc(h, a.part, nb * kNPartF64)) ||
+      (rc = f64_alloc(h, a.last_r, n)) || (rc = f64_alloc(h, a.im, n)) || (rc = f64_alloc(h, a.im2, n)) ||
+      (rc = f64_alloc(h, a.uid, n)) || (rc = f64_alloc(h, a.uid2, n)) || (rc = f64_alloc(h, a.cell, n)) ||
+      (rc = f64_alloc(h, a.rank, n)) || (rc = f64_alloc(h, a.order, n)) || (rc = f64_alloc(h, a.cnt, a.ncell)) ||
+      (rc = f64_alloc(h, a.cstart, a.ncell)) || (rc = f64_alloc(h, a.ctot, h->rb_grid)) ||
+      (rc = f64_alloc(h, a.nn, n)) || (rc = f64_alloc(h, a.nbl, rows * n)) ||
+      (rc = f64_alloc(h, a.part, nb * kNPartF64)) || (rc = f64_alloc(h, a.part_f, (size_t)a.fblocks * 2)) ||
       (rc = f64_alloc(h, h->st, 1)) || (rc = f64_alloc(h, h->par, pars.size())))
     return done(rc);
   a.st = h->st;
@@ -523,6 +679,7 @@ int b2md_f64_destroy(b2md_f64* h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->bufs) cudaFree(p);
+  if (h->elog) cudaFree(h->elog);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return B2MD_OK;
@@ -547,6 +704,8 @@ int b2md_f64_set_state(b2md_f64* h, const double* pos4, const double* vel4, cons
   F64_CK(cudaMemcpyAsync(h->a.r, r.data(), n * sizeof(double4), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaMemcpyAsync(h->a.v, v.data(), n * sizeof(double4), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaMemcpyAsync(h->a.im, im.data(), n * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
+  k64_iota<<<nblocks(h), kB, 0, h->stream>>>(h->a.uid, n);
+  F64_CK(cudaGetLastError());
   const int one = 1;
   F64_CK(cudaMemcpyAsync(&h->st->need, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaStreamSynchronize(h->stream));
@@ -583,7 +742,7 @@ int b2md_f64_calc_f(b2md_f64* h) {
   F64_CK(cudaSetDevice(h->device));
   int rc = launch_forces(h);
   if (rc) return rc;
-  k64_finish<<<1, kB, 0, h->stream>>>(h->a, nblocks(h), 0, nullptr);
+  k64_finish<<<1, kB, 0, h->stream>>>(h->a);
   F64_CK(cudaGetLastError());
   return check_overflow(h);
 }
@@ -594,7 +753,17 @@ int b2md_f64_run(b2md_f64* h, long long nsteps, double* energies) {
   if (!h->have_state) return f64_fail(B2MD_ERR_STATE, "b2md_f64_run: no state set");
   F64_CK(cudaSetDevice(h->device));
   double* d_log = nullptr;
-  if (energies && nsteps > 0) F64_CK(cudaMalloc(&d_log, (size_t)nsteps * 4 * sizeof(double)));
+  if (energies && nsteps > 0) {
+    if (nsteps > h->elog_cap) {
+      F64_CK(cudaStreamSynchronize(h->stream));
+      if (h->elog) cudaFree(h->elog);
+      h->elog = nullptr;
+      h->elog_cap = 0;
+      F64_CK(cudaMalloc(&h->elog, (size_t)nsteps * 4 * sizeof(double)));
+      h->elog_cap = nsteps;
+    }
+    d_log = h->elog;
+  }
   const int B = nblocks(h);
   int rc = B2MD_OK;
   for (long long k = 0; k < nsteps && rc == B2MD_OK; ++k) {
@@ -605,8 +774,7 @@ int b2md_f64_run(b2md_f64* h, long long nsteps, double* energies) {
     }
     rc = launch_forces(h);
     if (rc) break;
-    k64_integrate<<<B, kB, 0, h->stream>>>(h->a);
-    k64_finish<<<1, kB, 0, h->stream>>>(h->a, B, 1, d_log ? d_log + 4 * k : nullptr);
+    k64_integrate<<<B, kB, 0, h->stream>>>(h->a, d_log ? d_log + 4 * k : nullptr);
     if (cudaGetLastError() != cudaSuccess) rc = f64_fail(B2MD_ERR_CUDA, "b2md_f64_run: launch failed");
     if (rc == B2MD_OK && (k + 1) % 256 == 0) rc = check_overflow(h);
   }
@@ -615,7 +783,12 @@ int b2md_f64_run(b2md_f64* h, long long nsteps, double* energies) {
     if (cudaMemcpy(energies, d_log, (size_t)nsteps * 4 * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = f64_fail(B2MD_ERR_CUDA, "b2md_f64_run: energy copy failed");
   }
-  if (d_log) cudaFree(d_log);
+  // (a log of more than 64 MB is not kept)
+  if (h->elog_cap > (1LL << 21)) {
+    cudaFree(h->elog);
+    h->elog = nullptr;
+    h->elog_cap = 0;
+  }
   return rc;
 }
 
@@ -624,16 +797,24 @@ int b2md_f64_get(b2md_f64* h, int field, void* out) {
   const int n = h->a.n;
   F64_CK(cudaSetDevice(h->device));
   F64_CK(cudaStreamSynchronize(h->stream));
+  std::vector<unsigned> uid(n);
+  F64_CK(cudaMemcpy(uid.data(), h->a.uid, n * sizeof(unsigned), cudaMemcpyDeviceToHost));
   if (field == B2MD_F64_POS || field == B2MD_F64_VEL || field == B2MD_F64_FORCE) {
     const double4* src = field == B2MD_F64_POS ? h->a.r : (field == B2MD_F64_VEL ? h->a.v : h->a.f);
-    F64_CK(cudaMemcpy(out, src, n * sizeof(double4), cudaMemcpyDeviceToHost));
+    std::vector<double4> tmp(n);
+    F64_CK(cudaMemcpy(tmp.data(), src, n * sizeof(double4), cudaMemcpyDeviceToHost));
+    double4* o = static_cast<double4*>(out);
+    for (int i = 0; i < n; ++i) o[uid[i]] = tmp[i];
     return B2MD_OK;
   }
   if (field == B2MD_F64_IMAGES) {
     std::vector<int4> im(n);
     F64_CK(cudaMemcpy(im.data(), h->a.im, n * sizeof(int4), cudaMemcpyDeviceToHost));
     int* o = static_cast<int*>(out);
-    for (int i = 0; i < n; ++i) { o[3 * i] = im[i].x; o[3 * i + 1] = im[i].y; o[3 * i + 2] = im[i].z; }
+    for (int i = 0; i < n; ++i) {
+      int* p = o + 3 * (size_t)uid[i];
+      p[0] = im[i].x; p[1] = im[i].y; p[2] = im[i].z;
+    }
     return B2MD_OK;
   }
   return f64_fail(B2MD_ERR_ARG, "b2md_f64_get: unknown field %d", field);
