@@ -11,6 +11,8 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 using namespace b2md;
@@ -180,8 +182,6 @@ struct b2md_engine {
   unsigned fqcap = 0;          // k_flow: queue slots
   PersistCtl* pctl = nullptr;  // k_steps control block
   int* h_budget = nullptr;     // pinned: the step budget written before each persistent launch
-  void* h_stage = nullptr;     // pinned staging for particle uploads and read-backs (grown on demand)
-  size_t h_stage_bytes = 0;
   // pinned ring for host-to-device copies that may wait behind running work
   // (admissions, layout uploads): a call fills a region and returns at once
   char* ring = nullptr;
@@ -253,23 +253,29 @@ void dev_grow(b2md_engine* e, T*& p, long long old_n, long long new_n, bool zero
   p = np;
 }
 
-// Pinned host staging of at least `bytes` (kept for the engine's life), so
-// that particle uploads and read-backs are DMA copies.  Sized per particle
-// for the largest use (read-back: id + r + v + images, plus alignment).
-constexpr size_t kStagePerParticle = 64;
-void* host_stage(b2md_engine* e, size_t bytes) {
-  if (bytes > e->h_stage_bytes) {
-    if (e->h_stage) {
-      CK(cudaStreamSynchronize(e->stream));
-      CK(cudaFreeHost(e->h_stage));
-      e->h_stage = nullptr;
-      e->h_stage_bytes = 0;
-    }
-    const size_t b = std::max(bytes, (size_t)1 << 20);
-    CK(cudaMallocHost(&e->h_stage, b));
-    e->h_stage_bytes = b;
+// Copies from the pinned staging to the caller's memory, by four threads when
+// it is large: fresh pages are faulted in by the copy, which is most of it.
+void copy_out(void* dst, const void* src, size_t bytes) {
+  constexpr size_t kPerThread = (size_t)2 << 20;
+  const size_t nt = std::min<size_t>(4, bytes / kPerThread);
+  if (nt < 2) {
+    std::memcpy(dst, src, bytes);
+    return;
   }
-  return e->h_stage;
+  const size_t part = (bytes / nt + 4095) & ~(size_t)4095;
+  auto piece = [&](size_t k) {
+    const size_t b = std::min(bytes, k * part), e = std::min(bytes, b + part);
+    std::memcpy(static_cast<char*>(dst) + b, static_cast<const char*>(src) + b, e - b);
+  };
+  std::vector<std::thread> th;
+  size_t k = 1;
+  try {
+    for (; k < nt; ++k) th.emplace_back(piece, k);
+  } catch (const std::system_error&) {  // no thread to be had: the rest here
+  }
+  piece(0);
+  for (size_t q = k; q < nt; ++q) piece(q);
+  for (auto& t : th) t.join();
 }
 
 // Page-locked host memory (cudaMallocHost / cudaHostRegister): DMA-able as is.
@@ -1545,6 +1551,54 @@ bool map_launch(int pb, int tp, int* pb_out, int* tp_out) {
   return true;
 }
 
+// One field of replica id from a region of the staging ring, in the caller's
+// order: queued behind what runs, nothing waits.
+void write_field4(b2md_engine* e, int id, HostRep& h, unsigned what, const float4* stage) {
+  EngArgs a = make_args(e);
+  const int blocks = (h.n + 255) / 256;
+  k_write_stream<<<std::min(blocks, 4 * std::max(e->nsm, 1)), 256, 0, e->stream>>>(a, id, h.p0, h.n, what, stage);
+  k_write_sort<<<blocks, 256, 0, e->stream>>>(a, id, h.p0, h.n, what);
+  check_launch();
+  stage_commit(e);
+}
+
+// A region of the staging ring for a read-back, given back at the end of the
+// call, by when the stream has been waited for.
+struct ReadStage {
+  b2md_engine* e;
+  size_t head;
+  char* p;
+  ReadStage(b2md_engine* eng, size_t bytes) : e(eng), head(eng->ring_head), p(stage_alloc(eng, bytes)) {}
+  void done() {
+    e->ring_open.pop_back();
+    e->ring_head = head;
+  }
+};
+
+// Fields of replica id to the caller's arrays, in the caller's order (vel also
+// receives the field src).  Everything the engine has queued before is
+// finished when this returns.
+void read_back(b2md_engine* e, int id, HostRep& h, unsigned what, const float4* src, void* pos, void* vel,
+               void* images) {
+  const size_t n = (size_t)h.n;
+  const size_t pb = pos ? n * sizeof(float4) : 0, vb = vel ? n * sizeof(float4) : 0;
+  const size_t ib = images ? n * 3 * sizeof(int) : 0;
+  ReadStage st(e, pb + vb + ib);
+  float4* sp = reinterpret_cast<float4*>(st.p);
+  float4* sv = reinterpret_cast<float4*>(st.p + pb);
+  int* si = reinterpret_cast<int*>(st.p + pb + vb);
+  EngArgs a = make_args(e);
+  const int blocks = (h.n + 255) / 256;
+  k_read_unsort<<<blocks, 256, 0, e->stream>>>(a, id, h.p0, h.n, what, src);
+  k_read_stream<<<std::min(blocks, 4 * std::max(e->nsm, 1)), 256, 0, e->stream>>>(a, id, h.p0, h.n, what, sp, sv, si);
+  check_launch();
+  CK(cudaStreamSynchronize(e->stream));
+  if (pos) copy_out(pos, sp, pb);
+  if (vel) copy_out(vel, sv, vb);
+  if (images) copy_out(images, si, ib);
+  st.done();
+}
+
 void launch_momentum(b2md_engine* e) {
   ensure_layout(e);
   if (e->ntiles == 0) return;
@@ -1612,9 +1666,8 @@ int b2md_engine_create(int device, long long max_particles, int max_replicas, lo
     // pinned staging for the expected particles, so that admissions and
     // read-backs do not allocate it later
     if (max_particles > 0) {
-      host_stage(e, (size_t)max_particles * kStagePerParticle);
-      ring_reserve(e, std::min<size_t>(std::max<size_t>((size_t)max_particles * 64, (size_t)4 << 20),
-                                       (size_t)64 << 20));
+      ring_reserve(e, std::min<size_t>(std::max<size_t>((size_t)max_particles * 128, (size_t)4 << 20),
+                                       (size_t)256 << 20));
     }
     init_func_attrs(device);
     CK(cudaMalloc(&e->fctr, sizeof(unsigned)));
@@ -1652,7 +1705,6 @@ int b2md_engine_destroy(b2md_engine* e) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->h_budget) cudaFreeHost(e->h_budget);
-  if (e->h_stage) cudaFreeHost(e->h_stage);
   ring_reset(e);
   if (e->ring) cudaFreeHost(e->ring);
   for (auto& c : e->chunk) {
@@ -1945,34 +1997,15 @@ int b2md_replica_get(b2md_engine* e, int id, int field, void* out) {
   return guarded([&] {
     HostRep& h = get_rep(e, id);
     CK(cudaSetDevice(e->device));
-    RepState s = read_state(e, id);
-    std::vector<unsigned> ids(h.n);
-    CK(cudaMemcpyAsync(ids.data(), e->uidx[s.abuf] + h.p0, h.n * sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
-    if (field == B2MD_FIELD_IMAGES) {
-      std::vector<int4> tmp(h.n);
-      CK(cudaMemcpyAsync(tmp.data(), e->im[s.abuf] + h.p0, h.n * sizeof(int4), cudaMemcpyDeviceToHost, e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      int* o = static_cast<int*>(out);
-      for (int k = 0; k < h.n; ++k) {
-        unsigned i = ids[k];
-        o[3 * i] = tmp[k].x; o[3 * i + 1] = tmp[k].y; o[3 * i + 2] = tmp[k].z;
-      }
-      return;
-    }
-    const float4* src = nullptr;
     switch (field) {
-      case B2MD_FIELD_POS: src = e->r[s.rbuf]; break;
-      case B2MD_FIELD_VEL: src = e->v[s.abuf]; break;
-      case B2MD_FIELD_FORCE: src = e->f; break;
-      case B2MD_FIELD_VIRIAL: src = e->w; break;
-      case B2MD_FIELD_STRESS: src = e->sts; break;
+      case B2MD_FIELD_POS: read_back(e, id, h, kReadPos, nullptr, out, nullptr, nullptr); break;
+      case B2MD_FIELD_VEL: read_back(e, id, h, kReadVel, nullptr, nullptr, out, nullptr); break;
+      case B2MD_FIELD_FORCE: read_back(e, id, h, kReadField, e->f, nullptr, out, nullptr); break;
+      case B2MD_FIELD_VIRIAL: read_back(e, id, h, kReadField, e->w, nullptr, out, nullptr); break;
+      case B2MD_FIELD_STRESS: read_back(e, id, h, kReadField, e->sts, nullptr, out, nullptr); break;
+      case B2MD_FIELD_IMAGES: read_back(e, id, h, kReadImages, nullptr, nullptr, nullptr, out); break;
       default: api_fail(B2MD_ERR_ARG, "unknown field");
     }
-    std::vector<float4> tmp(h.n);
-    CK(cudaMemcpyAsync(tmp.data(), src + h.p0, h.n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    float4* o = static_cast<float4*>(out);
-    for (int k = 0; k < h.n; ++k) o[ids[k]] = tmp[k];
   });
 }
 
@@ -1980,30 +2013,8 @@ int b2md_replica_read(b2md_engine* e, int id, float* pos4, float* vel4, int* im3
   return guarded([&] {
     HostRep& h = get_rep(e, id);
     CK(cudaSetDevice(e->device));
-    RepState s = read_state(e, id);
-    const size_t n = (size_t)h.n;
-    char* stage = static_cast<char*>(host_stage(e, n * kStagePerParticle));
-    unsigned* ids = reinterpret_cast<unsigned*>(stage);
-    float4* sr = reinterpret_cast<float4*>(stage + ((n * sizeof(unsigned) + 15) & ~(size_t)15));
-    float4* sv = sr + n;
-    int4* si = reinterpret_cast<int4*>(sv + n);
-    CK(cudaMemcpyAsync(ids, e->uidx[s.abuf] + h.p0, n * sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
-    if (pos4) CK(cudaMemcpyAsync(sr, e->r[s.rbuf] + h.p0, n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
-    if (vel4) CK(cudaMemcpyAsync(sv, e->v[s.abuf] + h.p0, n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
-    if (im3) CK(cudaMemcpyAsync(si, e->im[s.abuf] + h.p0, n * sizeof(int4), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    float4* po = reinterpret_cast<float4*>(pos4);
-    float4* vo = reinterpret_cast<float4*>(vel4);
-    for (size_t k = 0; k < n; ++k) {
-      const unsigned i = ids[k];
-      if (pos4) po[i] = sr[k];
-      if (vel4) vo[i] = sv[k];
-      if (im3) {
-        im3[3 * (size_t)i] = si[k].x;
-        im3[3 * (size_t)i + 1] = si[k].y;
-        im3[3 * (size_t)i + 2] = si[k].z;
-      }
-    }
+    const unsigned what = (pos4 ? kReadPos : 0u) | (vel4 ? kReadVel : 0u) | (im3 ? kReadImages : 0u);
+    if (what) read_back(e, id, h, what, nullptr, pos4, vel4, im3);
   });
 }
 
@@ -2012,37 +2023,28 @@ int b2md_replica_set(b2md_engine* e, int id, int field, const void* in) {
   return guarded([&] {
     HostRep& h = get_rep(e, id);
     CK(cudaSetDevice(e->device));
-    RepState s = read_state(e, id);
-    std::vector<unsigned> ids(h.n);
-    CK(cudaMemcpyAsync(ids.data(), e->uidx[s.abuf] + h.p0, h.n * sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    if (field == B2MD_FIELD_IMAGES) {
-      const int* src = static_cast<const int*>(in);
-      std::vector<int4> tmp(h.n);
-      for (int k = 0; k < h.n; ++k) {
-        unsigned i = ids[k];
-        tmp[k] = make_int4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0);
-      }
-      CK(cudaMemcpyAsync(e->im[s.abuf] + h.p0, tmp.data(), h.n * sizeof(int4), cudaMemcpyHostToDevice, e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      return;
-    }
     const float4* src = static_cast<const float4*>(in);
-    std::vector<float4> tmp(h.n);
-    for (int k = 0; k < h.n; ++k) tmp[k] = src[ids[k]];
-    if (field == B2MD_FIELD_POS) {
+    const size_t nb = (size_t)h.n * sizeof(float4);
+    if (field == B2MD_FIELD_IMAGES) {
+      const int* im = static_cast<const int*>(in);
+      int4* stage = reinterpret_cast<int4*>(stage_alloc(e, nb));
+      for (int k = 0; k < h.n; ++k) stage[k] = make_int4(im[3 * k], im[3 * k + 1], im[3 * k + 2], 0);
+      write_field4(e, id, h, kReadImages, reinterpret_cast<const float4*>(stage));
+    } else if (field == B2MD_FIELD_POS) {
       for (int k = 0; k < h.n; ++k) {
         int t;
-        std::memcpy(&t, &tmp[k].w, 4);
+        std::memcpy(&t, &src[k].w, 4);
         if (t < 0 || t >= h.d.ntypes) api_fail(B2MD_ERR_ARG, "particle type out of range");
       }
-      CK(cudaMemcpyAsync(e->r[s.rbuf] + h.p0, tmp.data(), h.n * sizeof(float4), cudaMemcpyHostToDevice, e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      WRITE_STATE(e, id, rebuild, 1);
+      float4* stage = reinterpret_cast<float4*>(stage_alloc(e, nb));
+      std::memcpy(stage, src, nb);
+      write_field4(e, id, h, kReadPos, stage);
     } else if (field == B2MD_FIELD_VEL) {
       for (int k = 0; k < h.n; ++k)
-        if (!(tmp[k].w > 0.f)) api_fail(B2MD_ERR_ARG, "inverse mass must be positive");
-      CK(cudaMemcpyAsync(e->v[s.abuf] + h.p0, tmp.data(), h.n * sizeof(float4), cudaMemcpyHostToDevice, e->stream));
+        if (!(src[k].w > 0.f)) api_fail(B2MD_ERR_ARG, "inverse mass must be positive");
+      float4* stage = reinterpret_cast<float4*>(stage_alloc(e, nb));
+      std::memcpy(stage, src, nb);
+      write_field4(e, id, h, kReadVel, stage);
       launch_momentum(e);
       CK(cudaStreamSynchronize(e->stream));
     } else {
@@ -2243,23 +2245,15 @@ int b2md_replica_stress(b2md_engine* e, int id, int include_kinetic, double* out
   return guarded([&] {
     HostRep& h = get_rep(e, id);
     CK(cudaSetDevice(e->device));
-    std::vector<float4> sts(h.n), w(h.n), v(h.n);
-    RepState s = read_state(e, id);
-    CK(cudaMemcpyAsync(sts.data(), e->sts + h.p0, h.n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaMemcpyAsync(w.data(), e->w + h.p0, h.n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaMemcpyAsync(v.data(), e->v[s.abuf] + h.p0, h.n * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
+    ensure_layout(e);
+    ReadStage stage(e, 6 * sizeof(double));
+    double* s6 = reinterpret_cast<double*>(stage.p);
+    k_stress<<<h.d.ntiles, e->pb, 0, e->stream>>>(make_args(e), id, include_kinetic, s6);
+    check_launch();
     CK(cudaStreamSynchronize(e->stream));
-    // Sample::GetStress (Sample.cu:393-444)
-    double st[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = 0; i < h.n; ++i) {
-      st[0] += sts[i].x; st[1] += sts[i].y; st[2] += sts[i].z; st[3] += sts[i].w;
-      st[4] += w[i].y; st[5] += w[i].z;
-      if (include_kinetic) {
-        float mass2 = 2.f / v[i].w;
-        st[0] -= mass2 * v[i].x * v[i].x; st[1] -= mass2 * v[i].y * v[i].y; st[2] -= mass2 * v[i].z * v[i].z;
-        st[3] -= mass2 * v[i].y * v[i].z; st[4] -= mass2 * v[i].x * v[i].z; st[5] -= mass2 * v[i].x * v[i].y;
-      }
-    }
+    double st[6];
+    std::memcpy(st, s6, sizeof st);
+    stage.done();
     double V = (double)h.d.L[0] * h.d.L[1] * h.d.L[2];
     for (int k = 0; k < 6; ++k) out6[k] = 0.5 * st[k] / V;
   });
