@@ -1622,6 +1622,16 @@ __global__ void k_gate_flag(EngArgs a, int* out) {
 // for replicas that are not flagged, so the same sequence serves batches.
 // ---------------------------------------------------------------------------
 
+// A list longer than its capacity freezes the replica until the host has
+// enlarged it.  Flagged by a build's last block: a block of the same build that
+// starts after the flag is up would take the replica for frozen and leave the
+// build's counters unfinished.
+__device__ __forceinline__ bool flag_overflow(const RepDev& R, RepState* S) {
+  const bool over = __ldcg(&S->actual_max_nbrs) > R.max_nbrs;
+  if (over) atomicExch(&S->overflow, 1);
+  return over;
+}
+
 __device__ __forceinline__ int cell_chunk(const RepDev& R) { return (R.ncell + R.ntiles - 1) / R.ntiles; }
 
 // (1) zero cell counts of this tile's chunk of the replica's cells
@@ -2272,12 +2282,12 @@ __global__ void __launch_bounds__(kMaxBlock) k_rb_build(EngArgs a) {
   if (threadIdx.x == 0) {
     const int s_max_v = s_max;
     atomicMax(&S->actual_max_nbrs, s_max_v);
-    if (s_max_v > R.max_nbrs) atomicExch(&S->overflow, 1);
     __threadfence();
     unsigned c = atomicAdd(&a.rctr[rep], 1u);
     s_last = (c == (unsigned)(R.ntiles - 1));
     if (s_last) {
       a.rctr[rep] = 0u;
+      flag_overflow(R, S);
       S->rebuild = 0;
       S->nrebuilds += 1;
     }
@@ -2460,11 +2470,11 @@ __global__ void __launch_bounds__(kCwWarps * 32) k_rb_build_cw(EngArgs a) {
   if (threadIdx.x == 0) {
     const int s_max_v = s_max;
     atomicMax(&S->actual_max_nbrs, s_max_v);
-    if (s_max_v > R.max_nbrs) atomicExch(&S->overflow, 1);
     __threadfence();
     const unsigned cdone = atomicAdd(&a.rctr[rep], 1u);
     if (cdone == (unsigned)(R.ntiles - 1)) {
       a.rctr[rep] = 0u;
+      flag_overflow(R, S);
       S->rebuild = 0;
       S->nrebuilds += 1;
     }
@@ -2716,10 +2726,6 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
   if (threadIdx.x == 0) {
     const int s_max_v = *s_max;
     atomicMax(&S->actual_max_nbrs, s_max_v);
-    if (s_max_v > R.max_nbrs) {
-      atomicExch(&S->overflow, 1);
-      if (COH) s_step_tally += 1ull << kTallyRebuildShift;  // k_batch: the launch stops at the step's end
-    }
     __threadfence();
     const unsigned cdone = atomicAdd(&a.rctr[rep], 1u);
     const bool fin = cdone == (unsigned)(R.ntiles * parts - 1);
@@ -2727,6 +2733,8 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
     if (fin) {
       a.rctr[rep] = 0u;
       if (GRID) S->build_next = 0;
+      if (flag_overflow(R, S) && COH)
+        s_step_tally += 1ull << kTallyRebuildShift;  // k_batch: the launch stops at the step's end
       S->nrebuilds += 1;
       // the replica's lists are complete: released to k_batch's force items
       st_release_u32(reinterpret_cast<unsigned*>(&S->rebuild), 0u);

@@ -249,3 +249,18 @@ def test_lists_over_full_cell(capi, oracle, lj_params):
     gc, gl = e.nbl(rid, n, 400)
     compare_lists(gc, gl, uidx, counts, nbl)
     e.close()
+
+
+def test_lists_after_an_overflow_with_more_blocks_than_resident(capi, oracle, lj_params):
+    """120000 LJ particles (more list-build blocks than the GPU holds at once),
+    70 of them in one cell, so that the estimated list capacity overflows while
+    blocks of the same build have yet to start: the repaired lists are the
+    oracle's, and so are those of a second build."""
+    from rumd_b200 import initconf as I
+    n, k = 120000, 70
+    c = I.lj_config(n, density=0.8442, T=1.0, seed=5)
+    pos = c["pos4"].copy()
+    rng = np.random.default_rng(5)
+    centre = np.asarray(c["box"], np.float32) * 0.3
+    pos[:k, :3] = centre + rng.uniform(-0.6, 0.6, (k, 3)).astype(np.float32)
+    identity_build(capi, oracle, pos, c["box"], lj_params, 1, max_nbrs=400)
