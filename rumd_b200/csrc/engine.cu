@@ -870,19 +870,21 @@ void place_list(b2md_engine* e, HostRep& h, int max_nbrs) {
 
 // ---- launches ----
 // Kernels in one rebuild sequence (launch_rebuild).
-int rebuild_launches(const b2md_engine* e) { return e->force_mode == FM_WINDOW ? 9 : 8; }
+int rebuild_launches(const b2md_engine* e) { return e->force_mode == FM_WINDOW ? 3 : 2; }
 
 void launch_rebuild(b2md_engine* e, cudaStream_t s, const EngArgs& a) {
   const int T = e->ntiles;
-  const int R = (int)e->reps.size();
   if (T == 0) return;
-  k_rb_clear<<<T, e->pb, 0, s>>>(a);
-  k_rb_count<<<T, e->pb, 0, s>>>(a);
-  k_rb_scan_local<<<T, e->pb, 0, s>>>(a);
-  k_rb_scan_tiles<<<R, 256, 0, s>>>(a);
-  k_rb_scatter<<<T, e->pb, 0, s>>>(a);
-  k_rb_fix<<<T, e->pb, 0, s>>>(a);
-  k_rb_permute<<<T, e->pb, 0, s>>>(a);
+  {
+    // two blocks per SM at most (all resident; fewer meet faster), enough for
+    // a thread per slot
+    EngArgs args = a;
+    int pb = e->pb;
+    void* ka[] = {&args, &pb};
+    const long long want = ((long long)T * e->pb + kSortBlock - 1) / kSortBlock;
+    const int grid = (int)std::max(1LL, std::min(want, 2LL * std::max(e->nsm, 1)));
+    CK(cudaLaunchCooperativeKernel((const void*)k_rb_sort, dim3(grid), dim3(kSortBlock), ka, 0, s));
+  }
   if (a.win_on) k_rb_window<<<T, e->pb, sizeof(WinScratch), s>>>(a);
   // list build: build_lanes lanes per particle (fewer when pb*lanes would
   // exceed a block), the list either assembled in shared memory or stored

@@ -131,6 +131,8 @@ struct PersistCtl {
   int active;
   int ran;
   unsigned exited;
+  // k_rb_sort's grid barrier
+  unsigned sort_arrive, sort_gen;
 };
 
 struct EngArgs {
@@ -150,7 +152,7 @@ struct EngArgs {
   int* cnt;
   int* cstart;
   int* ctot;    // per tile: cell-chunk total (scan)
-  int* cpref;   // per tile: exclusive prefix of chunk totals within the replica
+  int* cpref;   // a replica's first entries: totals of kScanGroup chunks
   const float* par;
   const RepDev* rep;
   RepState* st;

@@ -1590,7 +1590,7 @@ __global__ void k_clear_overflow(RepState* s) {
 // batched kernels do.
 __device__ __forceinline__ bool rb_active(const EngArgs& a, int rep) {
   const RepState* S = a.st + rep;
-  return a.rep[rep].active && S->rebuild && !S->overflow && (!a.rb_steps_only || S->steps_left > 0);
+  return a.rep[rep].active && S->rebuild && !S->overflow && !S->err && (!a.rb_steps_only || S->steps_left > 0);
 }
 
 // Gate: publishes "any replica flagged for rebuild" to the first conditional node.
@@ -1634,224 +1634,193 @@ __device__ __forceinline__ bool flag_overflow(const RepDev& R, RepState* S) {
 
 __device__ __forceinline__ int cell_chunk(const RepDev& R) { return (R.ncell + R.ntiles - 1) / R.ntiles; }
 
-// (1) zero cell counts of this tile's chunk of the replica's cells
-__global__ void k_rb_clear(EngArgs a) {
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  // the replica's first tile also resets the per-build maximum list length
-  if (tile == R.tile0 && threadIdx.x == 0) a.st[rep].actual_max_nbrs = 0;
-  if (R.nb_method != NB_CELLS) return;
-  const int ch = cell_chunk(R), lt = tile - R.tile0;
-  const int c0 = lt * ch, c1 = min(R.ncell, c0 + ch);
-  for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) a.cnt[R.cell0 + c] = 0;
-}
-
-// (2) cell key per particle (calculateCellIndices, NeighborList.cu:1142-1172) and
-//     its arrival rank in the cell
-__global__ void k_rb_count(EngArgs a) {
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  const int i = a.tile_first[tile] + threadIdx.x;
-  if (i >= R.n) return;
-  const size_t gi = (size_t)R.p0 + i;
-  const float4 r = a.r[a.st[rep].rbuf][gi];
-  const int cx = cell_coord(r.x, R.invL[0], R.nc[0]);
-  const int cy = cell_coord(r.y, R.invL[1], R.nc[1]);
-  const int cz = cell_coord(r.z, R.invL[2], R.nc[2]);
-  const int key = cx + cy * R.nc[0] + cz * R.nc[0] * R.nc[1];
-  a.key[gi] = key;
-  a.slot[gi] = atomicAdd(&a.cnt[R.cell0 + key], 1);
-}
-
-// (3a) chunk-local exclusive prefix of cell counts; chunk total per tile
-__global__ void k_rb_scan_local(EngArgs a) {
-  __shared__ int s_w[kMaxBlock / 32];
-  __shared__ int s_carry;
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  const int ch = cell_chunk(R), lt = tile - R.tile0;
-  const int c0 = lt * ch, c1 = min(R.ncell, c0 + ch);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (int base = c0; base < c1; base += blockDim.x) {
-    const int c = base + threadIdx.x;
-    const int x = c < c1 ? a.cnt[R.cell0 + c] : 0;
-    int incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) s_w[wid] = incl;
-    __syncthreads();
-    int woff = 0;
-    for (int w = 0; w < wid; ++w) woff += s_w[w];
-    const int carry = s_carry;
-    if (c < c1) a.cstart[R.cell0 + c] = carry + woff + incl - x;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) {
-      int tot = 0;
-      for (int w = 0; w < nw; ++w) tot += s_w[w];
-      s_carry = carry + tot;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) a.ctot[tile] = s_carry;
-}
-
-// (3b) exclusive prefix of chunk totals over the replica's tiles (block per
-//      replica): thread t sums a run of consecutive tiles (its loads all in
-//      flight together), the block scans the run sums, and each thread
-//      writes its run's prefixes
-constexpr int kScanRun = 8;  // tiles per thread and pass
-__global__ void k_rb_scan_tiles(EngArgs a) {
-  __shared__ int s_w[32];
-  __shared__ int s_carry;
-  const int rep = blockIdx.x;
-  if (rep >= a.nrep || !rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int* __restrict__ tot = a.ctot + R.tile0;
-  int* __restrict__ pref = a.cpref + R.tile0;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (int base = 0; base < R.ntiles; base += blockDim.x * kScanRun) {
-    const int t0 = base + threadIdx.x * kScanRun;
-    int x[kScanRun];
-    int sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanRun; ++k) {
-      x[k] = t0 + k < R.ntiles ? tot[t0 + k] : 0;
-      sum += x[k];
-    }
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) s_w[wid] = incl;
-    __syncthreads();
-    int woff = 0;
-    for (int w = 0; w < wid; ++w) woff += s_w[w];
-    const int carry = s_carry;
-    int run = carry + woff + incl - sum;
-#pragma unroll
-    for (int k = 0; k < kScanRun; ++k) {
-      if (t0 + k < R.ntiles) pref[t0 + k] = run;
-      run += x[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) {
-      int t = 0;
-      for (int w = 0; w < nw; ++w) t += s_w[w];
-      s_carry = carry + t;
-    }
-    __syncthreads();
-  }
-}
-
-__device__ __forceinline__ int cell_begin(const EngArgs& a, const RepDev& R, int c, int ch) {
-  return a.cstart[R.cell0 + c] + a.cpref[R.tile0 + c / ch];
-}
-
-// (4) scatter particle ids to their cell buckets (arrival order)
-__global__ void k_rb_scatter(EngArgs a) {
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  const int i = a.tile_first[tile] + threadIdx.x;
-  if (i >= R.n) return;
-  const size_t gi = (size_t)R.p0 + i;
-  const int key = a.key[gi];
-  const int pos = cell_begin(a, R, key, cell_chunk(R)) + a.slot[gi];
-  a.order[(size_t)R.p0 + pos] = (unsigned)i;
-}
-
-// (5) order each bucket by old index: the result equals a stable sort by key
-//     (thrust::sort_by_key on (cellIndex, iota), Sample.h:174-188).  Also
-//     turns cstart into each cell's absolute first slot (cstart + the chunk's
-//     prefix), which the list build reads without a division.
-constexpr int kFixRegs = 8;  // buckets up to this size are sorted in registers
-__global__ void k_rb_fix(EngArgs a) {
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  const int ch = cell_chunk(R), lt = tile - R.tile0;
-  const int c0 = lt * ch, c1 = min(R.ncell, c0 + ch);
-  const int pref = a.cpref[R.tile0 + lt];
-  for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-    const int b = a.cstart[R.cell0 + c] + pref, m = a.cnt[R.cell0 + c];
-    a.cstart[R.cell0 + c] = b;
-    unsigned* o = a.order + (size_t)R.p0 + b;
-    if (m <= kFixRegs) {
-      // the bucket in registers (padding sorts last), odd-even transposition
-      unsigned x[kFixRegs];
-#pragma unroll
-      for (int k = 0; k < kFixRegs; ++k) x[k] = k < m ? o[k] : 0xffffffffu;
-#pragma unroll
-      for (int r = 0; r < kFixRegs; ++r)
-#pragma unroll
-        for (int k = r & 1; k + 1 < kFixRegs; k += 2) {
-          const unsigned lo = min(x[k], x[k + 1]), hi = max(x[k], x[k + 1]);
-          x[k] = lo;
-          x[k + 1] = hi;
-        }
-#pragma unroll
-      for (int k = 0; k < kFixRegs; ++k)
-        if (k < m) o[k] = x[k];
-      continue;
-    }
-    for (int p = 1; p < m; ++p) {
-      unsigned x = o[p];
-      int q = p - 1;
-      while (q >= 0 && o[q] > x) { o[q + 1] = o[q]; --q; }
-      o[q + 1] = x;
-    }
-  }
-}
-
-// (6) gather r, v, images, unsorted index into the sorted order
-//     (ParticleData::UpdateAfterSorting, ParticleData.cu:493-528); the last
-//     block of the replica flips the buffer parities
-__global__ void k_rb_permute(EngArgs a) {
-  const int tile = blockIdx.x, rep = a.tile_rep[tile];
-  if (!rb_active(a, rep)) return;
-  const RepDev& R = a.rep[rep];
-  if (R.nb_method != NB_CELLS) return;
-  RepState* S = a.st + rep;
-  const int s = a.tile_first[tile] + threadIdx.x;
-  const int rb = S->rbuf, ab = S->abuf;
-  if (s < R.n) {
-    const size_t gs = (size_t)R.p0 + s;
-    const size_t go = (size_t)R.p0 + a.order[gs];
-    a.r[rb ^ 1][gs] = a.r[rb][go];
-    a.v[ab ^ 1][gs] = a.v[ab][go];
-    a.im[ab ^ 1][gs] = a.im[ab][go];
-    a.uidx[ab ^ 1][gs] = a.uidx[ab][go];
-  }
-  __shared__ int s_last;
+// Grid barrier of k_rb_sort (every block resident); false, in every thread,
+// when the wait gave up.
+__device__ bool sort_barrier(PersistCtl* c) {
+  __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
+    s_ok = 1;
+    const unsigned gen = ld_acquire_u32(&c->sort_gen);
+    if (atom_add_acq_rel(&c->sort_arrive, 1u) == gridDim.x - 1) {
+      c->sort_arrive = 0u;
+      st_release_u32(&c->sort_gen, gen + 1u);
+    } else {
+      unsigned it = 0;
+      while (ld_acquire_u32(&c->sort_gen) == gen && it < kBarrierPolls) {
+        __nanosleep(20);
+        ++it;
+      }
+      if (it >= kBarrierPolls) s_ok = 0;
+    }
     __threadfence();
-    unsigned c = atomicAdd(&a.rctr[rep], 1u);
-    s_last = (c == (unsigned)(R.ntiles - 1));
-    if (s_last) {
-      a.rctr[rep] = 0u;
-      S->rbuf = rb ^ 1;
-      S->abuf = ab ^ 1;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// The stable cell-key sort of every flagged replica's particles in one
+// cooperative launch (the permutation of thrust::sort_by_key on (cell key,
+// current slot), Sample.h:174-188), whose blocks meet between the phases:
+//   clear     the cell counts and the totals; the per-build maximum
+//   count     cell key (calculateCellIndices, NeighborList.cu:1142-1172) and
+//             arrival rank; totals per chunk of cells (one chunk per tile) and
+//             per kScanGroup chunks, a warp's equal ones added together
+//   scan      a warp per chunk: the groups and chunks before it, then its
+//             cells; cstart is each cell's first slot (NeighborList.cu:1175-1202)
+//   scatter   ids to their buckets in arrival order
+//   permute   each bucket's members by old slot (counted against each other),
+//             r, v, images and ids moved there (ParticleData::
+//             UpdateAfterSorting, ParticleData.cu:493-528); a replica's last
+//             warp flips its buffer parities
+// It returns at once when no list is due, so a step or force evaluation that
+// needs no rebuild pays one launch for it.  The phases are a microsecond or
+// two of latency each, so the number of launches and of blocks that meet is
+// what costs: as seven kernels of a block per tile the sort took 37 us at KA
+// N=65536 (ncu, 4.6 to 9.5 us each), as one launch 11 us less of the rebuild (119 -> 111 us with the
+// build at KA N=65536), and a force evaluation without a rebuild launches two
+// kernels instead of eight.
+constexpr int kScanGroup = 128;
+constexpr int kSortBlock = 512;
+__global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
+  {
+    int any = 0;
+    for (int r = tid; r < a.nrep; r += kSortBlock) any |= rb_active(a, r) ? 1 : 0;
+    if (!__syncthreads_or(any)) return;
+  }
+  const int gid = blockIdx.x * kSortBlock + tid, gsz = gridDim.x * kSortBlock;
+  const int warps = gsz >> 5;
+  PersistCtl* ctl = a.pctl;
+  bool ok = true;
+  // clear
+  for (int tile = gid >> 5; tile < a.ntiles; tile += warps) {
+    const int rep = a.tile_rep[tile];
+    if (!rb_active(a, rep)) continue;
+    const RepDev& R = a.rep[rep];
+    const int lt = tile - R.tile0;
+    if (lt == 0 && lane == 0) a.st[rep].actual_max_nbrs = 0;
+    if (R.nb_method != NB_CELLS) continue;
+    const int ch = cell_chunk(R), c1 = min(R.ncell, (lt + 1) * ch);
+    for (int c = lt * ch + lane; c < c1; c += 32) a.cnt[R.cell0 + c] = 0;
+    if (lane == 0) {
+      a.ctot[tile] = 0;
+      a.cpref[tile] = 0;  // (the groups' totals are the replica's first entries)
+    }
+  }
+  ok = sort_barrier(ctl);
+  // count (whole warps work on 32 slots of one tile: pb is a multiple of 32)
+  const int tpt = pb >> 5;  // warps per tile
+  if (ok) {
+    for (int w = gid >> 5; w < a.ntiles * tpt; w += warps) {
+      const int tile = w / tpt, rep = a.tile_rep[tile];
+      if (!rb_active(a, rep)) continue;
+      const RepDev& R = a.rep[rep];
+      if (R.nb_method != NB_CELLS) continue;
+      const int i = a.tile_first[tile] + (w - tile * tpt) * 32 + lane;
+      const bool in = i < R.n;
+      int chunk = -1;
+      if (in) {
+        const size_t gi = (size_t)R.p0 + i;
+        const float4 r = a.r[a.st[rep].rbuf][gi];
+        const int key = cell_coord(r.x, R.invL[0], R.nc[0]) + cell_coord(r.y, R.invL[1], R.nc[1]) * R.nc[0] +
+                        cell_coord(r.z, R.invL[2], R.nc[2]) * R.nc[0] * R.nc[1];
+        a.key[gi] = key;
+        a.slot[gi] = atomicAdd(&a.cnt[R.cell0 + key], 1);
+        chunk = key / cell_chunk(R);
+      }
+      const unsigned same = __match_any_sync(FULL, chunk);
+      if (in && lane == __ffs(same) - 1) atomicAdd(&a.ctot[R.tile0 + chunk], __popc(same));
+      const int group = in ? chunk / kScanGroup : -1;
+      const unsigned sg = __match_any_sync(FULL, group);
+      if (in && lane == __ffs(sg) - 1) atomicAdd(&a.cpref[R.tile0 + group], __popc(sg));
+    }
+    ok = sort_barrier(ctl);
+  }
+  // scan
+  if (ok) {
+    for (int tile = gid >> 5; tile < a.ntiles; tile += warps) {
+      const int rep = a.tile_rep[tile];
+      if (!rb_active(a, rep)) continue;
+      const RepDev& R = a.rep[rep];
+      if (R.nb_method != NB_CELLS) continue;
+      const int lt = tile - R.tile0, g = lt / kScanGroup;
+      int sum = 0;
+      for (int k = lane; k < g; k += 32) sum += __ldcg(a.cpref + R.tile0 + k);
+      for (int k = g * kScanGroup + lane; k < lt; k += 32) sum += __ldcg(a.ctot + R.tile0 + k);
+      int first = __reduce_add_sync(FULL, sum);
+      const int ch = cell_chunk(R), c0 = lt * ch, c1 = min(R.ncell, c0 + ch);
+      for (int cb = c0; cb < c1; cb += 32) {
+        const int c = cb + lane;
+        const int m = c < c1 ? __ldcg(a.cnt + R.cell0 + c) : 0;
+        int incl = m;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(FULL, incl, o);
+          if (lane >= o) incl += y;
+        }
+        if (c < c1) a.cstart[R.cell0 + c] = first + incl - m;
+        first += __shfl_sync(FULL, incl, 31);
+      }
+    }
+    ok = sort_barrier(ctl);
+  }
+  // scatter
+  if (ok) {
+    for (int w = gid >> 5; w < a.ntiles * tpt; w += warps) {
+      const int tile = w / tpt, rep = a.tile_rep[tile];
+      if (!rb_active(a, rep)) continue;
+      const RepDev& R = a.rep[rep];
+      const int i = a.tile_first[tile] + (w - tile * tpt) * 32 + lane;
+      if (R.nb_method != NB_CELLS || i >= R.n) continue;
+      const size_t gi = (size_t)R.p0 + i;
+      a.order[(size_t)R.p0 + __ldcg(a.cstart + R.cell0 + a.key[gi]) + a.slot[gi]] = (unsigned)i;
+    }
+    ok = sort_barrier(ctl);
+  }
+  if (!ok) {
+    // (reported by the host; nothing else acts on a replica whose err is set)
+    for (int r = gid; r < a.nrep; r += gsz)
+      if (rb_active(a, r)) atomicExch(&a.st[r].err, 1);
+    return;
+  }
+  // permute
+  for (int w = gid >> 5; w < a.ntiles * tpt; w += warps) {
+    const int tile = w / tpt, rep = a.tile_rep[tile];
+    if (!rb_active(a, rep)) continue;
+    const RepDev& R = a.rep[rep];
+    if (R.nb_method != NB_CELLS) continue;
+    RepState* S = a.st + rep;
+    const int rb = S->rbuf, ab = S->abuf;
+    const int s = a.tile_first[tile] + (w - tile * tpt) * 32 + lane;
+    if (s < R.n) {
+      const unsigned* ord = a.order + R.p0;
+      const unsigned i = __ldcg(ord + s);
+      const size_t go = (size_t)R.p0 + i;
+      const int key = __ldcg(a.key + go);
+      const int b = __ldcg(a.cstart + R.cell0 + key), m = __ldcg(a.cnt + R.cell0 + key);
+      int place = b;
+      for (int k = 0; k < m; ++k) place += __ldcg(ord + b + k) < i;
+      const size_t gs = (size_t)R.p0 + place;
+      a.r[rb ^ 1][gs] = a.r[rb][go];
+      a.v[ab ^ 1][gs] = a.v[ab][go];
+      a.im[ab ^ 1][gs] = a.im[ab][go];
+      a.uidx[ab ^ 1][gs] = a.uidx[ab][go];
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      if (atomicAdd(&a.rctr[rep], 1u) == (unsigned)(R.ntiles * tpt - 1)) {
+        a.rctr[rep] = 0u;
+        S->rbuf = rb ^ 1;
+        S->abuf = ab ^ 1;
+      }
     }
   }
 }
+
+constexpr int kFixRegs = 8;  // block_sort, split_sort_item: buckets up to this size are sorted in registers
 
 // (7) sorted 5x5x5 cell scan (calculateNBL_CellsSorted, NeighborList.cu:1204-1319):
 //     neighbours in the reference's order (dz, dy, dx, ascending slot).
@@ -1997,7 +1966,7 @@ __device__ void tile_window(const EngArgs& a, const RepDev& R, int tile, int np,
   }
   if (S > kWinSeg) bad = true;
   __syncwarp();
-  const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_fix)
+  const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_sort)
   const int* __restrict__ ccnt = a.cnt + R.cell0;
   if (!bad)
     for (int e = lane; e < ne; e += 32) {
@@ -2189,7 +2158,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_rb_build(EngArgs a) {
     }
   };
   if (R.nb_method == NB_CELLS) {
-    const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_fix)
+    const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_sort)
     const int* __restrict__ ccnt = a.cnt + R.cell0;
     const int nx = R.nc[0], ny = R.nc[1], nz = R.nc[2];
     const int cx = cell_coord(ri.x, iLx, nx), cy = cell_coord(ri.y, iLy, ny), cz = cell_coord(ri.z, iLz, nz);
@@ -2334,7 +2303,7 @@ __global__ void __launch_bounds__(kCwWarps * 32) k_rb_build_cw(EngArgs a) {
   int* wslot = s_slot + warp * kCwCand;
   const bool cells = R.nb_method == NB_CELLS;
   const int nx = R.nc[0], ny = R.nc[1], nz = R.nc[2];
-  const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_fix)
+  const int* __restrict__ cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_sort)
   const int* __restrict__ ccnt = a.cnt + R.cell0;
   // units of work: the cells from the first to the last particle's (keys
   // ascend along the slots), or one unit for all pairs
@@ -2615,7 +2584,7 @@ __device__ __forceinline__ void build_runs_tile(const EngArgs& a, int tile, floa
   int4* tab = s_rows + warp * kRunRows;
   const bool cells = R.nb_method == NB_CELLS;
   const int nx = R.nc[0], ny = R.nc[1], nz = R.nc[2];
-  const int* cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_fix / block_sort)
+  const int* cbeg = a.cstart + R.cell0;  // absolute first slot (k_rb_sort / block_sort)
   const int* ccnt = a.cnt + R.cell0;
   // units of work: cells (of the replica, or from the tile's first to its last
   // particle's: keys ascend along the slots), or four particles each for all
@@ -2804,7 +2773,7 @@ __device__ __forceinline__ int block_excl_scan(int x, int* s_w, int* total) {
 }
 
 // The stable cell-key sort of one replica by the calling block, the same
-// permutation as the sort kernels (k_rb_clear .. k_rb_permute; RUMD's
+// permutation as the sort kernels (k_rb_sort; RUMD's
 // thrust::sort_by_key on (cell key, current slot), Sample.h:174-188):
 // count with an arrival rank per cell, exclusive scan of the counts into
 // absolute cell starts, scatter, order each bucket by current slot, gather
@@ -2976,7 +2945,7 @@ __device__ __noinline__ void block_sort(const EngArgs& a, int rep, unsigned epoc
     }
   }
   if (tid == 0) {
-    S->actual_max_nbrs = 0;  // the per-build maximum (k_rb_clear)
+    S->actual_max_nbrs = 0;  // the per-build maximum (as k_rb_sort)
     __threadfence();
     st_release_u32(&S->sort_done, epoch);
   }
@@ -3381,7 +3350,7 @@ __global__ void __maxnreg__(64) k_batch(EngArgs a, cudaGraphConditionalHandle h_
               // the last item: flip the parities, reset the count, publish
               S->rbuf = (s_max & 1) ^ 1;
               S->abuf = (s_max >> 1) ^ 1;
-              S->actual_max_nbrs = 0;  // the per-build maximum (k_rb_clear)
+              S->actual_max_nbrs = 0;  // the per-build maximum (as k_rb_sort)
               S->sort_items = 0u;
               __threadfence();
               st_release_u32(&S->sort_done, epoch);
@@ -3673,7 +3642,7 @@ __global__ void __maxnreg__(64) k_flow(EngArgs a, cudaGraphConditionalHandle h_l
         if (threadIdx.x == 0) {
           if (kind == kFlowSplit && phase == 4u) {
             // the sort is complete: flip the parities (the per-build maximum
-            // starts again, as k_rb_clear does)
+            // starts again, as in k_rb_sort)
             S->rbuf = (s_max & 1) ^ 1;
             S->abuf = (s_max >> 1) ^ 1;
             S->actual_max_nbrs = 0;
