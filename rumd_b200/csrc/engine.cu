@@ -890,9 +890,10 @@ void launch_rebuild(b2md_engine* e, cudaStream_t s, const EngArgs& a) {
   // exceed a block), the list either assembled in shared memory or stored
   // straight to global memory
   if (e->build_lanes == 0 && !a.win_on) {
-    // one warp per cell; with few tiles, as many blocks per tile as the GPU
-    // holds at once and the tile has cells for (about three particles each)
-    const int parts = std::max(1, std::min(e->nsm * 8 / T, e->pb / (3 * kRunWarps)));
+    // one warp per cell; with few tiles, several blocks per tile: up to 16 per
+    // SM (twice what is resident, so that none runs dry) and no more than the
+    // tile has cells for (about three particles each)
+    const int parts = std::max(1, std::min(e->nsm * 16 / T, e->pb / (3 * kRunWarps)));
     k_rb_build_runs<<<T * parts, kRunWarps * 32, 0, s>>>(a, parts);
     return;
   }

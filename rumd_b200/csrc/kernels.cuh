@@ -52,30 +52,24 @@ __device__ __forceinline__ void block_sum8(double (&v)[kNPart], double* s_warp, 
   __syncthreads();
 }
 
-// Ordered strided sum of count rows of kNPart doubles (deterministic).
-__device__ __forceinline__ void block_rows_sum(const double* base, int count, double* s_scr, double* s_out) {
-  const int nslot = blockDim.x / kNPart;
-  const int k = threadIdx.x % kNPart, slot = threadIdx.x / kNPart;
+// Sum of count rows of kNPart doubles by one warp: lane 8 q + k adds column k
+// of rows q, q + 4, ... in order (eight rows' loads in flight), then the four
+// partial sums are added; every lane with the same k returns column k's total.
+__device__ __forceinline__ double warp_rows_sum(const double* base, int count) {
+  const int lane = threadIdx.x & 31;
+  const double* p = base + lane;  // row q, column k
   double acc = 0.0;
-  if (slot < nslot) {
-    // two rows' loads in flight at a time (the sum stays in row order)
-    int t = slot;
-    for (; t + nslot < count; t += 2 * nslot) {
-      const double x0 = __ldcg(base + (size_t)t * kNPart + k);
-      const double x1 = __ldcg(base + (size_t)(t + nslot) * kNPart + k);
-      acc += x0;
-      acc += x1;
-    }
-    if (t < count) acc += __ldcg(base + (size_t)t * kNPart + k);
+#pragma unroll 1
+  for (int t = lane >> 3; t < count; t += 32, p += 32 * kNPart) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = t + 4 * u < count ? __ldcg(p + 4 * u * kNPart) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc += x[u];
   }
-  s_scr[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x < kNPart) {
-    double s = 0.0;
-    for (int q = 0; q < nslot; ++q) s += s_scr[q * kNPart + threadIdx.x];
-    s_out[threadIdx.x] = s;
-  }
-  __syncthreads();
+  acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+  return acc;
 }
 
 // atomicAdd with release (the block's earlier writes, ordered before by a
@@ -90,9 +84,9 @@ __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
 
 // Two-level deterministic replica reduction.  Every block of the replica
 // calls it with its block totals in s_blk; returns true in exactly one block
-// (the last to finish) with the replica totals in s_tot.
-__device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int lt,
-                               const double* s_blk, double* s_scr, double* s_tot) {
+// (the last to finish) with the replica totals in s_tot.  A replica of one
+// group needs the first level only.
+__device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int lt, const double* s_blk, double* s_tot) {
   __shared__ int s_last;
   const int g = lt / kGroup;
   const int gfirst = g * kGroup;
@@ -105,30 +99,36 @@ __device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int l
   }
   __syncthreads();
   if (!s_last) return false;
-  block_rows_sum(a.tpart + (size_t)(R.tile0 + gfirst) * kNPart, gsize, s_scr, s_tot);
-  if (threadIdx.x < kNPart) a.gpart[(size_t)(R.group0 + g) * kNPart + threadIdx.x] = s_tot[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  double x = 0.0;
+  if (threadIdx.x < 32) x = warp_rows_sum(a.tpart + (size_t)(R.tile0 + gfirst) * kNPart, gsize);
+  if (R.ngroups > 1) {
+    if (threadIdx.x < kNPart) a.gpart[(size_t)(R.group0 + g) * kNPart + threadIdx.x] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atom_add_acq_rel(&a.rctr[rep], 1u) == (unsigned)(R.ngroups - 1);
+    __syncthreads();
+    if (threadIdx.x == 0) a.gctr[R.group0 + g] = 0u;
+    if (!s_last) return false;
+    if (threadIdx.x == 0) a.rctr[rep] = 0u;
+    if (threadIdx.x < 32) x = warp_rows_sum(a.gpart + (size_t)R.group0 * kNPart, R.ngroups);
+  } else if (threadIdx.x == 0) {
     a.gctr[R.group0 + g] = 0u;
-    unsigned c = atom_add_acq_rel(&a.rctr[rep], 1u);
-    s_last = (c == (unsigned)(R.ngroups - 1));
   }
+  if (threadIdx.x < kNPart) s_tot[threadIdx.x] = x;
   __syncthreads();
-  if (!s_last) return false;
-  block_rows_sum(a.gpart + (size_t)R.group0 * kNPart, R.ngroups, s_scr, s_tot);
-  if (threadIdx.x == 0) a.rctr[rep] = 0u;
   return true;
 }
 
-// The replica reduction of k_steps, run by every block after its step-barrier
-// arrival, on the step's half (par) of the partial-sum and counter buffers:
-// the tile's group counter, then (last block of the group) the group total
-// and the replica counter.  Returns true in the replica's last block, which
-// then sums the group totals and finishes the step; the other blocks have
-// gone on to the next step and wait for that only before they integrate.
-__device__ bool post_reduce(const EngArgs& a, int tile, int rep, const RepDev& R, int par, double* s_scr,
-                            double* s_tot) {
-  __shared__ int s_last;
+// The replica reduction of k_steps, run by warp 0 of every block after its
+// step-barrier arrival, on the step's half (par) of the partial-sum and
+// counter buffers: the same sums.  True in warp 0 of the replica's last block,
+// which then finishes the step; the other blocks have gone on to the next step
+// and wait for that only before they integrate.  The chain of L2 round trips
+// from a step's last tile to the replica totals bounds a small replica's step;
+// one warp walks it without block barriers.
+__device__ __forceinline__ bool post_reduce(const EngArgs& a, int tile, int rep, const RepDev& R, int par,
+                                            double* s_tot) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const int lt = tile - R.tile0;
   const int g = lt / kGroup;
   const int gfirst = g * kGroup;
@@ -137,24 +137,23 @@ __device__ bool post_reduce(const EngArgs& a, int tile, int rep, const RepDev& R
   unsigned* rctr = a.rctr + (size_t)par * a.rctr_half;
   double* gpart = a.gpart + (size_t)par * a.gpart_half;
   const double* tpart = a.tpart + (size_t)par * a.tpart_half;
-  if (threadIdx.x == 0) {
-    unsigned c = atom_add_acq_rel(&gctr[R.group0 + g], 1u);
-    s_last = (c == (unsigned)(gsize - 1));
+  unsigned last = 0u;
+  if (lane == 0) last = atom_add_acq_rel(&gctr[R.group0 + g], 1u) == (unsigned)(gsize - 1);
+  __syncwarp();
+  if (!__shfl_sync(FULL, last, 0)) return false;
+  if (lane == 0) gctr[R.group0 + g] = 0u;
+  double x = warp_rows_sum(tpart + (size_t)(R.tile0 + gfirst) * kNPart, gsize);
+  if (R.ngroups > 1) {
+    if (lane < kNPart) gpart[(size_t)(R.group0 + g) * kNPart + lane] = x;
+    __syncwarp();  // the lanes' stores before lane 0's release
+    if (lane == 0) last = atom_add_acq_rel(&rctr[rep], 1u) == (unsigned)(R.ngroups - 1);
+    __syncwarp();
+    if (!__shfl_sync(FULL, last, 0)) return false;
+    if (lane == 0) rctr[rep] = 0u;
+    x = warp_rows_sum(gpart + (size_t)R.group0 * kNPart, R.ngroups);
   }
-  __syncthreads();
-  if (!s_last) return false;
-  block_rows_sum(tpart + (size_t)(R.tile0 + gfirst) * kNPart, gsize, s_scr, s_tot);
-  if (threadIdx.x < kNPart) gpart[(size_t)(R.group0 + g) * kNPart + threadIdx.x] = s_tot[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    gctr[R.group0 + g] = 0u;
-    unsigned c = atom_add_acq_rel(&rctr[rep], 1u);
-    s_last = (c == (unsigned)(R.ngroups - 1));
-    if (s_last) rctr[rep] = 0u;
-  }
-  __syncthreads();
-  if (!s_last) return false;
-  block_rows_sum(gpart + (size_t)R.group0 * kNPart, R.ngroups, s_scr, s_tot);
+  if (lane < kNPart) s_tot[lane] = x;
+  __syncwarp();
   return true;
 }
 
@@ -783,7 +782,7 @@ __device__ __forceinline__ void force_loop_any(unsigned wrap, int pot, int nt, P
 // neighbour loop the block reduction's scratch (force_red_bytes) overlays it.
 constexpr int kParSmemFloats = kMaxTypes * kMaxTypes * kParStride;
 __host__ __device__ constexpr int force_red_bytes(int threads) {
-  return ((threads + 31) / 32) * kNPart * (int)sizeof(double) + threads * (int)sizeof(double);
+  return ((threads + 31) / 32) * kNPart * (int)sizeof(double);
 }
 // k_steps keeps the pair table (of the engine's largest type count) at the
 // start of its dynamic shared memory; the reduction scratch follows it.
@@ -858,7 +857,6 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
   // every thread is past the neighbour loop (force_red_bytes); in k_steps it
   // follows the pair table, which stays loaded for the whole launch
   double* s_warp = reinterpret_cast<double*>(s_dyn + (PERSIST ? persist_table_bytes(a) : 0));
-  double* s_scr = s_warp + (blockDim.x >> 5) * kNPart;
   const int rep = a.tile_rep[tile];
   // PERSIST: k_steps' shared-memory copy of the replica's descriptor
   const RepDev& R = PERSIST ? *prep : a.rep[rep];
@@ -1107,7 +1105,7 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
     } else {
       if (FUSED && ex && threadIdx.x == 0) atomicAdd(&S->exceed, 1);
       block_sum8(acc, s_warp, s_blk);
-      if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_scr, s_tot)) {
+      if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_tot)) {
         if (FUSED) {
           finish_step(a, rep, R, S, s_tot, true, bpar);
         } else if (threadIdx.x == 0) {
@@ -1340,7 +1338,6 @@ __global__ void __maxnreg__(72) k_steps(EngArgs a, cudaGraphConditionalHandle h_
       }
     }
   }
-  double* s_red = reinterpret_cast<double*>(s_dyn + persist_table_bytes(a)) + (blockDim.x >> 5) * kNPart;
   for (int step = 0; s_go; ++step) {
     if (threadIdx.x == 0) {
       s_step_tally = 0ull;
@@ -1352,20 +1349,24 @@ __global__ void __maxnreg__(72) k_steps(EngArgs a, cudaGraphConditionalHandle h_
       stepped = force_tile<TP, true, false, FM_STREAMED, true>(a, tile, s_dyn, s_blk, s_tot, s_bar, s_rows, &s_view,
                                                                step & 1, &s_rep, &pr, &s_wdone);
     budget -= 1;
-    __syncthreads();  // the tile's partial sums are written
-    unsigned long long now = 0ull;
-    if (threadIdx.x == 0) now = step_arrive(a, step);
-    // the replica reduction and the step's finish, between the arrival and
-    // the barrier's completion
-    if (stepped && post_reduce(a, tile, rep_id, s_rep, step & 1, s_red, s_tot))
-      finish_step_persist(a, s_rep, a.st + rep_id, s_tot);
-    if (threadIdx.x == 0) {
-      s_go = step_decide(a, step, budget, seen, now, h_loop);
-      if (stepped) {
-        s_view.rbuf ^= 1;
-        if (s_view.steps_left > 0) s_view.steps_left -= 1;
-        s_view.run_step += 1;
-        s_view.steps += 1;
+    // warp 0 goes on alone: every thread's positions were written before the
+    // block sum's barrier, the tile's partial sums by this warp
+    if (threadIdx.x < 32) {
+      __syncwarp();
+      unsigned long long now = 0ull;
+      if (threadIdx.x == 0) now = step_arrive(a, step);
+      // the replica reduction and the step's finish, between the arrival and
+      // the barrier's completion
+      if (stepped && post_reduce(a, tile, rep_id, s_rep, step & 1, s_tot))
+        finish_step_persist(a, s_rep, a.st + rep_id, s_tot);
+      if (threadIdx.x == 0) {
+        s_go = step_decide(a, step, budget, seen, now, h_loop);
+        if (stepped) {
+          s_view.rbuf ^= 1;
+          if (s_view.steps_left > 0) s_view.steps_left -= 1;
+          s_view.run_step += 1;
+          s_view.steps += 1;
+        }
       }
     }
     __syncthreads();
@@ -1393,7 +1394,6 @@ __global__ void k_gate_loop(EngArgs a, cudaGraphConditionalHandle h_loop) {
 // hence every bit of the result) is the same as the fused step's.
 __global__ void __launch_bounds__(kMaxBlock) k_integrate(EngArgs a, int tp) {
   __shared__ double s_warp[(kMaxBlock / 32) * kNPart];
-  __shared__ double s_scr[kMaxBlock];
   __shared__ double s_blk[kNPart], s_tot[kNPart];
   const int tile = blockIdx.x;
   const int rep = a.tile_rep[tile];
@@ -1419,7 +1419,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate(EngArgs a, int tp) {
   const int ex = __syncthreads_or(exceed);
   if (ex && threadIdx.x == 0) atomicAdd(&S->exceed, 1);
   block_sum8(acc, s_warp, s_blk);
-  if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_scr, s_tot)) {
+  if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_tot)) {
     if (threadIdx.x == 0) {
       double pe = S->pe, vir = S->vir;
       finish_step(a, rep, R, S, s_tot, false);
@@ -1433,7 +1433,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate(EngArgs a, int tp) {
 // Tiles tile0 .. tile0 + gridDim.x - 1 (all tiles, or one replica's).
 __global__ void __launch_bounds__(kMaxBlock) k_momentum(EngArgs a, int tp, int tile0) {
   __shared__ double s_warp[(kMaxBlock / 32) * kNPart];
-  __shared__ double s_scr[kMaxBlock];
   __shared__ double s_blk[kNPart], s_tot[kNPart];
   const int tile = tile0 + blockIdx.x;
   const int rep = a.tile_rep[tile];
@@ -1450,7 +1449,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_momentum(EngArgs a, int tp, int t
     acc[P_PX] = m * v.x; acc[P_PY] = m * v.y; acc[P_PZ] = m * v.z; acc[P_M] = m;
   }
   block_sum8(acc, s_warp, s_blk);
-  if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_scr, s_tot)) {
+  if (replica_reduce(a, rep, R, tile - R.tile0, s_blk, s_tot)) {
     if (threadIdx.x == 0) {
       S->P[0] = s_tot[P_PX]; S->P[1] = s_tot[P_PY]; S->P[2] = s_tot[P_PZ]; S->M = s_tot[P_M];
     }
@@ -1537,7 +1536,6 @@ __global__ void __launch_bounds__(256) k_write_sort(EngArgs a, int rep, long lon
 // FP32 terms added in FP64 (block_sum8 and replica_reduce's fixed tree).
 __global__ void __launch_bounds__(kMaxBlock) k_stress(EngArgs a, int rep, int kinetic, double* out6) {
   __shared__ double s_warp[(kMaxBlock / 32) * kNPart];
-  __shared__ double s_scr[kMaxBlock];
   __shared__ double s_blk[kNPart], s_tot[kNPart];
   const RepDev& R = a.rep[rep];
   const int i = a.tile_first[R.tile0 + blockIdx.x] + threadIdx.x;
@@ -1556,7 +1554,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_stress(EngArgs a, int rep, int ki
     }
   }
   block_sum8(acc, s_warp, s_blk);
-  if (replica_reduce(a, rep, R, blockIdx.x, s_blk, s_scr, s_tot) && threadIdx.x < 6) out6[threadIdx.x] = s_tot[threadIdx.x];
+  if (replica_reduce(a, rep, R, blockIdx.x, s_blk, s_tot) && threadIdx.x < 6) out6[threadIdx.x] = s_tot[threadIdx.x];
 }
 
 // Original particle ids 0..n-1 (a replica's slot order before its first sort).
@@ -1677,9 +1675,9 @@ __device__ bool sort_barrier(PersistCtl* c) {
 // needs no rebuild pays one launch for it.  The phases are a microsecond or
 // two of latency each, so the number of launches and of blocks that meet is
 // what costs: as seven kernels of a block per tile the sort took 37 us at KA
-// N=65536 (ncu, 4.6 to 9.5 us each), as one launch 11 us less of the rebuild (119 -> 111 us with the
-// build at KA N=65536), and a force evaluation without a rebuild launches two
-// kernels instead of eight.
+// N=65536 (ncu, 4.6 to 9.5 us each); as one launch a rebuild takes 111 us
+// instead of 115 there, 985 instead of 1042 at LJ N = 2^20, and a force
+// evaluation without a rebuild launches two kernels instead of eight.
 constexpr int kScanGroup = 128;
 constexpr int kSortBlock = 512;
 __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
@@ -2498,16 +2496,29 @@ __device__ __forceinline__ int build_cell(const RepDev& R, const float4* rc, con
     cnt[q] = 0u;
   }
   int rows = 0;  // non-empty rows that start before this round
-#pragma unroll 1
-  for (int ch = 0; ch < cr.total; ch += 32) {
+  // the round's candidate (slot; one past the last repeats the cell's first
+  // particle): the next round's is loaded while the current one is tested
+  // (the chain row mask - table - position bounds a round; a rebuild at KA
+  // N=65536 120 -> 111 us, with twice the blocks in flight 103)
+  auto candidate = [&](int ch) -> int {
     const int v = ch + lane;
     const unsigned rel = (unsigned)(cr.off - ch);
     const unsigned st = __reduce_or_sync(FULL, cr.len > 0 && rel < 32u ? 1u << rel : 0u);
     const int4 t = cr.tab[rows + __popc(st & (lt + lt + 1u)) - 1];
     rows += __popc(st);
-    const bool have = v < cr.total;
-    const int j = have ? v + (v < t.z ? t.y : t.w) : pg;
-    const float4 rj = COH ? ld_ca_f4(rc + j) : __ldg(rc + j);
+    return v < cr.total ? v + (v < t.z ? t.y : t.w) : pg;
+  };
+  int jn = candidate(0);
+  float4 rn = COH ? ld_ca_f4(rc + jn) : __ldg(rc + jn);
+#pragma unroll 1
+  for (int ch = 0; ch < cr.total; ch += 32) {
+    const int j = jn;
+    const float4 rj = rn;
+    const bool have = ch + lane < cr.total;
+    if (ch + 32 < cr.total) {
+      jn = candidate(ch + 32);
+      rn = COH ? ld_ca_f4(rc + jn) : __ldg(rc + jn);
+    }
     const int tj = __float_as_int(rj.w);
     float dx[G], dy[G], dz[G];
 #pragma unroll
