@@ -360,6 +360,19 @@ char* stage_alloc(b2md_engine* e, size_t bytes) {
   return e->ring + lo;
 }
 
+// A region of the staging ring for a read-back, given back at the end of the
+// call, by when the stream has been waited for.
+struct ReadStage {
+  b2md_engine* e;
+  size_t head;
+  char* p;
+  ReadStage(b2md_engine* eng, size_t bytes) : e(eng), head(eng->ring_head), p(stage_alloc(eng, bytes)) {}
+  void done() {
+    e->ring_open.pop_back();
+    e->ring_head = head;
+  }
+};
+
 // Why valid step graphs were dropped (b2md_engine_counters).
 enum { INV_OTHER = 0, INV_LAYOUT = 1, INV_POOL = 2, INV_REPAIR = 3, INV_REASONS = 4 };
 
@@ -656,19 +669,28 @@ HostRep& get_rep(b2md_engine* e, int id) {
   return e->reps[id];
 }
 
-RepState read_state(b2md_engine* e, int id) {
-  RepState s;
-  CK(cudaMemcpyAsync(&s, e->st + id, sizeof(RepState), cudaMemcpyDeviceToHost, e->stream));
+// The states of all replicas after what is queued (and, with err, the
+// persistent kernels' error word): one wait.
+std::vector<RepState> read_states(b2md_engine* e, int* err = nullptr) {
+  std::vector<RepState> s(e->reps.size());
+  const size_t nb = s.size() * sizeof(RepState);
+  ReadStage st(e, nb + sizeof(int));
+  if (nb) CK(cudaMemcpyAsync(st.p, e->st, nb, cudaMemcpyDeviceToHost, e->stream));
+  if (err) CK(cudaMemcpyAsync(st.p + nb, &e->pctl->err, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
   CK(cudaStreamSynchronize(e->stream));
+  if (nb) std::memcpy(s.data(), st.p, nb);
+  if (err) std::memcpy(err, st.p + nb, sizeof(int));
+  st.done();
   return s;
 }
 
-std::vector<RepState> read_states(b2md_engine* e) {
-  std::vector<RepState> s(e->reps.size());
-  if (!s.empty()) {
-    CK(cudaMemcpyAsync(s.data(), e->st, s.size() * sizeof(RepState), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-  }
+RepState read_state(b2md_engine* e, int id) {
+  RepState s;
+  ReadStage st(e, sizeof s);
+  CK(cudaMemcpyAsync(st.p, e->st + id, sizeof s, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  std::memcpy(&s, st.p, sizeof s);
+  st.done();
   return s;
 }
 
@@ -1324,9 +1346,10 @@ void ensure_graphs(b2md_engine* e) {
 }
 
 // A step-barrier wait of k_steps that gave up (reported, then cleared).
-void check_persist(b2md_engine* e) {
+void check_persist(b2md_engine* e, const int* known = nullptr) {
   int err = 0;
-  CK(cudaMemcpy(&err, &e->pctl->err, sizeof(int), cudaMemcpyDeviceToHost));
+  if (known) err = *known;
+  else CK(cudaMemcpy(&err, &e->pctl->err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
     CK(cudaMemset(&e->pctl->err, 0, sizeof(int)));
     api_fail(B2MD_ERR_CUDA, "a step-barrier wait of the persistent step kernel gave up");
@@ -1334,8 +1357,7 @@ void check_persist(b2md_engine* e) {
 }
 
 // Overflowed lists: double the capacity (NeighborList.cu:657-676) and flag a rebuild.
-bool repair_overflow(b2md_engine* e) {
-  std::vector<RepState> s = read_states(e);
+bool repair_overflow(b2md_engine* e, const std::vector<RepState>& s) {
   bool any = false;
   for (size_t r = 0; r < e->reps.size(); ++r)
     if (e->reps[r].active && s[r].err)
@@ -1369,44 +1391,48 @@ void calc_f(b2md_engine* e, bool stress) {
     launch_rebuild(e, e->stream, a);
     launch_force(e, e->stream, a, false, stress);
     check_launch();
-    if (!repair_overflow(e)) return;
+    if (!repair_overflow(e, read_states(e))) return;
   }
   api_fail(B2MD_ERR_OVERFLOW, "neighbour list overflow persists");
 }
 
-long long max_steps_left(b2md_engine* e) {
-  std::vector<RepState> s = read_states(e);
+long long max_steps_left(const b2md_engine* e, const std::vector<RepState>& s) {
   long long m = 0;
   for (size_t r = 0; r < e->reps.size(); ++r)
     if (e->reps[r].active && !s[r].overflow) m = std::max(m, s[r].steps_left);
   return m;
 }
 
-// Runs up to `limit` steps of the queued work with the step graphs.
-long long run_steps(b2md_engine* e, long long limit) {
+// Runs up to `limit` steps of the queued work with the step graphs.  known:
+// the longest queue, when the caller has just set it.  The replicas' states
+// are read once after each launch, for all that the host decides from them.
+long long run_steps(b2md_engine* e, long long limit, long long known = -1) {
   ensure_layout(e);
   long long done = 0;
   for (int guard = 0; guard < 64; ++guard) {
-    long long todo = std::min(max_steps_left(e), limit - done);
+    const long long left = known >= 0 ? known : max_steps_left(e, read_states(e));
+    known = -1;
+    long long todo = std::min(left, limit - done);
     if (todo <= 0) break;
     ensure_graphs(e);
+    int err = 0;
     if (e->persist_on) {
       todo = std::min<long long>(todo, 1 << 30);
       *e->h_budget = (int)todo;
       CK(cudaMemcpyAsync(&e->pctl->budget, e->h_budget, sizeof(int), cudaMemcpyHostToDevice, e->stream));
       CK(cudaGraphLaunch(e->gexec[2], e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      check_persist(e);
     } else {
       long long big = todo / kChunk, small = todo % kChunk;
       for (long long k = 0; k < big; ++k) CK(cudaGraphLaunch(e->gexec[1], e->stream));
       for (long long k = 0; k < small; ++k) CK(cudaGraphLaunch(e->gexec[0], e->stream));
-      CK(cudaStreamSynchronize(e->stream));
     }
+    const std::vector<RepState> s = read_states(e, e->persist_on ? &err : nullptr);
+    if (e->persist_on) check_persist(e, &err);
     done += todo;
-    if (!repair_overflow(e)) {
+    if (!repair_overflow(e, s)) {
       // replicas that were frozen by an overflow keep their queue; others are done
-      if (max_steps_left(e) == 0) break;
+      known = max_steps_left(e, s);
+      if (known == 0) break;
     }
     done = std::min(done, limit);
   }
@@ -1564,19 +1590,6 @@ void write_field4(b2md_engine* e, int id, HostRep& h, unsigned what, const float
   check_launch();
   stage_commit(e);
 }
-
-// A region of the staging ring for a read-back, given back at the end of the
-// call, by when the stream has been waited for.
-struct ReadStage {
-  b2md_engine* e;
-  size_t head;
-  char* p;
-  ReadStage(b2md_engine* eng, size_t bytes) : e(eng), head(eng->ring_head), p(stage_alloc(eng, bytes)) {}
-  void done() {
-    e->ring_open.pop_back();
-    e->ring_head = head;
-  }
-};
 
 // Fields of replica id to the caller's arrays, in the caller's order (vel also
 // receives the field src).  Everything the engine has queued before is
@@ -2157,7 +2170,20 @@ int b2md_replica_stats(b2md_engine* e, int id, double* out) {
     HostRep& h = get_rep(e, id);
     CK(cudaSetDevice(e->device));
     ensure_layout(e);
-    RepState s = read_state(e, id);
+    ReadStage stage(e, sizeof(ReplicaStats));
+    ReplicaStats* rs = reinterpret_cast<ReplicaStats*>(stage.p);
+    const int blocks = std::min(kStatBlocks, (h.n + 1023) / 1024);
+    k_replica_stats<<<blocks, 256, 0, e->stream>>>(make_args(e), id, h.p0, h.n, h.d.tile0, h.d.ntiles, rs);
+    check_launch();
+    CK(cudaStreamSynchronize(e->stream));
+    const RepState s = rs->st;
+    unsigned long long nn = 0;
+    int wt = 0;  // tiles whose neighbours k_force reads from a position window
+    for (int k = 0; k < blocks; ++k) {
+      nn += rs->nn[k];
+      wt += rs->windows[k];
+    }
+    stage.done();
     out[B2MD_STAT_PE] = s.pe;
     out[B2MD_STAT_VIRIAL] = s.vir;
     out[B2MD_STAT_KE] = s.ke_t;
@@ -2170,21 +2196,7 @@ int b2md_replica_stats(b2md_engine* e, int id, double* out) {
     out[B2MD_STAT_TARGET_T] = s.T;
     out[B2MD_STAT_MAX_NBRS] = h.d.max_nbrs;
     out[B2MD_STAT_ACTUAL_MAX_NBRS] = s.actual_max_nbrs;
-    std::vector<unsigned> nn(h.n);
-    CK(cudaMemcpyAsync(nn.data(), e->nn + h.p0, h.n * sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    double tot = 0;
-    for (unsigned c : nn) tot += c;
-    out[B2MD_STAT_MEAN_NBRS] = tot / h.n;
-    // tiles whose neighbours k_force reads from a position window
-    int wt = 0;
-    if (e->force_mode == FM_WINDOW && h.d.ntiles > 0) {
-      std::vector<int2> wm(h.d.ntiles);
-      CK(cudaMemcpyAsync(wm.data(), e->wmeta + h.d.tile0, h.d.ntiles * sizeof(int2), cudaMemcpyDeviceToHost,
-                         e->stream));
-      CK(cudaStreamSynchronize(e->stream));
-      for (const int2& m : wm) wt += m.x >= 0;
-    }
+    out[B2MD_STAT_MEAN_NBRS] = (double)nn / h.n;
     out[B2MD_STAT_WINDOW_TILES] = wt;
     out[B2MD_STAT_TILES] = h.d.ntiles;
   });
@@ -2214,9 +2226,11 @@ int b2md_replica_set_energy_log(b2md_engine* e, int id, int interval, int capaci
       h.d.energy_cap = capacity;
       h.d.energy_interval = interval;
     }
+    // (the step graphs read the log's place from the replica table; a pool
+    // growth has dropped them already.  Instantiating them again took 300 us of
+    // every Simulation.Run.)
     upload_rep(e, id);
     WRITE_STATE(e, id, nlog, 0);
-    invalidate_graphs(e);
   });
 }
 
@@ -2311,7 +2325,7 @@ int b2md_run(b2md_engine* e, long long nsteps) {
     check_launch();
     // every queue holds exactly nsteps; run until all are empty (a replica
     // frozen by a list overflow catches up after its repair)
-    if (nsteps > 0) run_steps(e, 1LL << 62);
+    if (nsteps > 0) run_steps(e, 1LL << 62, nsteps);
     calc_f(e, false);
     CK(cudaStreamSynchronize(e->stream));
   });
@@ -2372,12 +2386,12 @@ int b2md_run_timed(b2md_engine* e, long long nsteps, double* step_kernel_ms, lon
         tot += ms;
         nl += 1;
         budget = *h_left;
-        if (repair_overflow(e)) {
+        if (repair_overflow(e, read_states(e))) {
           a = make_args(e);  // the repaired list moved
           bsmem = flow ? flow_smem(e, a) : batch_smem(e, a);
           continue;
         }
-        if (max_steps_left(e) == 0) break;
+        if (max_steps_left(e, read_states(e)) == 0) break;
       }
       cudaFreeHost(h_left);
       cudaEventDestroy(e0);
@@ -2427,12 +2441,12 @@ int b2md_run_timed(b2md_engine* e, long long nsteps, double* step_kernel_ms, lon
           nl += 1;
           const int ran = budget - *h_left;
           budget = *h_left;
-          if (ran <= 0 || max_steps_left(e) == 0) break;  // no replica has steps left
+          if (ran <= 0 || max_steps_left(e, read_states(e)) == 0) break;  // no replica has steps left
         }
         cudaFreeHost(h_left);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (repair_overflow(e)) run_steps(e, nsteps);
+        if (repair_overflow(e, read_states(e))) run_steps(e, nsteps);
         calc_f(e, false);
         CK(cudaStreamSynchronize(e->stream));
         *step_kernel_ms = tot;
@@ -2471,7 +2485,7 @@ int b2md_run_timed(b2md_engine* e, long long nsteps, double* step_kernel_ms, lon
       tot += ms;
     }
     for (auto& x : ev) cudaEventDestroy(x);
-    if (repair_overflow(e)) run_steps(e, nsteps);
+    if (repair_overflow(e, read_states(e))) run_steps(e, nsteps);
     calc_f(e, false);
     CK(cudaStreamSynchronize(e->stream));
     *step_kernel_ms = tot;
@@ -2539,7 +2553,7 @@ int b2md_run_queued_async(b2md_engine* e, long long max_steps, long long* ticket
         CK(cudaGraphLaunch(e->gexec[2], e->stream));
       } else {
         // per-step graphs: the queue lengths decide how many (read first)
-        const long long todo = std::min(max_steps_left(e), lim);
+        const long long todo = std::min(max_steps_left(e, read_states(e)), lim);
         for (long long k = 0; k < todo / kChunk; ++k) CK(cudaGraphLaunch(e->gexec[1], e->stream));
         for (long long k = 0; k < todo % kChunk; ++k) CK(cudaGraphLaunch(e->gexec[0], e->stream));
         c.budget = todo;

@@ -42,6 +42,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -494,6 +495,20 @@ __global__ void __launch_bounds__(kB) k64_finish(F64Args a) {
   a.st->W = s_out[1] / 6.0;
 }
 
+// A field in the caller's order in the list build's scratch arrays (idle
+// between builds): 32-byte vectors, or images as 3 ints.
+__global__ void __launch_bounds__(kB) k64_unsort(F64Args a, const double4* src, double4* out, int* images) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const size_t o = a.uid[i];
+  if (src) {
+    out[o] = src[i];
+  } else {
+    const int4 im = a.im[i];
+    images[3 * o] = im.x; images[3 * o + 1] = im.y; images[3 * o + 2] = im.z;
+  }
+}
+
 __global__ void __launch_bounds__(kB) k64_iota(unsigned* ids, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) ids[i] = (unsigned)i;
@@ -514,6 +529,8 @@ struct b2md_f64 {
   double* elog = nullptr;  // energies of a run, kept for the next
   long long elog_cap = 0;
   std::vector<void*> bufs;
+  double4* scratch = nullptr;  // the list build's per-particle scratch: im2, uid2, cell, rank, order
+  void* pinned = nullptr;      // read-backs pass through it (32 bytes per particle)
 };
 
 namespace {
@@ -655,9 +672,8 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
   h->rb_grid = (int)std::max(1LL, std::min((long long)sms * std::min(per_sm, 2), (8LL * n + kB - 1) / kB));
   const size_t nb = (size_t)((n + kB - 1) / kB), rows = ((size_t)a.max_nbrs + 3) / 4 * 4;
   if ((rc = f64_alloc(h, a.r, n)) || (rc = f64_alloc(h, a.v, n)) || (rc = f64_alloc(h, a.f, n)) ||
-      (rc = f64_alloc(h, a.last_r, n)) || (rc = f64_alloc(h, a.im, n)) || (rc = f64_alloc(h, a.im2, n)) ||
-      (rc = f64_alloc(h, a.uid, n)) || (rc = f64_alloc(h, a.uid2, n)) || (rc = f64_alloc(h, a.cell, n)) ||
-      (rc = f64_alloc(h, a.rank, n)) || (rc = f64_alloc(h, a.order, n)) || (rc = f64_alloc(h, a.cnt, a.ncell)) ||
+      (rc = f64_alloc(h, a.last_r, n)) || (rc = f64_alloc(h, a.im, n)) || (rc = f64_alloc(h, h->scratch, n)) ||
+      (rc = f64_alloc(h, a.uid, n)) || (rc = f64_alloc(h, a.cnt, a.ncell)) ||
       (rc = f64_alloc(h, a.cstart, a.ncell)) || (rc = f64_alloc(h, a.ctot, h->rb_grid)) ||
       (rc = f64_alloc(h, a.nn, n)) || (rc = f64_alloc(h, a.nbl, rows * n)) ||
       (rc = f64_alloc(h, a.part, nb * kNPartF64)) || (rc = f64_alloc(h, a.part_f, (size_t)a.fblocks * 2)) ||
@@ -665,6 +681,12 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
     return done(rc);
   a.st = h->st;
   a.par = h->par;
+  a.im2 = reinterpret_cast<int4*>(h->scratch);
+  a.uid2 = reinterpret_cast<unsigned*>(a.im2 + n);
+  a.cell = reinterpret_cast<int*>(a.uid2 + n);
+  a.rank = a.cell + n;
+  a.order = a.rank + n;
+  static_assert(sizeof(double4) == sizeof(int4) + 4 * sizeof(int), "the scratch arrays of a particle");
   if (cudaMemcpy(h->par, pars.data(), pars.size() * sizeof(F64Pair), cudaMemcpyHostToDevice) != cudaSuccess)
     return done(f64_fail(B2MD_ERR_CUDA, "b2md_f64_create: parameter upload failed"));
   F64Dev d0 = {};
@@ -680,6 +702,7 @@ int b2md_f64_destroy(b2md_f64* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->bufs) cudaFree(p);
   if (h->elog) cudaFree(h->elog);
+  if (h->pinned) cudaFreeHost(h->pinned);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return B2MD_OK;
@@ -796,25 +819,15 @@ int b2md_f64_get(b2md_f64* h, int field, void* out) {
   if (!h || !out) return f64_fail(B2MD_ERR_ARG, "b2md_f64_get: null argument");
   const int n = h->a.n;
   F64_CK(cudaSetDevice(h->device));
-  F64_CK(cudaStreamSynchronize(h->stream));
-  std::vector<unsigned> uid(n);
-  F64_CK(cudaMemcpy(uid.data(), h->a.uid, n * sizeof(unsigned), cudaMemcpyDeviceToHost));
-  if (field == B2MD_F64_POS || field == B2MD_F64_VEL || field == B2MD_F64_FORCE) {
-    const double4* src = field == B2MD_F64_POS ? h->a.r : (field == B2MD_F64_VEL ? h->a.v : h->a.f);
-    std::vector<double4> tmp(n);
-    F64_CK(cudaMemcpy(tmp.data(), src, n * sizeof(double4), cudaMemcpyDeviceToHost));
-    double4* o = static_cast<double4*>(out);
-    for (int i = 0; i < n; ++i) o[uid[i]] = tmp[i];
-    return B2MD_OK;
-  }
-  if (field == B2MD_F64_IMAGES) {
-    std::vector<int4> im(n);
-    F64_CK(cudaMemcpy(im.data(), h->a.im, n * sizeof(int4), cudaMemcpyDeviceToHost));
-    int* o = static_cast<int*>(out);
-    for (int i = 0; i < n; ++i) {
-      int* p = o + 3 * (size_t)uid[i];
-      p[0] = im[i].x; p[1] = im[i].y; p[2] = im[i].z;
-    }
+  if (field >= B2MD_F64_POS && field <= B2MD_F64_IMAGES) {
+    const double4* src = field == B2MD_F64_POS ? h->a.r : field == B2MD_F64_VEL ? h->a.v : field == B2MD_F64_FORCE ? h->a.f : nullptr;
+    const size_t bytes = (size_t)n * (src ? sizeof(double4) : 3 * sizeof(int));
+    if (!h->pinned) F64_CK(cudaMallocHost(&h->pinned, (size_t)n * sizeof(double4)));
+    k64_unsort<<<nblocks(h), kB, 0, h->stream>>>(h->a, src, h->scratch, reinterpret_cast<int*>(h->scratch));
+    F64_CK(cudaGetLastError());
+    F64_CK(cudaMemcpyAsync(h->pinned, h->scratch, bytes, cudaMemcpyDeviceToHost, h->stream));
+    F64_CK(cudaStreamSynchronize(h->stream));
+    std::memcpy(out, h->pinned, bytes);
     return B2MD_OK;
   }
   return f64_fail(B2MD_ERR_ARG, "b2md_f64_get: unknown field %d", field);

@@ -1532,6 +1532,46 @@ __global__ void __launch_bounds__(256) k_write_sort(EngArgs a, int rep, long lon
   if (what & kReadImages) a.im[ab][gi] = a.im[ab ^ 1][go];
 }
 
+// A replica's state and, per block, the sum of its list lengths and its tiles
+// that have a position window, to page-locked host memory.
+constexpr int kStatBlocks = 64;
+struct ReplicaStats {
+  RepState st;
+  unsigned long long nn[kStatBlocks];
+  int windows[kStatBlocks];
+};
+__global__ void __launch_bounds__(256) k_replica_stats(EngArgs a, int rep, long long p0, int n, int tile0, int ntiles,
+                                                       ReplicaStats* out) {
+  __shared__ unsigned long long s_nn[8];
+  __shared__ int s_w[8];
+  static_assert(sizeof(RepState) % sizeof(int) == 0, "state copied as words");
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < (int)(sizeof(RepState) / sizeof(int)); k += blockDim.x)
+      reinterpret_cast<int*>(&out->st)[k] = reinterpret_cast<const int*>(a.st + rep)[k];
+  unsigned long long nn = 0ull;
+  int w = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) nn += a.nn[p0 + i];
+  if (a.win_on)
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
+      w += a.wmeta[tile0 + t].x >= 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
+  w = __reduce_add_sync(0xffffffffu, w);
+  if ((threadIdx.x & 31) == 0) {
+    s_nn[threadIdx.x >> 5] = nn;
+    s_w[threadIdx.x >> 5] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) {
+      s_nn[0] += s_nn[k];
+      s_w[0] += s_w[k];
+    }
+    out->nn[blockIdx.x] = s_nn[0];
+    out->windows[blockIdx.x] = s_w[0];
+  }
+}
+
 // Sample::GetStress's sums (Sample.cu:393-444) of one replica: the particles'
 // FP32 terms added in FP64 (block_sum8 and replica_reduce's fixed tree).
 __global__ void __launch_bounds__(kMaxBlock) k_stress(EngArgs a, int rep, int kinetic, double* out6) {
