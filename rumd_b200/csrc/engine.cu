@@ -186,6 +186,7 @@ struct b2md_engine {
   // (admissions, layout uploads): a call fills a region and returns at once
   char* ring = nullptr;
   size_t ring_cap = 0, ring_head = 0;
+  std::vector<cudaEvent_t> read_ev;  // two per thread of a read-back
   std::vector<StageBlk> ring_pending;                  // regions with copies possibly in flight
   std::vector<std::pair<size_t, size_t>> ring_open;    // regions of the current call (no event yet)
   bool layout_dirty = false;     // admissions/removals since the last tile layout upload
@@ -251,31 +252,6 @@ void dev_grow(b2md_engine* e, T*& p, long long old_n, long long new_n, bool zero
     CK(cudaFree(p));
   }
   p = np;
-}
-
-// Copies from the pinned staging to the caller's memory, by four threads when
-// it is large: fresh pages are faulted in by the copy, which is most of it.
-void copy_out(void* dst, const void* src, size_t bytes) {
-  constexpr size_t kPerThread = (size_t)2 << 20;
-  const size_t nt = std::min<size_t>(4, bytes / kPerThread);
-  if (nt < 2) {
-    std::memcpy(dst, src, bytes);
-    return;
-  }
-  const size_t part = (bytes / nt + 4095) & ~(size_t)4095;
-  auto piece = [&](size_t k) {
-    const size_t b = std::min(bytes, k * part), e = std::min(bytes, b + part);
-    std::memcpy(static_cast<char*>(dst) + b, static_cast<const char*>(src) + b, e - b);
-  };
-  std::vector<std::thread> th;
-  size_t k = 1;
-  try {
-    for (; k < nt; ++k) th.emplace_back(piece, k);
-  } catch (const std::system_error&) {  // no thread to be had: the rest here
-  }
-  piece(0);
-  for (size_t q = k; q < nt; ++q) piece(q);
-  for (auto& t : th) t.join();
 }
 
 // Page-locked host memory (cudaMallocHost / cudaHostRegister): DMA-able as is.
@@ -1593,25 +1569,74 @@ void write_field4(b2md_engine* e, int id, HostRep& h, unsigned what, const float
 
 // Fields of replica id to the caller's arrays, in the caller's order (vel also
 // receives the field src).  Everything the engine has queued before is
-// finished when this returns.
+// finished when this returns.  The data passes in pieces through a region of
+// the staging ring that is there since the first admission (page-locking more
+// costs milliseconds); large results are copied out by four threads, each with
+// two pieces in turn, since faulting in the caller's fresh pages is most of it.
+constexpr size_t kReadRegion = (size_t)3 << 19;   // staging of a read-back
+constexpr size_t kReadThreads = (size_t)8 << 20;  // results from this size on are copied out by four threads
 void read_back(b2md_engine* e, int id, HostRep& h, unsigned what, const float4* src, void* pos, void* vel,
                void* images) {
   const size_t n = (size_t)h.n;
-  const size_t pb = pos ? n * sizeof(float4) : 0, vb = vel ? n * sizeof(float4) : 0;
-  const size_t ib = images ? n * 3 * sizeof(int) : 0;
-  ReadStage st(e, pb + vb + ib);
-  float4* sp = reinterpret_cast<float4*>(st.p);
-  float4* sv = reinterpret_cast<float4*>(st.p + pb);
-  int* si = reinterpret_cast<int*>(st.p + pb + vb);
-  EngArgs a = make_args(e);
-  const int blocks = (h.n + 255) / 256;
-  k_read_unsort<<<blocks, 256, 0, e->stream>>>(a, id, h.p0, h.n, what, src);
-  k_read_stream<<<std::min(blocks, 4 * std::max(e->nsm, 1)), 256, 0, e->stream>>>(a, id, h.p0, h.n, what, sp, sv, si);
+  const size_t bpp = (pos ? sizeof(float4) : 0) + (vel ? sizeof(float4) : 0) + (images ? 3 * sizeof(int) : 0);
+  const int nthr = n * bpp >= kReadThreads ? 4 : 1;
+  const bool whole = n * bpp <= kReadRegion;
+  // particles of a piece (whole sets of 64, so that every part stays aligned)
+  const size_t piece = whole ? n : kReadRegion / (2 * nthr) / bpp / 64 * 64;
+  const size_t pbytes = (piece * bpp + 15) / 16 * 16;
+  ReadStage st(e, whole ? pbytes : 2 * nthr * pbytes);
+  const EngArgs a = make_args(e);
+  k_read_unsort<<<(h.n + 255) / 256, 256, 0, e->stream>>>(a, id, h.p0, h.n, what, src);
   check_launch();
-  CK(cudaStreamSynchronize(e->stream));
-  if (pos) copy_out(pos, sp, pb);
-  if (vel) copy_out(vel, sv, vb);
-  if (images) copy_out(images, si, ib);
+  auto part = [&](int t, cudaEvent_t* ev) -> cudaError_t {
+    cudaError_t err = cudaSetDevice(e->device);
+    if (err != cudaSuccess) return err;
+    const size_t share = (n + nthr - 1) / nthr, lo = std::min(n, t * share), hi = std::min(n, lo + share);
+    const size_t np = (hi - lo + piece - 1) / piece;
+    for (size_t k = 0; k <= np; ++k) {
+      if (k < np) {
+        const size_t i0 = lo + k * piece, m = std::min(piece, hi - i0);
+        char* b = st.p + (2 * t + (k & 1)) * (whole ? 0 : pbytes);
+        float4* sp = reinterpret_cast<float4*>(b);
+        float4* sv = sp + (pos ? m : 0);
+        int* si = reinterpret_cast<int*>(sv + (vel ? m : 0));
+        const int blocks = (int)std::min<size_t>((m + 255) / 256, 4 * std::max(e->nsm, 1));
+        k_read_stream<<<blocks, 256, 0, e->stream>>>(a, id, h.p0, (int)i0, (int)m, what, sp, sv, si);
+        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+        if ((err = cudaEventRecord(ev[k & 1], e->stream)) != cudaSuccess) return err;
+      }
+      if (k > 0) {
+        const size_t i0 = lo + (k - 1) * piece, m = std::min(piece, hi - i0);
+        if ((err = cudaEventSynchronize(ev[(k - 1) & 1])) != cudaSuccess) return err;
+        const char* b = st.p + (2 * t + ((k - 1) & 1)) * (whole ? 0 : pbytes);
+        if (pos) std::memcpy(static_cast<float4*>(pos) + i0, b, m * sizeof(float4));
+        if (pos) b += m * sizeof(float4);
+        if (vel) std::memcpy(static_cast<float4*>(vel) + i0, b, m * sizeof(float4));
+        if (vel) b += m * sizeof(float4);
+        if (images) std::memcpy(static_cast<int*>(images) + 3 * i0, b, m * 3 * sizeof(int));
+      }
+    }
+    return cudaSuccess;
+  };
+  while (e->read_ev.size() < (size_t)2 * nthr) {
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    e->read_ev.push_back(ev);
+  }
+  std::vector<cudaError_t> err(nthr, cudaSuccess);
+  std::vector<std::thread> th;
+  int started = 1;
+  try {
+    for (; started < nthr; ++started) {
+      const int t = started;
+      th.emplace_back([&, t] { err[t] = part(t, &e->read_ev[2 * t]); });
+    }
+  } catch (const std::system_error&) {  // no thread to be had: the rest here
+  }
+  err[0] = part(0, &e->read_ev[0]);
+  for (int t = started; t < nthr; ++t) err[t] = part(t, &e->read_ev[2 * t]);
+  for (auto& t : th) t.join();
+  for (const cudaError_t x : err) CK(x);
   st.done();
 }
 
@@ -1682,8 +1707,8 @@ int b2md_engine_create(int device, long long max_particles, int max_replicas, lo
     // pinned staging for the expected particles, so that admissions and
     // read-backs do not allocate it later
     if (max_particles > 0) {
-      ring_reserve(e, std::min<size_t>(std::max<size_t>((size_t)max_particles * 128, (size_t)4 << 20),
-                                       (size_t)256 << 20));
+      ring_reserve(e, std::min<size_t>(std::max<size_t>((size_t)max_particles * 64, (size_t)4 << 20),
+                                       (size_t)64 << 20));
     }
     init_func_attrs(device);
     CK(cudaMalloc(&e->fctr, sizeof(unsigned)));
@@ -1720,6 +1745,7 @@ int b2md_engine_destroy(b2md_engine* e) {
                   e->fq, e->fseq};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  for (cudaEvent_t ev : e->read_ev) cudaEventDestroy(ev);
   if (e->h_budget) cudaFreeHost(e->h_budget);
   ring_reset(e);
   if (e->ring) cudaFreeHost(e->ring);

@@ -43,6 +43,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -530,12 +531,20 @@ struct b2md_f64 {
   long long elog_cap = 0;
   std::vector<void*> bufs;
   double4* scratch = nullptr;  // the list build's per-particle scratch: im2, uid2, cell, rank, order
-  void* pinned = nullptr;      // read-backs pass through it (32 bytes per particle)
 };
 
 namespace {
 
 std::string f64_errmsg;
+
+// Page-locked staging of the read-backs, one piece for all engines of the
+// process (page-locking costs milliseconds, which every engine would pay for
+// its first read-back): allocated by the first read-back, freed with the last
+// engine; the lock is held while it is used.
+constexpr size_t kStageBytes = (size_t)1 << 20;
+std::mutex g_stage_mu;
+void* g_stage = nullptr;
+int g_engines = 0;
 
 int f64_fail(int code, const char* fmt, ...) {
   char buf[512];
@@ -632,6 +641,10 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
     rc_max = std::max(rc_max, q.rc);
   }
   b2md_f64* h = new b2md_f64();
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    ++g_engines;
+  }
   h->device = device;
   F64Args& a = h->a;
   a.n = n; a.ntypes = ntypes; a.cutoff = cutoff_method;
@@ -702,9 +715,13 @@ int b2md_f64_destroy(b2md_f64* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->bufs) cudaFree(p);
   if (h->elog) cudaFree(h->elog);
-  if (h->pinned) cudaFreeHost(h->pinned);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
+  std::lock_guard<std::mutex> lock(g_stage_mu);
+  if (--g_engines == 0 && g_stage) {
+    cudaFreeHost(g_stage);
+    g_stage = nullptr;
+  }
   return B2MD_OK;
 }
 
@@ -822,12 +839,16 @@ int b2md_f64_get(b2md_f64* h, int field, void* out) {
   if (field >= B2MD_F64_POS && field <= B2MD_F64_IMAGES) {
     const double4* src = field == B2MD_F64_POS ? h->a.r : field == B2MD_F64_VEL ? h->a.v : field == B2MD_F64_FORCE ? h->a.f : nullptr;
     const size_t bytes = (size_t)n * (src ? sizeof(double4) : 3 * sizeof(int));
-    if (!h->pinned) F64_CK(cudaMallocHost(&h->pinned, (size_t)n * sizeof(double4)));
     k64_unsort<<<nblocks(h), kB, 0, h->stream>>>(h->a, src, h->scratch, reinterpret_cast<int*>(h->scratch));
     F64_CK(cudaGetLastError());
-    F64_CK(cudaMemcpyAsync(h->pinned, h->scratch, bytes, cudaMemcpyDeviceToHost, h->stream));
-    F64_CK(cudaStreamSynchronize(h->stream));
-    std::memcpy(out, h->pinned, bytes);
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    if (!g_stage) F64_CK(cudaHostAlloc(&g_stage, kStageBytes, cudaHostAllocPortable));
+    for (size_t b = 0; b < bytes; b += kStageBytes) {
+      const size_t m = std::min(kStageBytes, bytes - b);
+      F64_CK(cudaMemcpyAsync(g_stage, reinterpret_cast<const char*>(h->scratch) + b, m, cudaMemcpyDeviceToHost, h->stream));
+      F64_CK(cudaStreamSynchronize(h->stream));
+      std::memcpy(static_cast<char*>(out) + b, g_stage, m);
+    }
     return B2MD_OK;
   }
   return f64_fail(B2MD_ERR_ARG, "b2md_f64_get: unknown field %d", field);

@@ -1491,9 +1491,11 @@ __global__ void __launch_bounds__(256) k_read_unsort(EngArgs a, int rep, long lo
   if (what & kReadImages) a.im[ab ^ 1][go] = a.im[ab][gi];
   if (what & kReadField) a.v[ab ^ 1][go] = src[gi];
 }
-__global__ void __launch_bounds__(256) k_read_stream(EngArgs a, int rep, long long p0, int n, unsigned what,
+// (n particles from i0 on)
+__global__ void __launch_bounds__(256) k_read_stream(EngArgs a, int rep, long long p0, int i0, int n, unsigned what,
                                                      float4* pos, float4* vel, int* images) {
   const int rb = a.st[rep].rbuf, ab = a.st[rep].abuf;
+  p0 += i0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (what & kReadPos) pos[i] = a.r[rb ^ 1][p0 + i];
     if (what & (kReadVel | kReadField)) vel[i] = a.v[ab ^ 1][p0 + i];
