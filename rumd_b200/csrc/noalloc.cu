@@ -65,6 +65,7 @@ struct NoAllocScratch {
   double part[kNoAllocMaxBlocks][2];  // per-block sums of u_i and w_i
 };
 constexpr unsigned kBadType = 0x80000000u;
+constexpr unsigned kNoParticle = 0xffffffffu;  // a group's place without a particle
 // One warp lists a cell's particles, so a few crowded cells (a cluster in a
 // box so large that its cells cannot be small) would leave the work to a few
 // warps: then the all-pairs form runs, which spreads evenly.
@@ -269,7 +270,8 @@ __device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned 
     unsigned me = id[0];
 #pragma unroll
     for (int q = 1; q < G; ++q) me = lane / (32 / G) == q ? id[q] : me;
-    if (me & kBadType) {
+    if (me == kNoParticle) {
+    } else if (me & kBadType) {
       const float nanf_ = __int_as_float(0x7fc00000);
       force[me & ~kBadType] = make_float4(nanf_, nanf_, nanf_, nanf_);
     } else {
@@ -280,31 +282,44 @@ __device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned 
   }
 }
 
+// The m <= G particles of a cell from p0 on (a missing one has a NaN position,
+// which is in range of nothing).  The next round's candidates are loaded while
+// the current one's pairs are computed.
 template <int G>
 __device__ __forceinline__ void cell_group(NoAllocScratch* scr, const int4* tab, int off, int len, int total, int p0,
-                                           unsigned wrap, const float* s_tab, int ntypes, const float3& L,
+                                           int m, unsigned wrap, const float* s_tab, int ntypes, const float3& L,
                                            const float3& iL, float4* __restrict__ force, double& u, double& w) {
   const int lane = threadIdx.x & 31;
+  const float nan = __int_as_float(0x7fc00000);
   const float4* __restrict__ sp = scr->pos;
   Sum5 A[G];
   float4 rp[G];
   unsigned id[G];
 #pragma unroll
   for (int q = 0; q < G; ++q) {
-    rp[q] = sp[p0 + q];
-    id[q] = scr->id[p0 + q];
+    rp[q] = q < m ? sp[p0 + q] : make_float4(nan, nan, nan, 0.f);
+    id[q] = q < m ? scr->id[p0 + q] : kNoParticle;
   }
-  int rows = 0;  // non-empty rows that start before this round
-#pragma unroll 1
-  for (int ch = 0; ch < total; ch += 32) {
+  int rows = 0;  // non-empty rows that start before the round
+  auto candidate = [&](int ch) -> int {
     const int v = ch + lane;
     const unsigned rel = (unsigned)(off - ch);
     const unsigned st = __reduce_or_sync(0xffffffffu, len > 0 && rel < 32u ? 1u << rel : 0u);
     const int4 t = tab[rows + __popc(st & ((2u << lane) - 1u)) - 1];
     rows += __popc(st);
-    const int j = v < total ? v + (v < t.z ? t.y : t.w) : p0;
-    float4 rj = sp[j];
-    if (v >= total) rj.x = __int_as_float(0x7fc00000);
+    return v < total ? v + (v < t.z ? t.y : t.w) : p0;
+  };
+  int jn = candidate(0);
+  float4 rn = sp[jn];
+#pragma unroll 1
+  for (int ch = 0; ch < total; ch += 32) {
+    const int j = jn;
+    float4 rj = rn;
+    if (ch + 32 < total) {
+      jn = candidate(ch + 32);
+      rn = sp[jn];
+    }
+    if (ch + lane >= total) rj.x = nan;
     add_candidate<G>(A, rp, p0, j, rj, wrap, s_tab, ntypes, L, iL);
   }
   store_forces<G>(A, id, force, u, w);
@@ -344,13 +359,14 @@ __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, 
 // per lane: of a cell's particles against its 5x5x5 neighbourhood (CELLS), or
 // of G consecutive particles against all.  Units go to warps in a fixed order.
 // What bounds the cell form is the pair arithmetic: about 300 candidates per
-// particle at KA density, of which a quarter is in range.  Held to 80
-// registers for six blocks per SM (137 us with 109 registers, 119 with 80, the
-// same with 64 and spills; KA N=65521).  Calls back to back, all pairs by one
-// thread per particle before: N=65521 7275 -> 119 us, N=16384 1388 -> 52,
-// N=4000 369 -> 37, N=1000 109 -> 17 (the last three mostly launches).
+// particle at KA density, of which a quarter is in range, and the chain to the
+// candidates' positions.  Held to 72 registers for seven blocks per SM (KA
+// N=65521: 109 us a call with 96 registers, 112 with 80, 106 with 72).  Calls
+// back to back, all pairs by one thread per particle before: N=65521 7275 ->
+// 106 us, N=16384 1388 -> 49, N=4000 369 -> 37, N=1000 109 -> 17 (the last
+// three mostly launches).
 template <int G, bool CELLS>
-__global__ void __launch_bounds__(kNoAllocBlock, 6)
+__global__ void __launch_bounds__(kNoAllocBlock, 7)
     k_forces_noalloc(const float4* __restrict__ pos, int n, float3 L, float3 iL, Grid3 g, int ntypes, PairTable tab,
                      float4* __restrict__ force, double* __restrict__ sums, NoAllocScratch* scr) {
   __shared__ __align__(16) float s_tab[kNoAllocMaxTypes * kNoAllocMaxTypes * kRow];
@@ -404,16 +420,10 @@ __global__ void __launch_bounds__(kNoAllocBlock, 6)
       if (len > 0) rowtab[__popc(ne & ((1u << lane) - 1u))] = make_int4(off, b0 - off, off + l0, b1 - off - l0);
       __syncwarp();
       for (int p = p0; p < p1; p += 4) {
-        const int m = p1 - p;
-#define CG(K) cell_group<K>(scr, rowtab, off, len, total, p, wrap, s_tab, ntypes, L, iL, force, u, w)
-        if (m >= 3) {
-          if (m >= 4) CG(4);
-          else {
-            CG(2);
-            cell_group<1>(scr, rowtab, off, len, total, p + 2, wrap, s_tab, ntypes, L, iL, force, u, w);
-          }
-        } else if (m == 2) CG(2);
-        else CG(1);
+        const int m = min(4, p1 - p);
+#define CG(K) cell_group<K>(scr, rowtab, off, len, total, p, m, wrap, s_tab, ntypes, L, iL, force, u, w)
+        if (m > 2) CG(4);
+        else CG(2);
 #undef CG
       }
     }
