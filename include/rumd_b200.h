@@ -167,9 +167,9 @@ B2MD_API int b2md_engine_set_graph_mode(b2md_engine* e, int conditional);
  *                                memory (one TMA bulk copy per segment), with
  *                                a 16-bit list of window offsets.
  *   B2MD_VARIANT_BUILD_LANES   the list build: 0 (default) one warp per
- *                              cell, each lane testing a contiguous run of
- *                              the cell's candidates against up to four of
- *                              its particles at once; 1,2,4,8 lanes per
+ *                              cell, testing 32 of the cell's candidates a
+ *                              round, one per lane, against up to four of
+ *                              its particles; 1,2,4,8 lanes per
  *                              particle; 32: one warp per cell, 32
  *                              candidates per round staged in shared memory
  *                              (with force mode 2 the lane build runs for 0

@@ -6,8 +6,9 @@
 //     (SimulationBox.h:111-125, NeighborList.cu:1106-1140, 1282-1285) with the
 //     multiply-add contractions that nvcc applies to it written out as
 //     __fmaf_rn, so list sets and the sort permutation are bit-exact.
-//   * Pair forces are FP32 (PairPotential.h:161-168, 1198-1244); 1/r^2 and 1/r
-//     are the hardware reciprocal and reciprocal square root.
+//   * Pair forces are FP32 (PairPotential.h:161-168, 1198-1244); 1/r is the
+//     hardware reciprocal square root refined by one Newton-Raphson step and
+//     1/r^2 its square.
 //   * Reductions (pe, virial, kinetic energy, momentum) are FP64 with a fixed
 //     summation tree, so results do not depend on scheduling or on which other
 //     replicas share the launch; the thermostat state is FP64.
@@ -470,13 +471,13 @@ struct RowsLJ {
 //   POT_LJ_12_6_SMOOTH_2_4 Pot_LJ_12_6_smooth_2_4::ComputeInteraction
 //                          (PairPotential.h:248-255)
 //   POT_IPL_N              Pot_IPL_n::ComputeInteraction (PairPotential.h:630-636)
-// 1/r^2 is the hardware reciprocal of d^2 (one unit in the last place); 1/r,
-// which only the small shifted-force term uses, the hardware reciprocal
-// square root.  (1/r^2 as the square of a Newton-refined rsqrt took five
-// operations more per pair and was no closer: forces are 2.2e-6 rms-rel from
-// the FP64 sums either way, KA N=32000.)  The cut-off method is folded into
+// 1/r comes from one MUFU rsqrt refined by one Newton-Raphson step
+// (y <- y (3/2 - x y^2 / 2)); 1/r^2 = y^2.  The cut-off method is folded into
 // the packed pair row: s -= c_s / r and u += c_s r + c_u0, which is
 // s(rc) rc / r and s(rc) rc (r - rc) - u(rc) for SF, -u(rc) for SP, 0 for NS.
+// (1/r^2 as a hardware reciprocal takes five operations less, 23.4 instead of
+// 24.1 us per k_steps step at KA N=65536, and is as close to the FP64 sums, but
+// its other roundings move every trajectory.)
 // wrap: the dimensions (x 1, y 2, z 4) in which the minimum-image step is not
 // exactly the identity for every particle of the warp (see k_force); the same
 // for the whole warp.  ok = false: the entry is not one of the lane's.
@@ -511,7 +512,9 @@ template <bool STRESS, int POT, class Rows>
 __device__ __forceinline__ void pair_add(PairAcc& A, bool ok, const PairDisp& d, int tj, const Rows& rows) {
   const float dx = d.dx, dy = d.dy, dz = d.dz;
   const float d2 = dist2_ref(dx, dy, dz);
-  const float i2 = rcp_approx(d2), y = rsqrt_approx(d2);
+  float y = rsqrt_approx(d2);
+  y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
+  const float i2 = y * y;
   float s, u;
   bool in;
   if constexpr (POT == POT_LJ_12_6) {
@@ -520,9 +523,8 @@ __device__ __forceinline__ void pair_add(PairAcc& A, bool ok, const PairDisp& d,
     rows.lj(tj, q, p);
     const float i6 = i2 * i2 * i2;
     const float t = q.y * i6;
-    const float w = q.w * y;
-    s = __fmaf_rn(i6 * i2, __fmaf_rn(12.f, t, p.y), -w);
-    u = __fmaf_rn(w, d2, __fmaf_rn(i6, t + q.z, p.x));
+    s = __fmaf_rn(-q.w, y, i6 * i2 * __fmaf_rn(12.f, t, p.y));
+    u = __fmaf_rn(i6, t + q.z, __fmaf_rn(q.w, d2 * y, p.x));
     in = d2 < q.x;
   } else if constexpr (POT == POT_LJ_12_6_SMOOTH_2_4) {
     const float* pp = rows.row(tj);

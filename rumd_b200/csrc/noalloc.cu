@@ -238,7 +238,9 @@ __device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G
     const float4 c = *reinterpret_cast<const float4*>(row);  // rc^2, A12, A6, c_s
     const bool in = d2 < c.x && j != p0 + q;
     if (!__any_sync(0xffffffffu, in)) continue;
-    // the engine's pair function (pair_add of the step kernels)
+    // the engine's pair function (pair_add of the step kernels), with 1/r^2 the
+    // hardware reciprocal of d^2 (one unit in the last place) and 1/r, which
+    // only the small shifted-force term uses, the reciprocal square root
     const float2 e = *reinterpret_cast<const float2*>(row + 4);  // c_u0, 6 A6
     const float i2 = b2md::rcp_approx(d2), y = b2md::rsqrt_approx(d2);
     const float i6 = i2 * i2 * i2, t = c.y * i6, w = c.w * y;
