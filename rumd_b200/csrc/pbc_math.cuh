@@ -30,8 +30,9 @@ __device__ __forceinline__ float dist2_ref(float dx, float dy, float dz) {
 }
 
 // Hardware approximate 1/x and 1/sqrt(x) (one MUFU operation each, denormals
-// flushed; relative errors at most 2^-23 and 2^-22.9).  Arguments here are
-// squared distances, far from the denormal range.
+// flushed; relative errors at most 2^-23 and 2^-22.9); the step kernels refine
+// 1/sqrt(x) with a Newton-Raphson step.  Arguments here are squared distances,
+// far from the denormal range.
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -77,7 +78,9 @@ __device__ __forceinline__ int cell_coord(float x, float invL, int nc) {
   // calculateCellCoordinates (NeighborList.cu:1106-1133)
   float scaled = __fmaf_rn(x, invL, 0.5f);
   int c = __float2int_rz(__fmul_rn((float)nc, scaled));
-  if (c == nc) c -= 1;
+  // (the reference tests c == nc; a coordinate that is far outside the box, as
+  // in a system that has blown up, must not leave the cell arrays either)
+  if (c >= nc) c = nc - 1;
   else if (c < 0) c = 0;
   return c;
 }

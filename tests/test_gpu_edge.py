@@ -113,3 +113,36 @@ def test_rumd_launch_shapes_are_mapped(capi, oracle, req, eff):
     e.close()
     ref, _, _ = oracle.forces_f64(c["pos4"][:, :3].astype(np.float64), c["types"], c["box"], 2, params, 2)
     assert rms_rel(f[:, :3].astype(np.float64), ref) < 1e-5
+
+
+def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi):
+    """Coordinates far outside the box, infinite or not a number (a system that
+    has blown up) go to some cell of the grid: the evaluation returns, and the
+    particles out of their reach keep their forces."""
+    from rumd_b200 import initconf as I
+    n = 4000
+    c = I.ka_config(n, T=0.8, seed=3)
+    p = np.ascontiguousarray(I.lj_params(2, I.KA), np.float32)
+    e = capi.Engine(device=0, pb=64, tp=2)
+    rid = e.add(c["pos4"], c["box"], p, 2, vel4=c["vel4"])
+    e.calc_f()
+    f0 = e.get(rid, "force", n)
+    bad = c["pos4"].copy()
+    bad[:4, 0] = [np.inf, -np.inf, np.nan, 3e30]
+    bad[4, 1], bad[5, 2] = -3e30, 5e9
+    e.set(rid, "pos", bad)
+    e.calc_f()
+    f1 = e.get(rid, "force", n)
+    L = c["box"]
+    d = c["pos4"][None, :6, :3] - c["pos4"][:, None, :3]
+    d -= L * np.rint(d / L)
+    far = ((d * d).sum(-1) > 2.5 ** 2).all(1)
+    far[:6] = False
+    same = np.isclose(f0[far], f1[far], rtol=1e-4, atol=1e-3).all(1)
+    # (the displaced particles land in some cell and may act on those near it)
+    assert same.mean() > 0.8
+    e.set(rid, "pos", c["pos4"])
+    e.calc_f()
+    assert np.array_equal(e.get(rid, "pos", n), c["pos4"])
+    assert np.allclose(e.get(rid, "force", n), f0, rtol=1e-4, atol=1e-3)
+    e.close()
