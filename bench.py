@@ -271,10 +271,10 @@ def time_run(capi, e, steps, device):
     return t0.elapsed_time(t1) / 1e3
 
 
-def launches_in_run(steps, rebuilds, per_rebuild=8, persistent=False):
+def launches_in_run(steps, rebuilds, per_rebuild=2, persistent=False):
     # run start: steps + momentum; run end: rebuild sequence + force kernel.
     # Per-step graphs: a fused kernel per step, a gate per graph launch and
-    # the rebuild kernels (8, 9 with position windows) per rebuild.
+    # the rebuild kernels (sort and list build, and position windows) per rebuild.
     # Persistent graph: one loop gate, then per loop pass (a pass ends at each
     # rebuild) the rebuild kernels, which exit at once when none is due, and
     # one k_steps launch.
@@ -747,7 +747,7 @@ def main():
     extra = {}
     cfg = config_block(args, world)
     variants = kernel_variants(e)
-    per_rebuild = 9 if variants.get("force_mode") == capi.FORCE_WINDOW else 8
+    per_rebuild = 3 if variants.get("force_mode") == capi.FORCE_WINDOW else 2
     if rank == 0:
         pos4, vel4, im3 = e.read(rid, N_PLAIN)
         e2e = e2e_run(capi, device, args.pb, args.tp, pos4, vel4, im3, box, params, args.steps)
