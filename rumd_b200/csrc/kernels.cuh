@@ -2539,7 +2539,7 @@ __device__ __forceinline__ int build_cell(const RepDev& R, const float4* rc, con
     rp[q] = COH ? ld_ca_f4(rc + pg + q) : __ldg(rc + pg + q);
     cnt[q] = 0u;
   }
-  int rows = 0;  // non-empty rows that start before this round
+  int rows = 0;  // non-empty rows that start before the current 32 candidates
   // the round's candidate (slot; one past the last repeats the cell's first
   // particle): the next round's is loaded while the current one is tested
   // (the chain row mask - table - position bounds a round; a rebuild at KA
