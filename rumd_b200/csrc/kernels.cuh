@@ -87,6 +87,10 @@ __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
 // calls it with its block totals in s_blk; returns true in exactly one block
 // (the last to finish) with the replica totals in s_tot.  A replica of one
 // group needs the first level only.
+// A group's last block resets the group's counter before its arrival at the
+// replica's, whose release then orders the reset before the replica's next
+// step: in k_flow nothing else does (another group's block may finish this
+// step and queue the next one's tiles while this block is still here).
 __device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int lt, const double* s_blk, double* s_tot) {
   __shared__ int s_last;
   const int g = lt / kGroup;
@@ -97,6 +101,7 @@ __device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int l
   if (threadIdx.x == 0) {
     unsigned c = atom_add_acq_rel(&a.gctr[R.group0 + g], 1u);
     s_last = (c == (unsigned)(gsize - 1));
+    if (s_last) a.gctr[R.group0 + g] = 0u;
   }
   __syncthreads();
   if (!s_last) return false;
@@ -107,12 +112,9 @@ __device__ bool replica_reduce(const EngArgs& a, int rep, const RepDev& R, int l
     __syncthreads();
     if (threadIdx.x == 0) s_last = atom_add_acq_rel(&a.rctr[rep], 1u) == (unsigned)(R.ngroups - 1);
     __syncthreads();
-    if (threadIdx.x == 0) a.gctr[R.group0 + g] = 0u;
     if (!s_last) return false;
     if (threadIdx.x == 0) a.rctr[rep] = 0u;
     if (threadIdx.x < 32) x = warp_rows_sum(a.gpart + (size_t)R.group0 * kNPart, R.ngroups);
-  } else if (threadIdx.x == 0) {
-    a.gctr[R.group0 + g] = 0u;
   }
   if (threadIdx.x < kNPart) s_tot[threadIdx.x] = x;
   __syncthreads();
