@@ -373,7 +373,9 @@ __global__ void __launch_bounds__(kB) k64_forces(F64Args a) {
   const double4 ri = a.r[valid ? i : 0];
   const F64Pair* row = a.par + type_of(ri) * a.ntypes;
   // a particle farther than rc_max + 2 skin from both faces of a dimension has
-  // its listed neighbours at their minimum image in it
+  // its listed neighbours at their minimum image in it, when these are inside
+  // the box (ilim < 0 until a state given with other coordinates has been
+  // wrapped by a step)
   const bool wx = __any_sync(FULL, !(fabs(ri.x) < a.ilim[0])), wy = __any_sync(FULL, !(fabs(ri.y) < a.ilim[1])),
              wz = __any_sync(FULL, !(fabs(ri.z) < a.ilim[2]));
   double fx = 0.0, fy = 0.0, fz = 0.0, u = 0.0, w = 0.0;
@@ -525,6 +527,9 @@ struct b2md_f64 {
   F64Pair* par = nullptr;
   int reset_interval = 100;
   bool have_state = false;
+  double ilim[3];       // k64_forces' limits for coordinates inside the box
+  double inside[3];     // largest |coordinate| that counts as inside: half a box and half a skin, by which a
+                        // listed neighbour still is at its minimum image (see k64_forces)
   int tp = 4;           // lanes per particle of the force kernel
   int rb_grid = 1;      // blocks of the list build, all resident at once
   double* elog = nullptr;  // energies of a run, kept for the next
@@ -656,7 +661,8 @@ int b2md_f64_create(int device, int n, int ntypes, const double* box3, const flo
     a.nc[d] = (int)std::floor(box3[d] / (rc_max + skin));
     if (a.nc[d] < 3) a.allpairs = 1;
     a.ncell *= std::max(a.nc[d], 1);
-    a.ilim[d] = 0.5 * box3[d] - (rc_max + 2.0 * skin) - 1e-9 * box3[d];
+    h->ilim[d] = a.ilim[d] = 0.5 * box3[d] - (rc_max + 2.0 * skin) - 1e-9 * box3[d];
+    h->inside[d] = 0.5 * (box3[d] + skin);
   }
   // lanes per particle: about as many threads as the GPU holds
   h->tp = n < 8192 ? 32 : n < 65536 ? 8 : 4;
@@ -730,6 +736,7 @@ int b2md_f64_set_state(b2md_f64* h, const double* pos4, const double* vel4, cons
   const int n = h->a.n;
   std::vector<double4> r(n), v(n);
   std::vector<int4> im(n);
+  bool inside = true;
   for (int i = 0; i < n; ++i) {
     const double t = pos4[4 * i + 3];
     if (!(t >= 0.0 && t < h->a.ntypes && t == std::floor(t)))
@@ -739,6 +746,8 @@ int b2md_f64_set_state(b2md_f64* h, const double* pos4, const double* vel4, cons
     r[i] = make_double4(pos4[4 * i], pos4[4 * i + 1], pos4[4 * i + 2], t);
     v[i] = make_double4(vel4[4 * i], vel4[4 * i + 1], vel4[4 * i + 2], vel4[4 * i + 3]);
     im[i] = im3 ? make_int4(im3[3 * i], im3[3 * i + 1], im3[3 * i + 2], 0) : make_int4(0, 0, 0, 0);
+    inside = inside && std::fabs(r[i].x) <= h->inside[0] && std::fabs(r[i].y) <= h->inside[1] &&
+             std::fabs(r[i].z) <= h->inside[2];
   }
   F64_CK(cudaSetDevice(h->device));
   F64_CK(cudaMemcpyAsync(h->a.r, r.data(), n * sizeof(double4), cudaMemcpyHostToDevice, h->stream));
@@ -749,6 +758,7 @@ int b2md_f64_set_state(b2md_f64* h, const double* pos4, const double* vel4, cons
   const int one = 1;
   F64_CK(cudaMemcpyAsync(&h->st->need, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaStreamSynchronize(h->stream));
+  for (int d = 0; d < 3; ++d) h->a.ilim[d] = inside ? h->ilim[d] : -1.0;
   h->have_state = true;
   return B2MD_OK;
 }
@@ -815,6 +825,7 @@ int b2md_f64_run(b2md_f64* h, long long nsteps, double* energies) {
     rc = launch_forces(h);
     if (rc) break;
     k64_integrate<<<B, kB, 0, h->stream>>>(h->a, d_log ? d_log + 4 * k : nullptr);
+    for (int d = 0; d < 3; ++d) h->a.ilim[d] = h->ilim[d];  // the step wraps what a state gave unwrapped
     if (cudaGetLastError() != cudaSuccess) rc = f64_fail(B2MD_ERR_CUDA, "b2md_f64_run: launch failed");
     if (rc == B2MD_OK && (k + 1) % 256 == 0) rc = check_overflow(h);
   }

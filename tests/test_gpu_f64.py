@@ -5,6 +5,8 @@ N = 1,048,576 at density 0.8442 (the HBM-scale plain configuration)."""
 import numpy as np
 import pytest
 
+from conftest import shifted_configuration
+
 pytestmark = pytest.mark.gpu
 
 
@@ -67,6 +69,31 @@ def test_f64_trajectory_matches_fp64_oracle(capi, oracle, thermostat):
     # the oracle hands positions back rounded to float32
     assert np.abs(pos[:, :3] - ref["pos4"][:, :3].astype(np.float64)).max() < 1e-5
     assert np.array_equal(im, ref["im3"])
+
+
+@pytest.mark.parametrize("n,box", [(500, (7.5, 7.5, 7.5)), (3000, (18.0, 19.5, 7.25)), (3001, (20.0, 7.0, 18.0))])
+def test_f64_coordinates_outside_the_box(capi, oracle, n, box):
+    """All-pairs lists (a side of fewer than three cells) take any image of a
+    coordinate: the forces, energies and the next steps are those of the
+    wrapped configuration, bit for bit (the separations are exact)."""
+    params = oracle.lj_params(2, oracle.ka_table())
+    box, types, pos4, out, k = shifted_configuration(n, box, seed=n)
+    f_ref, u_ref, _ = oracle.forces_f64(pos4[:, :3].astype(np.float64), types, box, 2, params, 2)
+    got = []
+    for p in (pos4, out):
+        e = capi.F64Engine(p, box, params, 2, cutoff="SF", dt=1e-4, T=0.8)
+        e.calc_f()
+        f, pe = e.get("force"), e.stats()["pe"]
+        en = e.run(3, energies=True)
+        got.append((f, pe, en, e.get("pos"), e.get("images")))
+        e.close()
+    a, b = got
+    assert np.sqrt(np.sum((a[0][:, :3] - f_ref) ** 2) / np.sum(f_ref ** 2)) < 1e-12
+    assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+    # the wrap itself rounds once more for a coordinate that starts outside
+    assert np.abs(a[2] - b[2]).max() <= 1e-9 * np.abs(a[2]).max()
+    assert np.abs(a[3] - b[3]).max() < 1e-9
+    assert np.array_equal(b[4] - a[4], k)
 
 
 def test_f64_rejects_bad_input(capi, oracle):
