@@ -121,6 +121,9 @@ struct HostRep {
   int potential1 = -1, cutoff1 = 0;
   long long par1 = -1;
   int npar1 = 0;
+  // positions were given outside the box and no run has wrapped them since:
+  // the force kernels take every pair's minimum image (derive_limits)
+  bool outside = false;
 };
 
 template <class T>
@@ -633,10 +636,18 @@ void relayout(b2md_engine* e) {
   ensure_layout(e);
 }
 
+void derive_limits(HostRep& h);
 void upload_rep(b2md_engine* e, int id) {
   const HostRep& h = e->reps[id];
   CK(cudaMemcpyAsync(e->rep + id, &h.d, sizeof(RepDev), cudaMemcpyHostToDevice, e->stream));
   CK(cudaStreamSynchronize(e->stream));
+}
+
+// Whether the minimum image may be skipped where k_force's limits allow it.
+void set_outside(b2md_engine* e, int id, bool outside) {
+  e->reps[id].outside = outside;
+  derive_limits(e->reps[id]);
+  upload_rep(e, id);
 }
 
 HostRep& get_rep(b2md_engine* e, int id) {
@@ -713,6 +724,33 @@ void set_potential(HostRep& h, int ntypes, const float* params, int cutoff, floa
   derive_grid(h);
 }
 
+// Limits below which k_force skips the minimum image (RepDev::ilim): they
+// hold for neighbours whose coordinates are inside the box.
+void derive_limits(HostRep& h) {
+  for (int d = 0; d < 3; ++d)
+    h.d.ilim[d] = h.outside ? -1.f : 0.5f * h.d.L[d] - (h.rcmax + 2.f * h.skin) - 0.01f;
+}
+
+// Positions given for replica h: types in range; returns whether a coordinate
+// lies outside the box.  Half a skin beyond it still counts as inside: a
+// neighbour listed from there is at its minimum image all the same (it is
+// within rc + skin, and a particle inside the limits of k_force is
+// rc + 2 skin + 0.01 from the faces).
+bool check_positions(const HostRep& h, const float* pos4) {
+  const float lx = 0.5f * (h.d.L[0] + h.skin) + 0.004f, ly = 0.5f * (h.d.L[1] + h.skin) + 0.004f,
+              lz = 0.5f * (h.d.L[2] + h.skin) + 0.004f;
+  int bad = 0, out = 0;
+  for (int k = 0; k < h.n; ++k) {
+    const float* p = pos4 + 4 * (size_t)k;
+    unsigned t;
+    std::memcpy(&t, p + 3, 4);
+    bad |= t >= (unsigned)h.d.ntypes;
+    out |= !(std::fabs(p[0]) <= lx) | !(std::fabs(p[1]) <= ly) | !(std::fabs(p[2]) <= lz);
+  }
+  if (bad) api_fail(B2MD_ERR_ARG, "particle type out of range");
+  return out != 0;
+}
+
 void derive_grid(HostRep& h) {
   const int ntypes = h.d.ntypes;
   const float skin = h.skin;
@@ -720,7 +758,7 @@ void derive_grid(HostRep& h) {
   for (int k = 0; k < ntypes * ntypes; ++k) h.rcmax = std::max(h.rcmax, h.params[k * kNumParam]);
   for (size_t k = 0; k < h.params1.size() / kNumParam; ++k) h.rcmax = std::max(h.rcmax, h.params1[k * kNumParam]);
   h.d.skin2_4 = (float)(0.25 * skin * skin);
-  for (int d = 0; d < 3; ++d) h.d.ilim[d] = 0.5f * h.d.L[d] - (h.rcmax + 2.f * skin) - 0.01f;
+  derive_limits(h);
   int ncheck[3];
   for (int d = 0; d < 3; ++d) {
     float q = 2 * h.d.L[d] / (h.rcmax + skin);
@@ -1886,11 +1924,8 @@ int b2md_replica_add(b2md_engine* e, const b2md_replica_desc* d, const float* po
     CK(cudaSetDevice(e->device));
     HostRep h = describe(d);
     // types must be in range, inverse masses positive
-    for (int i = 0; i < d->n; ++i) {
-      int t;
-      std::memcpy(&t, &pos4[4 * i + 3], 4);
-      if (t < 0 || t >= d->ntypes) api_fail(B2MD_ERR_ARG, "particle type out of range");
-    }
+    h.outside = check_positions(h, pos4);
+    derive_limits(h);
     if (vel4)
       for (int i = 0; i < h.n; ++i)
         if (!(vel4[4 * i + 3] > 0.f)) api_fail(B2MD_ERR_ARG, "inverse mass (vel4[.,3]) must be positive");
@@ -2073,14 +2108,11 @@ int b2md_replica_set(b2md_engine* e, int id, int field, const void* in) {
       for (int k = 0; k < h.n; ++k) stage[k] = make_int4(im[3 * k], im[3 * k + 1], im[3 * k + 2], 0);
       write_field4(e, id, h, kReadImages, reinterpret_cast<const float4*>(stage));
     } else if (field == B2MD_FIELD_POS) {
-      for (int k = 0; k < h.n; ++k) {
-        int t;
-        std::memcpy(&t, &src[k].w, 4);
-        if (t < 0 || t >= h.d.ntypes) api_fail(B2MD_ERR_ARG, "particle type out of range");
-      }
+      const bool outside = check_positions(h, static_cast<const float*>(in));
       float4* stage = reinterpret_cast<float4*>(stage_alloc(e, nb));
       std::memcpy(stage, src, nb);
       write_field4(e, id, h, kReadPos, stage);
+      if (outside != h.outside) set_outside(e, id, outside);
     } else if (field == B2MD_FIELD_VEL) {
       for (int k = 0; k < h.n; ++k)
         if (!(src[k].w > 0.f)) api_fail(B2MD_ERR_ARG, "inverse mass must be positive");
@@ -2352,6 +2384,10 @@ int b2md_run(b2md_engine* e, long long nsteps) {
     // every queue holds exactly nsteps; run until all are empty (a replica
     // frozen by a list overflow catches up after its repair)
     if (nsteps > 0) run_steps(e, 1LL << 62, nsteps);
+    // every replica has stepped, which wraps its positions
+    if (nsteps > 0)
+      for (size_t r = 0; r < e->reps.size(); ++r)
+        if (e->reps[r].active && e->reps[r].outside) set_outside(e, (int)r, false);
     calc_f(e, false);
     CK(cudaStreamSynchronize(e->stream));
   });

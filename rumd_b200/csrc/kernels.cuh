@@ -955,7 +955,8 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
     // A particle farther than rc_max + 2 skin from both faces of a dimension
     // has all its listed neighbours (within rc + skin at the build, each moved
     // at most skin/2 since) at their minimum image in it, so the correction is
-    // exactly zero there; warps made only of such particles skip it.  Decided
+    // exactly zero there; warps made only of such particles skip it.  (The
+    // limits are negative while positions given outside the box are in use.)  Decided
     // per dimension: a warp's particles are a run of cells along x, so at KA
     // N=65536 about half of the warps need some dimension and few need all.
     const unsigned wrap = (__any_sync(0xffffffffu, valid && !(fabsf(ri.x) < R.ilim[0])) ? 1u : 0u) |

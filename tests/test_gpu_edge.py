@@ -3,6 +3,8 @@ boundary, tiles that are mostly empty, and rejected inputs."""
 import numpy as np
 import pytest
 
+from conftest import shifted_configuration
+
 pytestmark = pytest.mark.gpu
 
 
@@ -113,6 +115,37 @@ def test_rumd_launch_shapes_are_mapped(capi, oracle, req, eff):
     e.close()
     ref, _, _ = oracle.forces_f64(c["pos4"][:, :3].astype(np.float64), c["types"], c["box"], 2, params, 2)
     assert rms_rel(f[:, :3].astype(np.float64), ref) < 1e-5
+
+
+@pytest.mark.parametrize("n,box,set_later", [(370, (6.75, 6.75, 6.75), False), (4500, (24.0, 6.75, 23.5), True),
+                                             (4500, (6.75, 24.0, 23.5), False)])
+def test_coordinates_outside_the_box(capi, n, box, set_later):
+    """All-pairs lists (here a side of fewer than five half cut-offs) take any
+    image of a coordinate: the forces of the wrapped configuration bit for bit
+    (the separations are exact), when a replica is added and when its positions
+    are set, and the same images after a run."""
+    from rumd_b200 import initconf as I
+    params = np.ascontiguousarray(I.lj_params(2, I.KA), np.float32)
+    box, types, pos4, out, k = shifted_configuration(n, box, seed=n)
+    got = []
+    for p in (pos4, out):
+        e = capi.Engine(device=0, pb=64, tp=4)
+        rid = e.add(pos4 if set_later else p, box, params, 2, cutoff="SF", dt=1e-4, T=0.8)
+        if set_later:
+            e.calc_f()
+            e.set(rid, "pos", p)
+        e.calc_f()
+        f, st = e.get(rid, "force", n), e.stats(rid)
+        assert np.array_equal(e.get(rid, "pos", n), p)
+        e.run(2)
+        got.append((f, st["pe"], st["virial"], e.get(rid, "pos", n), e.get(rid, "images", n), e.get(rid, "force", n)))
+        e.close()
+    a, b = got
+    assert np.array_equal(a[0], b[0]) and a[1] == b[1] and a[2] == b[2]
+    # a coordinate that starts outside is rounded at its larger magnitude once
+    # (up to 2.5 boxes: 2^-19), which the stiffest pairs' forces multiply
+    assert np.abs(a[3] - b[3])[:, :3].max() < 1e-5
+    assert np.array_equal(b[4] - a[4], k)
 
 
 def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi):
