@@ -433,6 +433,7 @@ B2MD_API int b2md_forces_noalloc(const float* pos4, int n, const float* box, int
  *   be NULL.  max_nbrs 0 = 1.6 x the ideal-gas estimate + 32.
  *   b2md_f64_run: energies (NULL or nsteps*4 doubles) = pe, W, KE(t), xi per
  *   step, as Simulation.Run's energies file rows.
+ *   b2md_f64_calc_f, _run and _get: B2MD_ERR_STATE before a state is set.
  *   b2md_f64_stats: out[7] = pe, W, KE(t), KE2, xi, rebuilds, steps. */
 typedef struct b2md_f64 b2md_f64;
 #define B2MD_F64_POS 0    /* double4 per particle */

@@ -848,6 +848,8 @@ int b2md_f64_get(b2md_f64* h, int field, void* out) {
   const int n = h->a.n;
   F64_CK(cudaSetDevice(h->device));
   if (field >= B2MD_F64_POS && field <= B2MD_F64_IMAGES) {
+    // (the order of the caller's particles comes with the state)
+    if (!h->have_state) return f64_fail(B2MD_ERR_STATE, "b2md_f64_get: no state set");
     const double4* src = field == B2MD_F64_POS ? h->a.r : field == B2MD_F64_VEL ? h->a.v : field == B2MD_F64_FORCE ? h->a.f : nullptr;
     const size_t bytes = (size_t)n * (src ? sizeof(double4) : 3 * sizeof(int));
     k64_unsort<<<nblocks(h), kB, 0, h->stream>>>(h->a, src, h->scratch, reinterpret_cast<int*>(h->scratch));

@@ -2,12 +2,16 @@
 built by changeToDouble.sh) against the FP64 oracle, and the FP32 engine
 against it: the accuracy statements for the single-component LJ system of
 N = 1,048,576 at density 0.8442 (the HBM-scale plain configuration)."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from conftest import shifted_configuration
 
 pytestmark = pytest.mark.gpu
+
+B2MD_ERR_STATE = 4
 
 
 @pytest.fixture(scope="module")
@@ -102,6 +106,30 @@ def test_f64_rejects_bad_input(capi, oracle):
     pos4[:, 3] = 3.0  # type 3 of a 1-type system
     with pytest.raises(ValueError):
         capi.F64Engine(pos4, [5.0, 5.0, 5.0], params, 1)
+
+
+def test_f64_needs_a_state(capi, oracle):
+    """calc_f, run and get of an engine without a state return an error and
+    leave the caller's array alone."""
+    lib, n = capi.lib(), 1000
+    params = np.ascontiguousarray(oracle.lj_params(1, oracle.lj_table()), np.float32)
+    box = np.full(3, 10.6)
+    h = ctypes.c_void_p()
+    capi.check(lib.b2md_f64_create(0, n, 1, capi._ptr(box), capi._ptr(params), capi.CUTOFF["SF"], 0.3, 0,
+                                   ctypes.byref(h)))
+    out = np.full((n, 4), 7.0)
+    for field in range(4):
+        assert lib.b2md_f64_get(h, field, capi._ptr(out)) == B2MD_ERR_STATE
+    assert lib.b2md_f64_calc_f(h) == B2MD_ERR_STATE
+    assert lib.b2md_f64_run(h, 1, None) == B2MD_ERR_STATE
+    assert (out == 7.0).all()
+    pos4 = np.zeros((n, 4))
+    pos4[:, :3] = (np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) * 1.06 - 5.3
+    vel4 = np.ones((n, 4))
+    capi.check(lib.b2md_f64_set_state(h, capi._ptr(pos4), capi._ptr(vel4), None))
+    capi.check(lib.b2md_f64_get(h, 0, capi._ptr(out)))
+    assert np.array_equal(out, pos4)
+    lib.b2md_f64_destroy(h)
 
 
 def lj_state(capi, oracle, n, T, steps):
