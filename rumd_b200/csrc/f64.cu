@@ -750,6 +750,12 @@ int b2md_f64_set_state(b2md_f64* h, const double* pos4, const double* vel4, cons
              std::fabs(r[i].z) <= h->inside[2];
   }
   F64_CK(cudaSetDevice(h->device));
+  if (h->have_state) {
+    // the last forces stay readable: into the caller's order, as the new state is
+    k64_unsort<<<nblocks(h), kB, 0, h->stream>>>(h->a, h->a.f, h->scratch, nullptr);
+    F64_CK(cudaGetLastError());
+    F64_CK(cudaMemcpyAsync(h->a.f, h->scratch, n * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
+  }
   F64_CK(cudaMemcpyAsync(h->a.r, r.data(), n * sizeof(double4), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaMemcpyAsync(h->a.v, v.data(), n * sizeof(double4), cudaMemcpyHostToDevice, h->stream));
   F64_CK(cudaMemcpyAsync(h->a.im, im.data(), n * sizeof(int4), cudaMemcpyHostToDevice, h->stream));

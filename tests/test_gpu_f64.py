@@ -132,6 +132,25 @@ def test_f64_needs_a_state(capi, oracle):
     lib.b2md_f64_destroy(h)
 
 
+def test_f64_forces_survive_a_new_state(capi, oracle):
+    """The last evaluation's forces, in the caller's order, also after another
+    state is set (the engine sorts its particles; a state resets that order)."""
+    from rumd_b200 import initconf as I
+    params = oracle.lj_params(2, oracle.ka_table())
+    c = I.ka_config(3000, T=1.0, seed=8)
+    e = capi.F64Engine(c["pos4"], c["box"], params, 2, cutoff="SF", vel4=c["vel4"].astype(np.float64))
+    e.run(20)
+    f, pos, vel = e.get("force"), e.get("pos"), e.get("vel")
+    e.set_state(pos[::-1], vel[::-1])
+    assert np.array_equal(e.get("force"), f)
+    assert np.array_equal(e.get("pos"), pos[::-1])
+    e.calc_f()
+    g = e.get("force")
+    e.set_state(pos, vel)
+    assert np.array_equal(e.get("force"), g)
+    e.close()
+
+
 def lj_state(capi, oracle, n, T, steps):
     from rumd_b200 import initconf as I
     params = oracle.lj_params(1, oracle.lj_table())
