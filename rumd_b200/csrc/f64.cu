@@ -542,14 +542,39 @@ namespace {
 
 std::string f64_errmsg;
 
-// Page-locked staging of the read-backs, one piece for all engines of the
-// process (page-locking costs milliseconds, which every engine would pay for
-// its first read-back): allocated by the first read-back, freed with the last
-// engine; the lock is held while it is used.
+// Page-locked staging of the read-backs, a piece for each that is under way
+// (page-locking one costs milliseconds, which every engine would pay for its
+// first read-back): taken from the free pieces of the process, allocated when
+// there is none, and given back; freed with the last engine.  The lock is held
+// for the taking and giving only, so that engines on several threads or GPUs
+// read back at the same time.
 constexpr size_t kStageBytes = (size_t)1 << 20;
+constexpr int kMaxFree = 8;  // free pieces kept
 std::mutex g_stage_mu;
-void* g_stage = nullptr;
-int g_engines = 0;
+void* g_free[kMaxFree];
+int g_nfree = 0, g_engines = 0;
+
+void* take_stage() {
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    if (g_nfree > 0) return g_free[--g_nfree];
+  }
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, kStageBytes, cudaHostAllocPortable) == cudaSuccess) return p;
+  (void)cudaGetLastError();
+  return nullptr;
+}
+
+void give_stage(void* p) {
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mu);
+    if (g_nfree < kMaxFree) {
+      g_free[g_nfree++] = p;
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
 
 int f64_fail(int code, const char* fmt, ...) {
   char buf[512];
@@ -724,10 +749,8 @@ int b2md_f64_destroy(b2md_f64* h) {
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   std::lock_guard<std::mutex> lock(g_stage_mu);
-  if (--g_engines == 0 && g_stage) {
-    cudaFreeHost(g_stage);
-    g_stage = nullptr;
-  }
+  if (--g_engines == 0)
+    while (g_nfree > 0) cudaFreeHost(g_free[--g_nfree]);
   return B2MD_OK;
 }
 
@@ -860,14 +883,20 @@ int b2md_f64_get(b2md_f64* h, int field, void* out) {
     const size_t bytes = (size_t)n * (src ? sizeof(double4) : 3 * sizeof(int));
     k64_unsort<<<nblocks(h), kB, 0, h->stream>>>(h->a, src, h->scratch, reinterpret_cast<int*>(h->scratch));
     F64_CK(cudaGetLastError());
-    std::lock_guard<std::mutex> lock(g_stage_mu);
-    if (!g_stage) F64_CK(cudaHostAlloc(&g_stage, kStageBytes, cudaHostAllocPortable));
-    for (size_t b = 0; b < bytes; b += kStageBytes) {
-      const size_t m = std::min(kStageBytes, bytes - b);
-      F64_CK(cudaMemcpyAsync(g_stage, reinterpret_cast<const char*>(h->scratch) + b, m, cudaMemcpyDeviceToHost, h->stream));
-      F64_CK(cudaStreamSynchronize(h->stream));
-      std::memcpy(static_cast<char*>(out) + b, g_stage, m);
+    void* stage = take_stage();
+    cudaError_t err = cudaSuccess;
+    if (!stage) {  // no page-locked memory to be had
+      err = cudaMemcpyAsync(out, h->scratch, bytes, cudaMemcpyDeviceToHost, h->stream);
+      if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
     }
+    for (size_t b = 0; stage && b < bytes && err == cudaSuccess; b += kStageBytes) {
+      const size_t m = std::min(kStageBytes, bytes - b);
+      err = cudaMemcpyAsync(stage, reinterpret_cast<const char*>(h->scratch) + b, m, cudaMemcpyDeviceToHost, h->stream);
+      if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
+      if (err == cudaSuccess) std::memcpy(static_cast<char*>(out) + b, stage, m);
+    }
+    if (stage) give_stage(stage);
+    F64_CK(err);
     return B2MD_OK;
   }
   return f64_fail(B2MD_ERR_ARG, "b2md_f64_get: unknown field %d", field);

@@ -3,6 +3,7 @@ built by changeToDouble.sh) against the FP64 oracle, and the FP32 engine
 against it: the accuracy statements for the single-component LJ system of
 N = 1,048,576 at density 0.8442 (the HBM-scale plain configuration)."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -149,6 +150,38 @@ def test_f64_forces_survive_a_new_state(capi, oracle):
     e.set_state(pos, vel)
     assert np.array_equal(e.get("force"), g)
     e.close()
+
+
+def test_f64_read_backs_of_several_engines_and_pieces(capi, oracle):
+    """Known states of several megabytes (an odd rest in the last piece) come
+    back whole, one engine per thread, all at once."""
+    params = oracle.lj_params(1, oracle.lj_table())
+    n, box = 100003, 49.2
+
+    def states(k):
+        rng = np.random.default_rng(k)
+        pos = np.zeros((n, 4))
+        pos[:, :3] = rng.uniform(-box / 2, box / 2, (n, 3))
+        vel = np.ones((n, 4))
+        vel[:, :3] = rng.standard_normal((n, 3))
+        return pos, vel, rng.integers(-9, 9, (n, 3)).astype(np.int32)
+
+    def work(k, bad):
+        pos, vel, im = states(k)
+        e = capi.F64Engine(pos, box, params, 1, cutoff="SP", vel4=vel, im3=im, max_nbrs=160)
+        for _ in range(4):
+            for name, want in (("pos", pos), ("vel", vel), ("images", im)):
+                if not np.array_equal(e.get(name), want):
+                    bad.append((k, name))
+        e.close()
+
+    bad = []
+    threads = [threading.Thread(target=work, args=(k, bad)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
 
 
 def lj_state(capi, oracle, n, T, steps):
