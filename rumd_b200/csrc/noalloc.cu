@@ -239,14 +239,16 @@ __device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G
     const bool in = d2 < c.x && j != p0 + q;
     if (!__any_sync(0xffffffffu, in)) continue;
     // the engine's pair function (pair_add of the step kernels), with 1/r^2 the
-    // hardware reciprocal of d^2 (one unit in the last place) and 1/r, which
-    // only the small shifted-force term uses, the reciprocal square root
+    // hardware reciprocal of d^2 (one unit in the last place; the energies'
+    // error against 64-bit sums is a tenth of that with the square of 1/r) and
+    // 1/r, which only the shifted-force term uses, refined as there
     const float2 e = *reinterpret_cast<const float2*>(row + 4);  // c_u0, 6 A6
-    const float i2 = b2md::rcp_approx(d2), y = b2md::rsqrt_approx(d2);
-    const float i6 = i2 * i2 * i2, t = c.y * i6, w = c.w * y;
-    const float s = __fmaf_rn(i6 * i2, __fmaf_rn(12.f, t, e.y), -w);
+    const float i2 = b2md::rcp_approx(d2), i6 = i2 * i2 * i2, t = c.y * i6;
+    float y = b2md::rsqrt_approx(d2);
+    y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
+    const float s = __fmaf_rn(-c.w, y, i6 * i2 * __fmaf_rn(12.f, t, e.y));
     if (in) {  // (dx is NaN in lanes without a candidate)
-      A[q].u += __fmaf_rn(w, d2, __fmaf_rn(i6, t + c.z, e.x));
+      A[q].u += __fmaf_rn(i6, t + c.z, __fmaf_rn(c.w, d2 * y, e.x));
       A[q].fx = __fmaf_rn(dx[q], s, A[q].fx);
       A[q].fy = __fmaf_rn(dy[q], s, A[q].fy);
       A[q].fz = __fmaf_rn(dz[q], s, A[q].fz);

@@ -30,9 +30,9 @@ __device__ __forceinline__ float dist2_ref(float dx, float dy, float dz) {
 }
 
 // Hardware approximate 1/x and 1/sqrt(x) (one MUFU operation each, denormals
-// flushed; relative errors at most 2^-23 and 2^-22.9); the step kernels refine
-// 1/sqrt(x) with a Newton-Raphson step.  Arguments here are squared distances,
-// far from the denormal range.
+// flushed; relative errors at most 2^-23 and 2^-22.9); callers refine 1/sqrt(x)
+// with a Newton-Raphson step.  Arguments here are squared distances, far from
+// the denormal range.
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -165,6 +165,44 @@ def test_noalloc_forms_against_fp64_sums(n, lengths, spread):
     assert abs(s[1] - W) <= 1e-5 * np.abs(ref[ok, :3]).sum()
 
 
+@pytest.mark.parametrize("pairs", [300, 1250, 2100])
+def test_noalloc_shifted_force_term_is_the_engines(pairs):
+    """Particles in isolated pairs, in all three forms, of a table without
+    repulsion and attraction: forces and energies are the shifted-force terms
+    c/r and c r alone, which must be the engine's bit for bit (1/r refined)."""
+    import torch
+    from rumd_b200 import capi, initconf
+    rng = np.random.default_rng(pairs)
+    n, m = 2 * pairs, int(np.ceil(pairs ** (1 / 3)))
+    box = np.full(3, 6.0 * m, np.float32)
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:pairs]
+    u = rng.standard_normal((pairs, 3))
+    u *= rng.uniform(0.85, 2.6, (pairs, 1)) / np.linalg.norm(u, axis=1, keepdims=True)
+    x = (g + 0.5) * 6.0 - 3.0 * m + rng.uniform(-0.4, 0.4, (pairs, 3))
+    pos4 = np.zeros((n, 4), np.float32)
+    pos4[:, :3] = np.concatenate([x - u / 2, x + u / 2])[rng.permutation(n)]
+    pos4[:, 3] = (rng.random(n) < 0.3).astype(np.int32).view(np.float32)
+    params = np.ascontiguousarray(initconf.lj_params(2, initconf.KA), np.float32)
+    params.reshape(-1, 12)[:, 1:3] = 0.0  # A12, A6
+    params.reshape(-1, 12)[:, 10:] = rng.uniform(0.5, 1.5, (4, 2))  # s(rc) rc, u(rc)
+    e = capi.Engine(device=0, pb=64, tp=4)
+    rid = e.add(pos4, box, params, 2, cutoff="SF")
+    e.calc_f()
+    want = e.get(rid, "force", n)
+    e.close()
+    dev = torch.device("cuda:0")
+    p = torch.from_numpy(pos4).to(dev)
+    force = torch.zeros((n, 4), dtype=torch.float32, device=dev)
+    sums = torch.zeros(2, dtype=torch.float64, device=dev)
+    rc = _call(capi.lib(), ctypes.c_void_p(p.data_ptr()), n, box, params, capi.CUTOFF["SF"],
+               ctypes.c_void_p(force.data_ptr()), ctypes.c_void_p(sums.data_ptr()),
+               ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    assert rc == capi.B2MD_OK
+    torch.cuda.synchronize(dev)
+    assert np.count_nonzero(want[:, 3]) > n // 2
+    assert np.array_equal(force.cpu().numpy(), want)
+
+
 def test_noalloc_rejects_sizes_beyond_its_maximum():
     from rumd_b200 import capi
     lib = capi.lib()
