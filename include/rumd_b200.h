@@ -413,8 +413,9 @@ B2MD_API int b2md_probe_nvt(const float* r4, const float* v4, const float* f4, c
  * are binned in cells where that pays).  n is at most 65536: the only scratch
  * is a fixed array of that capacity (about 3 MB) in the library's device
  * image, one per GPU, kept until the process exits and shared by every
- * call, so calls that overlap on the GPU race; order them on one stream.  The
- * first call on each device looks up the array's device address
+ * call, so the results of calls that overlap on the GPU are undefined (each
+ * still writes its own outputs only); order them on one stream.  The first
+ * call on each device looks up the array's device address
  * (cudaGetSymbolAddress) with that device current; make that first call
  * before any stream capture.  A later call in another CUDA context of the
  * device (after cudaDeviceReset, say) looks it up again.  Every cut-off must

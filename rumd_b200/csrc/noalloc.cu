@@ -15,8 +15,11 @@
 // The array exists once per GPU that loads the library and lives until the
 // process exits.  Every call shares it, so calls whose kernels overlap on the
 // GPU (different streams, no ordering between them) race on it; order them on
-// one stream or with events.  The completion counter and the cell counts are
-// cleared at the start of every call; the rest is overwritten before it is read.
+// one stream or with events.  Their results are then undefined, but nothing
+// outside the scratch and the calls' own outputs is touched: every index that
+// comes from the scratch is held to the call's particles.  The completion
+// counter and the cell counts are cleared at the start of every call; the rest
+// is overwritten before it is read.
 //
 // Host code cannot use the array's name as a device address (it names a
 // host-side stand-in).  The first call on a device, with that device current,
@@ -65,7 +68,7 @@ struct NoAllocScratch {
   double part[kNoAllocMaxBlocks][2];  // per-block sums of u_i and w_i
 };
 constexpr unsigned kBadType = 0x80000000u;
-constexpr unsigned kNoParticle = 0xffffffffu;  // a group's place without a particle
+constexpr unsigned kNoParticle = 0xffffffffu;  // a group's place without a particle: past every n
 // One warp lists a cell's particles, so a few crowded cells (a cluster in a
 // box so large that its cells cannot be small) would leave the work to a few
 // warps: then the all-pairs form runs, which spreads evenly.
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(1024) k_na_scan(int ncell, NoAllocScratch* scr
 
 __global__ void __launch_bounds__(256) k_na_scatter(int n, NoAllocScratch* scr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) scr->order[scr->start[scr->key[i]] + scr->rank[i]] = i;
+  if (i < n) scr->order[min(scr->start[scr->key[i]] + scr->rank[i], n - 1)] = i;
 }
 
 // Each bucket by index (its members counted against each other; a few per
@@ -160,9 +163,10 @@ __global__ void __launch_bounds__(256) k_na_gather(const float4* __restrict__ po
                                                    int ntypes, NoAllocScratch* scr) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n || scr->dense) return;
-  const int i = scr->order[s], c = scr->key[i], b = scr->start[c], m = scr->cnt[c];
+  const int i = min(scr->order[s], n - 1), c = scr->key[i], b = min(scr->start[c], n), m = min(scr->cnt[c], n - b);
   int place = b;
   for (int k = 0; k < m; ++k) place += scr->order[b + k] < i;
+  place = min(place, n - 1);
   float4 r = pos[i];
   const int t = __float_as_int(r.w);
   const bool ok = t >= 0 && t < ntypes;
@@ -260,8 +264,8 @@ __device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G
 // Forces of particles p0 .. p0 + G - 1 from the sums, by the lanes that hold
 // them; their energies and virials are added to u, w.
 template <int G>
-__device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned (&id)[G], float4* __restrict__ force,
-                                             double& u, double& w) {
+__device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned (&id)[G], int n,
+                                             float4* __restrict__ force, double& u, double& w) {
   float v[5][G];
 #pragma unroll
   for (int q = 0; q < G; ++q) {
@@ -274,7 +278,7 @@ __device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned 
     unsigned me = id[0];
 #pragma unroll
     for (int q = 1; q < G; ++q) me = lane / (32 / G) == q ? id[q] : me;
-    if (me == kNoParticle) {
+    if ((me & ~kBadType) >= (unsigned)n) {
     } else if (me & kBadType) {
       const float nanf_ = __int_as_float(0x7fc00000);
       force[me & ~kBadType] = make_float4(nanf_, nanf_, nanf_, nanf_);
@@ -290,8 +294,8 @@ __device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned 
 // which is in range of nothing).  The next round's candidates are loaded while
 // the current one's pairs are computed.
 template <int G>
-__device__ __forceinline__ void cell_group(NoAllocScratch* scr, const int4* tab, int off, int len, int total, int p0,
-                                           int m, unsigned wrap, const float* s_tab, int ntypes, const float3& L,
+__device__ __forceinline__ void cell_group(NoAllocScratch* scr, int n, const int4* tab, int off, int len, int total,
+                                           int p0, int m, unsigned wrap, const float* s_tab, int ntypes, const float3& L,
                                            const float3& iL, float4* __restrict__ force, double& u, double& w) {
   const int lane = threadIdx.x & 31;
   const float nan = __int_as_float(0x7fc00000);
@@ -326,7 +330,7 @@ __device__ __forceinline__ void cell_group(NoAllocScratch* scr, const int4* tab,
     if (ch + lane >= total) rj.x = nan;
     add_candidate<G>(A, rp, p0, j, rj, wrap, s_tab, ntypes, L, iL);
   }
-  store_forces<G>(A, id, force, u, w);
+  store_forces<G>(A, id, n, force, u, w);
 }
 
 template <int G>
@@ -356,7 +360,7 @@ __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, 
     }
     add_candidate<G>(A, rp, p0, j, rj, 7u, s_tab, ntypes, L, iL);
   }
-  store_forces<G>(A, id, force, u, w);
+  store_forces<G>(A, id, n, force, u, w);
 }
 
 // One warp works on up to four particles at a time, 32 candidates a round, one
@@ -376,18 +380,19 @@ __global__ void __launch_bounds__(kNoAllocBlock, 7)
   __shared__ __align__(16) float s_tab[kNoAllocMaxTypes * kNoAllocMaxTypes * kRow];
   __shared__ int4 s_rows[kNoAllocWarps * kRows];
   __shared__ double s_red[kNoAllocBlock][2];
-  __shared__ int s_last;
+  __shared__ int s_last, s_cells;
+  if (threadIdx.x == 0) s_cells = CELLS && !scr->dense;
   for (int k = threadIdx.x; k < ntypes * ntypes * kRow; k += blockDim.x) s_tab[k] = tab.p[k];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int stride = gridDim.x * kNoAllocWarps;
   double u = 0.0, w = 0.0;
-  const bool by_cell = CELLS && !scr->dense;
-  if (by_cell) {
+  if (s_cells) {
     int4* rowtab = s_rows + warp * kRows;
     const int ncell = g.nx * g.ny * g.nz;
     for (int c = blockIdx.x * kNoAllocWarps + warp; c < ncell; c += stride) {
-      const int p0 = scr->start[c], p1 = p0 + scr->cnt[c];
+      const int p0 = __shfl_sync(0xffffffffu, min(scr->start[c], n), 0);
+      const int p1 = __shfl_sync(0xffffffffu, min(p0 + scr->cnt[c], n), 0);
       if (p0 >= p1) continue;
       const int cx = c % g.nx, cy = (c / g.nx) % g.ny, cz = c / (g.nx * g.ny);
       // with at least 7 cells and none of the five wrapped, candidates are
@@ -404,11 +409,11 @@ __global__ void __launch_bounds__(kNoAllocBlock, 7)
         const int ca = row + (lo < 0 ? lo + g.nx : lo), cb = row + (hi >= g.nx ? hi - g.nx : hi);
         const bool two = lo < 0 || hi >= g.nx;
         const int ce = two ? row + g.nx - 1 : cb;  // last cell of the first run
-        b0 = scr->start[ca];
-        l0 = scr->start[ce] + scr->cnt[ce] - b0;
+        b0 = min(scr->start[ca], n);
+        l0 = max(min(scr->start[ce] + scr->cnt[ce], n) - b0, 0);
         if (two) {
-          b1 = scr->start[row];
-          l1 = scr->start[cb] + scr->cnt[cb] - b1;
+          b1 = min(scr->start[row], n);
+          l1 = max(min(scr->start[cb] + scr->cnt[cb], n) - b1, 0);
         }
       }
       const int len = l0 + l1;
@@ -419,13 +424,14 @@ __global__ void __launch_bounds__(kNoAllocBlock, 7)
         if (lane >= o) incl += y;
       }
       const int off = incl - len, total = __shfl_sync(0xffffffffu, incl, 31);
+      if (total == 0) continue;  // (only beside an overlapping call: a cell is its own neighbour)
       const unsigned ne = __ballot_sync(0xffffffffu, len > 0);
       __syncwarp();
       if (len > 0) rowtab[__popc(ne & ((1u << lane) - 1u))] = make_int4(off, b0 - off, off + l0, b1 - off - l0);
       __syncwarp();
       for (int p = p0; p < p1; p += 4) {
         const int m = min(4, p1 - p);
-#define CG(K) cell_group<K>(scr, rowtab, off, len, total, p, m, wrap, s_tab, ntypes, L, iL, force, u, w)
+#define CG(K) cell_group<K>(scr, n, rowtab, off, len, total, p, m, wrap, s_tab, ntypes, L, iL, force, u, w)
         if (m > 2) CG(4);
         else CG(2);
 #undef CG

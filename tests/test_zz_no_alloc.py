@@ -203,6 +203,44 @@ def test_noalloc_shifted_force_term_is_the_engines(pairs):
     assert np.array_equal(force.cpu().numpy(), want)
 
 
+def test_noalloc_overlapping_calls_stay_in_their_outputs():
+    """Calls that share the scratch because nothing orders them have undefined
+    results, but write only their own outputs, and leave the next call right."""
+    import torch
+    from rumd_b200 import capi, initconf
+    lib, dev, pad = capi.lib(), torch.device("cuda:0"), 4096
+    params = np.ascontiguousarray(initconf.lj_params(2, initconf.KA), np.float32)
+    calls = []
+    for n, T in ((65521, 1.0), (3000, 1.0), (30011, 1.0)):
+        c = initconf.ka_config(n, T=T, seed=n)
+        calls.append(dict(n=n, box=np.ascontiguousarray(c["box"], np.float32), pos=torch.from_numpy(c["pos4"]).to(dev),
+                          out=torch.full((n + 2 * pad, 4), 7.0, device=dev),
+                          sums=torch.zeros(2, dtype=torch.float64, device=dev), stream=torch.cuda.Stream(dev)))
+
+    def launch(c):
+        rc = _call(lib, ctypes.c_void_p(c["pos"].data_ptr()), c["n"], c["box"], params, capi.CUTOFF["SP"],
+                   ctypes.c_void_p(c["out"][pad:].data_ptr()), ctypes.c_void_p(c["sums"].data_ptr()),
+                   ctypes.c_void_p(c["stream"].cuda_stream))
+        assert rc == capi.B2MD_OK
+
+    torch.cuda.synchronize(dev)
+    want = []
+    for c in calls:
+        launch(c)
+        torch.cuda.synchronize(dev)
+        want.append(c["out"].clone())
+    for _ in range(30):
+        for c in calls:
+            launch(c)
+    torch.cuda.synchronize(dev)
+    for c in calls:
+        assert (c["out"][:pad] == 7.0).all() and (c["out"][pad + c["n"]:] == 7.0).all()
+    for c, w in zip(calls, want):
+        launch(c)
+        torch.cuda.synchronize(dev)
+        assert torch.equal(c["out"], w)
+
+
 def test_noalloc_rejects_sizes_beyond_its_maximum():
     from rumd_b200 import capi
     lib = capi.lib()
