@@ -647,7 +647,9 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
     k_na_scan<<<1, 1024, 0, s>>>(ncell, scr);
     k_na_scatter<<<tb, 256, 0, s>>>(n, scr);
     k_na_gather<<<tb, 256, 0, s>>>(p4, n, L, iL, ntypes, scr);
-    NA(4, true, ncell);
+    // (a warp per cell, and warps enough for all pairs, four particles each,
+    // should the cells turn out crowded)
+    NA(4, true, std::max(ncell, (n + 3) / 4));
   } else if (n <= 2400) {
     NA(1, false, n);
   } else if (n <= 4800) {
