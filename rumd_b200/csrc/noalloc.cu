@@ -58,7 +58,7 @@ constexpr int kRows = 25;  // (dz, dy) rows of a cell's 5x5x5 neighbourhood
 
 struct NoAllocScratch {
   unsigned counter;            // blocks finished in this call; cleared with cnt
-  int dense;                   // a cell holds more than kDense particles: all pairs instead
+  int dense;                   // a cell is too crowded (crowd_limit): all pairs instead
   unsigned pad[62];
   int cnt[kNoAllocMaxCells];   // particles per cell
   int start[kNoAllocMaxCells]; // first sorted place of each cell
@@ -69,10 +69,26 @@ struct NoAllocScratch {
 };
 constexpr unsigned kBadType = 0x80000000u;
 constexpr unsigned kNoParticle = 0xffffffffu;  // a group's place without a particle: past every n
-// One warp lists a cell's particles, so a few crowded cells (a cluster in a
-// box so large that its cells cannot be small) would leave the work to a few
-// warps: then the all-pairs form runs, which spreads evenly.
+// One warp works on a cell's particles, so a few crowded cells (a cluster in a
+// much larger box) would leave the work to a few warps: then the all-pairs form
+// runs, which spreads evenly.  A round of 32 candidates takes a warp about
+// 0.5 us in both, so their longest chains are compared: the fullest cell's
+// groups of four against 125 cells as full, and a warp's share of all pairs.
+// The first is three to four times what the fullest cell of an even liquid
+// has, whose neighbours hold the mean, hence the factor.  With the number in a
+// cell as the only bound, a droplet of density 0.06 in a box of 400 took
+// 1297 us at N=8000 and 747 at N=3500, now 172 and 94 (one thread per particle
+// against all, before there were cells: 673 and 302).
 constexpr int kDense = 64;
+constexpr int kResidentWarps = 148 * 7 * kNoAllocWarps;  // k_forces_noalloc
+
+// The largest number of particles in a cell for which the cells are used.
+int crowd_limit(int n) {
+  const long long all = (long long)(((n + 3) / 4 + kResidentWarps - 1) / kResidentWarps) * n;
+  int most = kDense;
+  while (most > 1 && (long long)((most + 3) / 4) * std::min(n, 125 * most) > 4 * all) --most;
+  return most;
+}
 
 // The scratch: a fixed array in the library's device image (no allocation).
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
@@ -114,7 +130,7 @@ __global__ void __launch_bounds__(256) k_na_count(const float4* __restrict__ pos
 
 // exclusive scan of the cell counts (and the largest) by one block: thread t
 // owns a run of cells
-__global__ void __launch_bounds__(1024) k_na_scan(int ncell, NoAllocScratch* scr) {
+__global__ void __launch_bounds__(1024) k_na_scan(int ncell, int limit, NoAllocScratch* scr) {
   __shared__ int s_w[32], s_m[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int run = ((ncell + 1023) / 1024 + 3) & ~3;  // whole int4 loads
@@ -141,7 +157,7 @@ __global__ void __launch_bounds__(1024) k_na_scan(int ncell, NoAllocScratch* scr
   for (int w = 0; w < wid; ++w) first += s_w[w];
   if (threadIdx.x == 0) {
     for (int w = 1; w < 32; ++w) most = max(most, s_m[w]);
-    scr->dense = most > kDense;
+    scr->dense = most > limit;
   }
   for (int c = c0; c < c1; c += 4) {
     const int4 x = *reinterpret_cast<const int4*>(scr->cnt + c);
@@ -644,7 +660,7 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
                            0, s>>>(p4, n, L, iL, g, ntypes, tab, f4, sums, scr)
   if (cells) {
     k_na_count<<<tb, 256, 0, s>>>(p4, n, L, iL, g, scr);
-    k_na_scan<<<1, 1024, 0, s>>>(ncell, scr);
+    k_na_scan<<<1, 1024, 0, s>>>(ncell, crowd_limit(n), scr);
     k_na_scatter<<<tb, 256, 0, s>>>(n, scr);
     k_na_gather<<<tb, 256, 0, s>>>(p4, n, L, iL, ntypes, scr);
     // (a warp per cell, and warps enough for all pairs, four particles each,

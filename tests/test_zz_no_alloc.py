@@ -106,11 +106,12 @@ def _brute_force(pos4, box, params, cutoff):
 
 # (particles, box, spread): the last sizes of the one-, two- and four-particle
 # all-pairs forms, the first of the cell form, a box too thin for cells, a
-# cluster that crowds its cells (all pairs again), and positions several box
-# lengths outside
+# cluster and a droplet that crowd their cells (all pairs again), one that
+# does not, and positions several box lengths outside
 EDGES = [(2, (9, 9, 9), "all"), (33, (9, 9, 9), "all"), (2400, (13, 13, 13), "all"), (2401, (13, 13, 13), "all"),
          (2999, (14, 14, 13), "all"), (3000, (14, 14, 13), "all"), (3001, (40, 11, 6.2), "all"),
-         (3100, (15, 13, 17.5), "outside"), (3500, (400, 390, 410), "cluster"), (4801, (36, 36, 6), "all")]
+         (3100, (15, 13, 17.5), "outside"), (3500, (400, 390, 410), "cluster"),
+         (3500, (400, 390, 410), "droplet"), (3501, (120, 110, 125), "droplet"), (4801, (36, 36, 6), "all")]
 
 
 @pytest.mark.parametrize("n,lengths,spread", EDGES)
@@ -122,7 +123,8 @@ def test_noalloc_forms_against_fp64_sums(n, lengths, spread):
     from rumd_b200 import capi, initconf
     rng = np.random.default_rng(n)
     box = np.array(lengths, np.float32)
-    ext = np.array((14.0, 14.0, 14.0)) if spread == "cluster" else box.astype(np.float64)
+    side = {"cluster": 14.0, "droplet": 46.0}.get(spread)
+    ext = box.astype(np.float64) if side is None else np.full(3, side)
     if n == 2:
         ext = np.full(3, 2.0)  # in range of each other
     m = np.maximum(1, np.ceil(ext * (n / ext.prod()) ** (1 / 3) * 1.08)).astype(int)
