@@ -395,6 +395,10 @@ B2MD_API int b2md_probe_cell(const float* x, int n, float box, int nc, int* out)
  * (TFLOP/s, independent FMA chains), best of `trials`, CUDA-event timed.
  * No counterpart in the reference (measurement only). */
 B2MD_API int b2md_measure_peaks(int trials, double* l2_gbs, double* fma_tflops);
+/* Makes the next particle sort's blocks wait for one that never comes, so that
+ * its bounded waits run out (about a second) and the call that sorts returns
+ * B2MD_ERR_CUDA; the calls after it work again.  For tests. */
+B2MD_API int b2md_probe_stall_sort(b2md_engine* e);
 B2MD_API int b2md_probe_nvt(const float* r4, const float* v4, const float* f4, const float* xi, float dt,
                             const float* box, int n, float* ref9, float* eng9);
 

@@ -44,7 +44,7 @@ EXPORTS = [
     "b2md_integrate", "b2md_zero_momentum", "b2md_run", "b2md_run_timed", "b2md_replica_queue_steps",
     "b2md_run_queued", "b2md_nbl_export", "b2md_sort_export", "b2md_cell_grid", "b2md_sync",
     "b2md_stream", "b2md_last_error", "b2md_version", "b2md_probe_dist2", "b2md_probe_cell",
-    "b2md_probe_nvt", "b2md_measure_peaks",
+    "b2md_probe_nvt", "b2md_probe_stall_sort", "b2md_measure_peaks",
     "b2md_forces_noalloc", "b2md_f64_create", "b2md_f64_destroy", "b2md_f64_set_state",
     "b2md_f64_set_integrator", "b2md_f64_set_xi", "b2md_f64_calc_f", "b2md_f64_run", "b2md_f64_get",
     "b2md_f64_stats",
@@ -118,6 +118,7 @@ def lib():
             "b2md_sync": [P],
             "b2md_probe_dist2": [P, P, P, i, P],
             "b2md_probe_cell": [P, i, f, i, P],
+            "b2md_probe_stall_sort": [P],
             "b2md_probe_nvt": [P, P, P, P, f, P, i, P, P],
             "b2md_measure_peaks": [i, ctypes.POINTER(d), ctypes.POINTER(d)],
             "b2md_forces_noalloc": [P, i, P, i, P, i, P, P, P],

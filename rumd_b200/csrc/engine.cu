@@ -1370,13 +1370,22 @@ void check_persist(b2md_engine* e, const int* known = nullptr) {
   }
 }
 
+// Reports the bounded device wait that gave up for replica r (RepState::err).
+[[noreturn]] void wait_failed(b2md_engine* e, size_t r, int err) {
+  if (err != ERR_WAIT_SORT)
+    api_fail(B2MD_ERR_CUDA, "a bounded device wait for the neighbour-list copy gave up (replica " + std::to_string(r) + ")");
+  CK(cudaStreamSynchronize(e->stream));
+  k_clear_sort<<<1, 256, 0, e->stream>>>(make_args(e));
+  check_launch();
+  api_fail(B2MD_ERR_CUDA, "a bounded wait of the particle sort's blocks for one another gave up (replica " +
+                              std::to_string(r) + "); its list is due again");
+}
+
 // Overflowed lists: double the capacity (NeighborList.cu:657-676) and flag a rebuild.
 bool repair_overflow(b2md_engine* e, const std::vector<RepState>& s) {
   bool any = false;
   for (size_t r = 0; r < e->reps.size(); ++r)
-    if (e->reps[r].active && s[r].err)
-      api_fail(B2MD_ERR_CUDA, "a bounded device wait for the neighbour-list copy gave up (replica " +
-                                  std::to_string(r) + ")");
+    if (e->reps[r].active && s[r].err) wait_failed(e, r, s[r].err);
   for (size_t r = 0; r < e->reps.size(); ++r) {
     HostRep& h = e->reps[r];
     if (!h.active || !s[r].overflow) continue;
@@ -1496,9 +1505,7 @@ void finish_chunk(b2md_engine* e, ChunkRec& c) {
     HostRep& h = e->reps[r];
     if (!c.active[r] || !h.active || h.admit_seq >= c.ticket) continue;  // not the replica the chunk ran
     const RepState& st = c.h_st[r];
-    if (st.err)
-      api_fail(B2MD_ERR_CUDA, "a bounded device wait for the neighbour-list copy gave up (replica " +
-                                  std::to_string(r) + ")");
+    if (st.err) wait_failed(e, r, st.err);
     if (!st.overflow || h.repair_seq >= c.ticket) continue;
     int want = std::max(h.d.max_nbrs * 2, st.actual_max_nbrs + 8);
     want = std::min(want, std::max(h.n - 1, 1));
@@ -2331,6 +2338,16 @@ int b2md_replica_stress(b2md_engine* e, int id, int include_kinetic, double* out
     stage.done();
     double V = (double)h.d.L[0] * h.d.L[1] * h.d.L[2];
     for (int k = 0; k < 6; ++k) out6[k] = 0.5 * st[k] / V;
+  });
+}
+
+int b2md_probe_stall_sort(b2md_engine* e) {
+  if (!e) return fail(B2MD_ERR_ARG, "null engine");
+  return guarded([&] {
+    CK(cudaSetDevice(e->device));
+    const unsigned far = 1u << 30;  // past any number of blocks
+    CK(cudaMemcpyAsync(&e->pctl->sort_arrive, &far, sizeof far, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaStreamSynchronize(e->stream));
   });
 }
 

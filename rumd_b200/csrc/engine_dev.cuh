@@ -100,13 +100,17 @@ struct RepState {
   int rebuild, exceed;
   int overflow, nrebuilds;
   int actual_max_nbrs, nlog;
-  int err;               // a bounded device wait gave up (reported to the host)
+  int err;               // a bounded device wait gave up: ERR_WAIT_* (reported to the host)
   unsigned sort_done;    // k_batch: epoch of the replica's last in-launch sort
   unsigned sort_items;   // k_batch: phase items of the replica's split sort completed (reset by the last)
   int flow_left;         // k_flow: items of the replica's current phase not yet finished
   int launch_steps;      // k_flow: steps the replica ran in the current launch
   int build_next;        // k_rb_build_runs: the replica's next unclaimed cell (0 between builds)
 };
+
+// RepState::err: the wait for the tile's list or window copies; the wait of
+// k_rb_sort's blocks for one another.
+enum { ERR_WAIT_COPY = 1, ERR_WAIT_SORT = 2 };
 
 // Control block of the persistent step kernel (k_steps), one per engine.
 struct PersistCtl {
@@ -131,8 +135,10 @@ struct PersistCtl {
   int active;
   int ran;
   unsigned exited;
-  // k_rb_sort's grid barrier
+  // k_rb_sort's grid barrier; sort_bad: one of its waits gave up, and no sort
+  // runs until the host has put the words back
   unsigned sort_arrive, sort_gen;
+  int sort_bad;
 };
 
 struct EngArgs {

@@ -981,7 +981,7 @@ __device__ __forceinline__ bool force_tile(const EngArgs& a, int tile, unsigned 
       } else {
         // the copies did not land in time: record it for the host and wait
         // (bounded) for them before this block's shared memory is released
-        if (threadIdx.x == 0) atomicExch(&S->err, 1);
+        if (threadIdx.x == 0) atomicExch(&S->err, ERR_WAIT_COPY);
         mbar_wait_bounded(&s_bar, 0, kWaitPolls);
       }
     } else {
@@ -1623,6 +1623,23 @@ __global__ void k_set_steps(EngArgs a, long long nsteps, int reset_run_step) {
 // before it).
 __global__ void k_queue_steps(RepState* s, long long nsteps) { s->steps_left += nsteps; }
 
+// After a sort that gave up (and with it nothing moved: the parities flip
+// last): its barrier's words and the counters of its permute phase as before
+// the launch, the replicas it froze due for a list again.
+__global__ void k_clear_sort(EngArgs a) {
+  for (int r = threadIdx.x; r < a.nrep; r += blockDim.x) {
+    a.rctr[r] = 0u;
+    if (a.st[r].err == ERR_WAIT_SORT) {
+      a.st[r].err = 0;
+      a.st[r].overflow = 0;
+    }
+  }
+  if (threadIdx.x == 0) {
+    a.pctl->sort_arrive = 0u;
+    a.pctl->sort_bad = 0;
+  }
+}
+
 // An enlarged list is in place: the replica's overflow flag is cleared and
 // its list is due (in stream order).
 __global__ void k_clear_overflow(RepState* s) {
@@ -1680,7 +1697,8 @@ __device__ __forceinline__ bool flag_overflow(const RepDev& R, RepState* S) {
 __device__ __forceinline__ int cell_chunk(const RepDev& R) { return (R.ncell + R.ntiles - 1) / R.ntiles; }
 
 // Grid barrier of k_rb_sort (every block resident); false, in every thread,
-// when the wait gave up.
+// when the wait gave up (about a second).
+constexpr unsigned kSortPolls = 1u << 20;
 __device__ bool sort_barrier(PersistCtl* c) {
   __shared__ int s_ok;
   __syncthreads();
@@ -1692,11 +1710,14 @@ __device__ bool sort_barrier(PersistCtl* c) {
       st_release_u32(&c->sort_gen, gen + 1u);
     } else {
       unsigned it = 0;
-      while (ld_acquire_u32(&c->sort_gen) == gen && it < kBarrierPolls) {
+      while (ld_acquire_u32(&c->sort_gen) == gen && it < kSortPolls) {
         __nanosleep(20);
         ++it;
       }
-      if (it >= kBarrierPolls) s_ok = 0;
+      if (it >= kSortPolls) {
+        atomicExch(&c->sort_bad, 1);
+        s_ok = 0;
+      }
     }
     __threadfence();
   }
@@ -1729,8 +1750,10 @@ constexpr int kScanGroup = 128;
 constexpr int kSortBlock = 512;
 __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
   constexpr unsigned FULL = 0xffffffffu;
+  __shared__ int s_bad;
   const int tid = threadIdx.x, lane = tid & 31;
   {
+    if (tid == 0) s_bad = __ldcg(&a.pctl->sort_bad);
     int any = 0;
     for (int r = tid; r < a.nrep; r += kSortBlock) any |= rb_active(a, r) ? 1 : 0;
     if (!__syncthreads_or(any)) return;
@@ -1738,9 +1761,9 @@ __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
   const int gid = blockIdx.x * kSortBlock + tid, gsz = gridDim.x * kSortBlock;
   const int warps = gsz >> 5;
   PersistCtl* ctl = a.pctl;
-  bool ok = true;
+  bool ok = s_bad == 0;
   // clear
-  for (int tile = gid >> 5; tile < a.ntiles; tile += warps) {
+  for (int tile = gid >> 5; ok && tile < a.ntiles; tile += warps) {
     const int rep = a.tile_rep[tile];
     if (!rb_active(a, rep)) continue;
     const RepDev& R = a.rep[rep];
@@ -1754,7 +1777,7 @@ __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
       a.cpref[tile] = 0;  // (the groups' totals are the replica's first entries)
     }
   }
-  ok = sort_barrier(ctl);
+  if (ok) ok = sort_barrier(ctl);
   // count (whole warps work on 32 slots of one tile: pb is a multiple of 32)
   const int tpt = pb >> 5;  // warps per tile
   if (ok) {
@@ -1825,9 +1848,14 @@ __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
     ok = sort_barrier(ctl);
   }
   if (!ok) {
-    // (reported by the host; nothing else acts on a replica whose err is set)
-    for (int r = gid; r < a.nrep; r += gsz)
-      if (rb_active(a, r)) atomicExch(&a.st[r].err, 1);
+    // reported by the host; until then the replicas are frozen, as by an
+    // overflow: nothing builds their lists or steps with the old ones.  Every
+    // block that gave up marks them (others may have got through).
+    for (int r = tid; r < a.nrep; r += kSortBlock)
+      if (rb_active(a, r)) {
+        atomicExch(&a.st[r].overflow, 1);
+        atomicExch(&a.st[r].err, ERR_WAIT_SORT);
+      }
     return;
   }
   // permute

@@ -148,6 +148,53 @@ def test_coordinates_outside_the_box(capi, n, box, set_later):
     assert np.array_equal(b[4] - a[4], k)
 
 
+@pytest.mark.parametrize("persistent", [0, 1])
+def test_a_sort_whose_wait_runs_out_is_contained(capi, persistent):
+    """The blocks of a sort wait for one that never comes: the call reports it,
+    nothing steps with the old list, and the engine goes on from the state
+    before; a replica added afterwards is sorted too."""
+    from rumd_b200 import initconf as I
+    n = 3000
+    params = np.ascontiguousarray(I.lj_params(2, I.KA), np.float32)
+    conf = [I.ka_config(n, T=1.2, seed=s) for s in (1, 2)]
+
+    def engine():
+        e = capi.Engine(device=0, pb=64, tp=2)
+        e.set_variant(capi.VARIANT_PERSISTENT, persistent)
+        return e, e.add(conf[0]["pos4"], conf[0]["box"], params, 2, T=1.2, vel4=conf[0]["vel4"])
+
+    e, rid = engine()
+    e.run(40)
+    want = e.get(rid, "pos", n), e.get(rid, "force", n)
+    e.close()
+    e, rid = engine()
+    for call in (e.calc_f, lambda: e.run(5)):
+        e.set(rid, "pos", conf[0]["pos4"])  # its list is due
+        capi.check(capi.lib().b2md_probe_stall_sort(e._h))
+        with pytest.raises(Exception, match="sort"):
+            call()
+        st = e.stats(rid)
+        assert st["steps"] == 0 and st["rebuilds"] == 0 and st["overflow"] == 0
+        assert np.array_equal(e.get(rid, "pos", n), conf[0]["pos4"])
+    e.run(40)
+    got = e.get(rid, "pos", n), e.get(rid, "force", n)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    capi.check(capi.lib().b2md_probe_stall_sort(e._h))
+    e.set(rid, "pos", conf[0]["pos4"])
+    with pytest.raises(Exception, match="sort"):
+        e.calc_f()
+    e.remove(rid)
+    rid = e.add(conf[1]["pos4"], conf[1]["box"], params, 2, T=1.2, vel4=conf[1]["vel4"])
+    e.calc_f()
+    f = e.get(rid, "force", n)
+    e.close()
+    e = capi.Engine(device=0, pb=64, tp=2)
+    rid = e.add(conf[1]["pos4"], conf[1]["box"], params, 2, T=1.2, vel4=conf[1]["vel4"])
+    e.calc_f()
+    assert np.array_equal(e.get(rid, "force", n), f)
+    e.close()
+
+
 def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi):
     """Coordinates far outside the box, infinite or not a number (a system that
     has blown up) go to some cell of the grid: the evaluation returns, and the
