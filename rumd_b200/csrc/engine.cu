@@ -2099,6 +2099,7 @@ int b2md_replica_read(b2md_engine* e, int id, float* pos4, float* vel4, int* im3
     CK(cudaSetDevice(e->device));
     const unsigned what = (pos4 ? kReadPos : 0u) | (vel4 ? kReadVel : 0u) | (im3 ? kReadImages : 0u);
     if (what) read_back(e, id, h, what, nullptr, pos4, vel4, im3);
+    else CK(cudaStreamSynchronize(e->stream));  // nothing to read: still waits for what is queued
   });
 }
 

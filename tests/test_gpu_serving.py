@@ -58,6 +58,23 @@ def _alone(capi, c, params, steps):
     return st, pos
 
 
+def test_read_of_no_field_waits_for_the_chunk():
+    """b2md_replica_read waits for what is queued, whichever fields it is asked for."""
+    from rumd_b200 import capi, initconf
+    n = 4000
+    c = initconf.ka_config(n, T=1.0, seed=3)
+    e = capi.Engine(device=0, pb=64, tp=2)
+    rid = e.add(c["pos4"], c["box"], initconf.lj_params(2, initconf.KA), 2, T=1.0, vel4=c["vel4"])
+    e.run(1)
+    e.queue(rid, 4000)
+    ticket = e.run_queued_async()
+    assert not e.poll(ticket)
+    capi.check(capi.lib().b2md_replica_read(e._h, rid, None, None, None))
+    assert e.poll(ticket)
+    e.wait(ticket)
+    e.close()
+
+
 @pytest.mark.parametrize("persistent", [2, 3])
 def test_admission_and_removal_under_a_running_chunk(persistent):
     """k_batch (k_flow) engine: replicas A, B run; while a chunk holds A, A is
