@@ -11,7 +11,7 @@
 #include <cstring>
 #include <map>
 #include <string>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -1671,12 +1671,13 @@ void read_back(b2md_engine* e, int id, HostRep& h, unsigned what, const float4* 
   std::vector<cudaError_t> err(nthr, cudaSuccess);
   std::vector<std::thread> th;
   int started = 1;
+  th.reserve(nthr);  // (nothing may throw past a thread that runs)
   try {
     for (; started < nthr; ++started) {
       const int t = started;
       th.emplace_back([&, t] { err[t] = part(t, &e->read_ev[2 * t]); });
     }
-  } catch (const std::system_error&) {  // no thread to be had: the rest here
+  } catch (const std::exception&) {  // no thread to be had: the rest here
   }
   err[0] = part(0, &e->read_ev[0]);
   for (int t = started; t < nthr; ++t) err[t] = part(t, &e->read_ev[2 * t]);
