@@ -195,12 +195,23 @@ def test_a_sort_whose_wait_runs_out_is_contained(capi, persistent):
     e.close()
 
 
-def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi):
-    """Coordinates far outside the box, infinite or not a number (a system that
-    has blown up) go to some cell of the grid: the evaluation returns, and the
-    particles out of their reach keep their forces."""
+def kernel_image(d, L):
+    """The minimum image of float32 separations d in a box of length L, with the
+    device's float32 operations: the rounding by adding 1.5 * 2^23 (which is none
+    far outside the box), the product and sum fused."""
+    d, L, m = np.asarray(d, np.float32), np.float32(L), np.float32(12582912.0)
+    k = (d * (np.float32(1) / L) + m) - m
+    return d.astype(np.float64) - np.float64(L) * k.astype(np.float64)
+
+
+@pytest.mark.parametrize("far", [False, True])
+def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi, far):
+    """Coordinates that are infinite or not a number, or far outside the box (a
+    system that has blown up), go to some cell of the grid: the evaluation
+    returns, and every particle out of their reach, where they were and where
+    the device's minimum image puts them, keeps its force."""
     from rumd_b200 import initconf as I
-    n = 4000
+    n, reach = 4000, 2.5 + 0.3 + 0.01
     c = I.ka_config(n, T=0.8, seed=3)
     p = np.ascontiguousarray(I.lj_params(2, I.KA), np.float32)
     e = capi.Engine(device=0, pb=64, tp=2)
@@ -208,21 +219,67 @@ def test_positions_of_a_blown_up_system_stay_in_the_cell_arrays(capi):
     e.calc_f()
     f0 = e.get(rid, "force", n)
     bad = c["pos4"].copy()
-    bad[:4, 0] = [np.inf, -np.inf, np.nan, 3e30]
-    bad[4, 1], bad[5, 2] = -3e30, 5e9
+    if far:
+        bad[0, 0], bad[1, 1], bad[2, 2], bad[3, :3] = 3e30, -3e30, 5e9, [4e4, -70.0, 1e6]
+    else:
+        bad[:3, 0] = [np.inf, -np.inf, np.nan]
+        bad[3, 1] = bad[3, 2] = np.nan
     e.set(rid, "pos", bad)
     e.calc_f()
     f1 = e.get(rid, "force", n)
     L = c["box"]
-    d = c["pos4"][None, :6, :3] - c["pos4"][:, None, :3]
+    d = c["pos4"][None, :4, :3] - c["pos4"][:, None, :3]
     d -= L * np.rint(d / L)
-    far = ((d * d).sum(-1) > 2.5 ** 2).all(1)
-    far[:6] = False
-    same = np.isclose(f0[far], f1[far], rtol=1e-4, atol=1e-3).all(1)
-    # (the displaced particles land in some cell and may act on those near it)
-    assert same.mean() > 0.8
+    keep = ((d * d).sum(-1) > reach ** 2).all(1)
+    if far:
+        d = np.stack([kernel_image(bad[:, None, k] - bad[None, :4, k], L[k]) for k in range(3)], -1)
+        keep &= ((d * d).sum(-1) > reach ** 2).all(1)
+    keep[:4] = False
+    assert keep.sum() > 3000
+    assert np.isclose(f0[keep], f1[keep], rtol=1e-4, atol=1e-3).all()
     e.set(rid, "pos", c["pos4"])
     e.calc_f()
     assert np.array_equal(e.get(rid, "pos", n), c["pos4"])
     assert np.allclose(e.get(rid, "force", n), f0, rtol=1e-4, atol=1e-3)
+    e.close()
+
+
+# (44 bytes a particle, 16 for one field): the largest read in one piece and one
+# more; the largest copied out by one thread and one more; an odd size beyond
+@pytest.mark.parametrize("n", [35746, 35747, 190650, 190651, 300007, 530003])
+def test_read_backs_return_every_particle_in_the_callers_order(capi, n):
+    """Positions, velocities and images, known and different for every particle,
+    before a sort, after one, and after they have been set anew."""
+    from rumd_b200 import initconf as I
+    rng = np.random.default_rng(n)
+    m = int(np.ceil(np.cbrt(n)))
+    box = np.full(3, 1.0625 * m, np.float32)
+    sites = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+
+    def state():
+        pos4 = np.zeros((n, 4), np.float32)
+        pos4[:, :3] = (sites[rng.permutation(len(sites))[:n]] + 0.5) * 1.0625 - 0.53125 * m
+        vel4 = np.ones((n, 4), np.float32)
+        vel4[:, :3] = rng.standard_normal((n, 3))
+        return pos4, vel4, rng.integers(-1000, 1000, (n, 3)).astype(np.int32)
+
+    def check(want):
+        for got, w in zip(e.read(rid, n), want):
+            assert np.array_equal(got, w)
+        for name, w in zip(("pos", "vel", "images"), want):
+            assert np.array_equal(e.get(rid, name, n), w)
+
+    e = capi.Engine(device=0, max_particles=n, pb=64, tp=2)
+    a = state()
+    rid = e.add(a[0], box, np.ascontiguousarray(I.lj_params(1, I.LJ), np.float32), 1, vel4=a[1], im3=a[2])
+    check(a)
+    e.calc_f()
+    check(a)
+    b = state()
+    e.set(rid, "pos", b[0])
+    e.set(rid, "vel", b[1])
+    e.set(rid, "images", b[2])
+    check(b)
+    e.calc_f()
+    check(b)
     e.close()
