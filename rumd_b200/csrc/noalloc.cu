@@ -230,7 +230,7 @@ __device__ __forceinline__ float warp_sum(const float (&v)[G]) {
 // Candidate j of every lane (a NaN position where the lane has none) against
 // the warp's G particles.  wrap: the dimensions (1, 2, 4) that need the
 // minimum-image step; uniform in the warp.
-template <int G>
+template <int G, bool SF>
 __device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G], int p0, int j, const float4& rj,
                                               unsigned wrap, const float* s_tab, int ntypes, const float3& L,
                                               const float3& iL) {
@@ -264,11 +264,15 @@ __device__ __forceinline__ void add_candidate(Sum5 (&A)[G], const float4 (&rp)[G
     // 1/r, which only the shifted-force term uses, refined as there
     const float2 e = *reinterpret_cast<const float2*>(row + 4);  // c_u0, 6 A6
     const float i2 = b2md::rcp_approx(d2), i6 = i2 * i2 * i2, t = c.y * i6;
-    float y = b2md::rsqrt_approx(d2);
-    y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
-    const float s = __fmaf_rn(-c.w, y, i6 * i2 * __fmaf_rn(12.f, t, e.y));
+    float s = i6 * i2 * __fmaf_rn(12.f, t, e.y), u0 = e.x;
+    if constexpr (SF) {
+      float y = b2md::rsqrt_approx(d2);
+      y = y * __fmaf_rn(-0.5f * d2 * y, y, 1.5f);
+      s = __fmaf_rn(-c.w, y, s);
+      u0 = __fmaf_rn(c.w, d2 * y, u0);
+    }
     if (in) {  // (dx is NaN in lanes without a candidate)
-      A[q].u += __fmaf_rn(i6, t + c.z, __fmaf_rn(c.w, d2 * y, e.x));
+      A[q].u += __fmaf_rn(i6, t + c.z, u0);
       A[q].fx = __fmaf_rn(dx[q], s, A[q].fx);
       A[q].fy = __fmaf_rn(dy[q], s, A[q].fy);
       A[q].fz = __fmaf_rn(dz[q], s, A[q].fz);
@@ -309,7 +313,7 @@ __device__ __forceinline__ void store_forces(const Sum5 (&A)[G], const unsigned 
 // The m <= G particles of a cell from p0 on (a missing one has a NaN position,
 // which is in range of nothing).  The next round's candidates are loaded while
 // the current one's pairs are computed.
-template <int G>
+template <int G, bool SF>
 __device__ __forceinline__ void cell_group(NoAllocScratch* scr, int n, const int4* tab, int off, int len, int total,
                                            int p0, int m, unsigned wrap, const float* s_tab, int ntypes, const float3& L,
                                            const float3& iL, float4* __restrict__ force, double& u, double& w) {
@@ -344,12 +348,12 @@ __device__ __forceinline__ void cell_group(NoAllocScratch* scr, int n, const int
       rn = sp[jn];
     }
     if (ch + lane >= total) rj.x = nan;
-    add_candidate<G>(A, rp, p0, j, rj, wrap, s_tab, ntypes, L, iL);
+    add_candidate<G, SF>(A, rp, p0, j, rj, wrap, s_tab, ntypes, L, iL);
   }
   store_forces<G>(A, id, n, force, u, w);
 }
 
-template <int G>
+template <int G, bool SF>
 __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, int n, int p0, const float* s_tab,
                                                 int ntypes, const float3& L, const float3& iL,
                                                 float4* __restrict__ force, double& u, double& w) {
@@ -374,7 +378,7 @@ __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, 
       rj.x = __int_as_float(0x7fc00000);
       rj.w = 0.f;
     }
-    add_candidate<G>(A, rp, p0, j, rj, 7u, s_tab, ntypes, L, iL);
+    add_candidate<G, SF>(A, rp, p0, j, rj, 7u, s_tab, ntypes, L, iL);
   }
   store_forces<G>(A, id, n, force, u, w);
 }
@@ -389,7 +393,7 @@ __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, 
 // back to back, all pairs by one thread per particle before: N=65521 7275 ->
 // 106 us, N=16384 1388 -> 49, N=4000 369 -> 37, N=1000 109 -> 17 (the last
 // three mostly launches).
-template <int G, bool CELLS>
+template <int G, bool CELLS, bool SF>
 __global__ void __launch_bounds__(kNoAllocBlock, 7)
     k_forces_noalloc(const float4* __restrict__ pos, int n, float3 L, float3 iL, Grid3 g, int ntypes, PairTable tab,
                      float4* __restrict__ force, double* __restrict__ sums, NoAllocScratch* scr) {
@@ -447,7 +451,7 @@ __global__ void __launch_bounds__(kNoAllocBlock, 7)
       __syncwarp();
       for (int p = p0; p < p1; p += 4) {
         const int m = min(4, p1 - p);
-#define CG(K) cell_group<K>(scr, n, rowtab, off, len, total, p, m, wrap, s_tab, ntypes, L, iL, force, u, w)
+#define CG(K) cell_group<K, SF>(scr, n, rowtab, off, len, total, p, m, wrap, s_tab, ntypes, L, iL, force, u, w)
         if (m > 2) CG(4);
         else CG(2);
 #undef CG
@@ -458,9 +462,9 @@ __global__ void __launch_bounds__(kNoAllocBlock, 7)
     for (int k = blockIdx.x * kNoAllocWarps + warp; k < units; k += stride) {
       const int p = k * G;
       if (p + G <= n) {
-        all_pairs_group<G>(pos, n, p, s_tab, ntypes, L, iL, force, u, w);
+        all_pairs_group<G, SF>(pos, n, p, s_tab, ntypes, L, iL, force, u, w);
       } else {
-        for (int r = p; r < n; ++r) all_pairs_group<1>(pos, n, r, s_tab, ntypes, L, iL, force, u, w);
+        for (int r = p; r < n; ++r) all_pairs_group<1, SF>(pos, n, r, s_tab, ntypes, L, iL, force, u, w);
       }
     }
   }
@@ -655,9 +659,13 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
   const float4* p4 = reinterpret_cast<const float4*>(pos4);
   float4* f4 = reinterpret_cast<float4*>(force4);
   const int tb = (n + 255) / 256;
-#define NA(G, C, UNITS)                                                                                               \
-  k_forces_noalloc<G, C><<<std::min(((UNITS) + kNoAllocWarps - 1) / kNoAllocWarps, kNoAllocMaxBlocks), kNoAllocBlock, \
-                           0, s>>>(p4, n, L, iL, g, ntypes, tab, f4, sums, scr)
+  const bool sf = cutoff_method == B2MD_CUTOFF_SF;
+#define NA(G, C, UNITS)                                                                                     \
+  {                                                                                                         \
+    const auto kernel = sf ? k_forces_noalloc<G, C, true> : k_forces_noalloc<G, C, false>;                  \
+    kernel<<<std::min(((UNITS) + kNoAllocWarps - 1) / kNoAllocWarps, kNoAllocMaxBlocks), kNoAllocBlock, 0, s>>>( \
+        p4, n, L, iL, g, ntypes, tab, f4, sums, scr);                                                       \
+  }
   if (cells) {
     k_na_count<<<tb, 256, 0, s>>>(p4, n, L, iL, g, scr);
     k_na_scan<<<1, 1024, 0, s>>>(ncell, crowd_limit(n), scr);
@@ -665,13 +673,13 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
     k_na_gather<<<tb, 256, 0, s>>>(p4, n, L, iL, ntypes, scr);
     // (a warp per cell, and warps enough for all pairs, four particles each,
     // should the cells turn out crowded)
-    NA(4, true, std::max(ncell, (n + 3) / 4));
+    NA(4, true, std::max(ncell, (n + 3) / 4))
   } else if (n <= 2400) {
-    NA(1, false, n);
+    NA(1, false, n)
   } else if (n <= 4800) {
-    NA(2, false, (n + 1) / 2);
+    NA(2, false, (n + 1) / 2)
   } else {
-    NA(4, false, (n + 3) / 4);
+    NA(4, false, (n + 3) / 4)
   }
 #undef NA
   const cudaError_t le = cudaGetLastError();
