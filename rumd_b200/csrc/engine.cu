@@ -172,7 +172,8 @@ struct b2md_engine {
   unsigned* smctr = nullptr;   // SM-region claim counters (nsm + 1)
   int win_cap = 2560;          // FM_WINDOW: window capacity in particles
   int wl_rows_cap = 128;       // FM_WINDOW: window-list rows staged in shared memory (0 = stream)
-  int build_lanes = 0;         // list build: 0 contiguous candidate runs per lane, else lanes per particle (32: one warp per cell)
+  int build_lanes = 0;         // list build: 0 k_rb_build_runs (one warp per cell, by ballots), else lanes per particle
+                               // (32: one warp per cell, candidates staged in shared memory)
   bool build_smem = false;     // list build: tile assembled in shared memory
   int persist = 1;             // runs: 0 one launch per step; 1 persistent (k_steps when every tile has a
                                // resident block, else k_flow); 2 k_batch, 3 k_flow whenever they apply

@@ -1743,9 +1743,11 @@ __device__ bool sort_barrier(PersistCtl* c) {
 // needs no rebuild pays one launch for it.  The phases are a microsecond or
 // two of latency each, so the number of launches and of blocks that meet is
 // what costs: as seven kernels of a block per tile the sort took 37 us at KA
-// N=65536 (ncu, 4.6 to 9.5 us each); as one launch a rebuild takes 111 us
-// instead of 115 there, 985 instead of 1042 at LJ N = 2^20, and a force
-// evaluation without a rebuild launches two kernels instead of eight.
+// N=65536 (ncu, 4.6 to 9.5 us each), as one launch 28 (ncu, barrier waits and
+// load latency), and a force evaluation without a rebuild launches two kernels
+// instead of eight.  With the list build of that time the step lost 0.9 us of
+// 35.5 there and 14 us of 364 at LJ N = 2^20.  A whole rebuild, with the
+// relaunch of the steps, takes 107 us and 1.10 ms.
 constexpr int kScanGroup = 128;
 constexpr int kSortBlock = 512;
 __global__ void __launch_bounds__(kSortBlock, 2) k_rb_sort(EngArgs a, int pb) {
@@ -2573,8 +2575,8 @@ __device__ __forceinline__ int build_cell(const RepDev& R, const float4* rc, con
   int rows = 0;  // non-empty rows that start before the current 32 candidates
   // the round's candidate (slot; one past the last repeats the cell's first
   // particle): the next round's is loaded while the current one is tested
-  // (the chain row mask - table - position bounds a round; a rebuild at KA
-  // N=65536 120 -> 111 us, with twice the blocks in flight 103)
+  // (the chain row mask - table - position bounds a round: loading ahead took
+  // 9 of 120 us off a rebuild at KA N=65536, twice the blocks in flight 8 more)
   auto candidate = [&](int ch) -> int {
     const int v = ch + lane;
     const unsigned rel = (unsigned)(cr.off - ch);

@@ -389,10 +389,11 @@ __device__ __forceinline__ void all_pairs_group(const float4* __restrict__ pos, 
 // What bounds the cell form is the pair arithmetic: about 300 candidates per
 // particle at KA density, of which a quarter is in range, and the chain to the
 // candidates' positions.  Held to 72 registers for seven blocks per SM (KA
-// N=65521: 109 us a call with 96 registers, 112 with 80, 106 with 72).  Calls
-// back to back, all pairs by one thread per particle before: N=65521 7275 ->
-// 106 us, N=16384 1388 -> 49, N=4000 369 -> 37, N=1000 109 -> 17 (the last
-// three mostly launches).
+// N=65521: 109 us a call with 96 registers, 112 with 80, 106 with 72, before 1/r
+// was refined).  Calls back to back, shifted force, all pairs by one thread per
+// particle before: N=65521 7275 -> 111 us (shifted potential 108), N=16384
+// 1388 -> 51, N=4000 369 -> 37, N=1000 109 -> 16 (the last three mostly
+// launches).
 template <int G, bool CELLS, bool SF>
 __global__ void __launch_bounds__(kNoAllocBlock, 7)
     k_forces_noalloc(const float4* __restrict__ pos, int n, float3 L, float3 iL, Grid3 g, int ntypes, PairTable tab,
@@ -635,10 +636,15 @@ extern "C" int b2md_forces_noalloc(const float* pos4, int n, const float* box, i
     q[5] = 6.f * p[2];
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Cells pay from about 3000 particles (N=2000: 25 us all pairs, 35 cells;
-  // N=4000: 50 and 37) and where a cell's neighbourhood is a third of the box
-  // or less; otherwise every warp tests its particles against all, one
-  // particle per warp while that is what fills the GPU.
+  // Cells pay from about 3000 particles (us a call with cells / all pairs, one
+  // particle per warp: KA N=2400 33 / 27, 3000 35 / 32, 3500 37 / 37, 4000
+  // 37 / 41; LJ 2400 31 / 27, 3000 32 / 31, 3500 34 / 36) and where a cell's
+  // neighbourhood is a third of the box or less.  Otherwise every warp tests one,
+  // two or four particles against all: one while the GPU's warps hold them all
+  // in one wave, and more where that would take several (KA with one / two /
+  // four: N=2400 27 / 31 / 44 us, 4000 41 / 50 / 70, 4800 81 / 58 / 83, 8000
+  // 135 / 101 / 142, 16000 491 / 364 / 354).  The lines at 2400 and 4800 lie
+  // before the crossings: only boxes without cells reach the larger sizes.
   Grid3 g{1, 1, 1};
   float reach = 0.f;  // (a pair's range is its cut-off squared, whatever its sign)
   for (int k = 0; k < ntypes * ntypes; ++k) reach = std::max(reach, fabsf(params[k * 12]));
